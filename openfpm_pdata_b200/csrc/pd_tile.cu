@@ -509,9 +509,13 @@ double fp32_band(pd_vd h, double r) {
     double X = 0;
     for (int d = 0; d < 3; ++d)
         X = std::max(X, std::max(std::fabs(h->lo[d] - 2 * h->g[d]), std::fabs(h->hi[d] + 2 * h->g[d])));
+    return fp32_band_at(X, r) + std::ldexp(1.0, -20);  // room for the cutoff's own rounding at any r
+}
+
+double fp32_band_at(double X, double r) {
     const double u = std::ldexp(1.0, -24);
     double D = 2 * u * X + u * r;                       // per-component error of the FP32 difference
-    double e = 2 * std::sqrt(3.0) * r * D + 3 * D * D + 4 * u * (r * r + 1.0);
+    double e = 2 * std::sqrt(3.0) * r * D + 3 * D * D + 4 * u * r * r;
     return 4 * e;                                       // safety factor 4
 }
 

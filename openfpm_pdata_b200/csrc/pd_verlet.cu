@@ -5,13 +5,13 @@
 // d2 < r_cut^2, found through a cell list of side r_cut over the domain
 // enlarged by the ghost magnified 1.013.  Here:
 //   1. the cell list is built by the counting sort of pd_celllist.cu;
-//   2. positions are gathered into cell order with the original index in the
-//      record's 4th word (pos_cs);
+//   2. FP32 copies of the positions are gathered into cell order with the original
+//      index in the record's 4th word;
 //   3. one CTA per tile of TX cells along x stages the 9 neighbour rows
-//      (x-1 .. x+TX for dy, dz in {-1,0,1}; each a contiguous range of pos_cs)
-//      in shared memory and every thread scans the 27-cell neighbourhood of its
-//      particles from there, in the reference walk order (dz, dy, dx, in-cell
-//      order), writing column-major rows nbr[k*stride + i].
+//      (x-1 .. x+TX for dy, dz in {-1,0,1}; each a contiguous range of the copies),
+//      three at a time, in shared memory and every thread scans the 27-cell
+//      neighbourhood of its particles from there, in the reference walk order (dz,
+//      dy, dx, in-cell order), writing column-major rows nbr[k*stride + i].
 // Rows longer than the capacity set ERR_NN_OVERFLOW and record the longest row;
 // the host grows the capacity and rebuilds.
 //
@@ -23,135 +23,266 @@
 // image are folded onto its source by ghost_put<add_> (vector_dist.hpp:2304).
 // The criterion is geometric, not cell-based, so it does not depend on the box
 // being a whole number of cells.
+#include <cmath>
+
 #include "pd_device.cuh"
 #include "pd_internal.cuh"
+#include "pd_tile.cuh"
+#include "pd_tile_dev.cuh"
 
 namespace pd {
 
-template <class T> struct IdxBits;
-template <> struct IdxBits<double> {
-    __device__ static double enc(int i) { return __longlong_as_double((long long)i); }
-    __device__ static int dec(double w) { return (int)__double_as_longlong(w); }
-};
-template <> struct IdxBits<float> {
-    __device__ static float enc(int i) { return __int_as_float(i); }
-    __device__ static int dec(float w) { return __float_as_int(w); }
-};
+// largest coordinate of a position inside the cell grid, padding cells included
+static double verlet_bound(pd_cl cl) {
+    double X = 0;
+    for (int d = 0; d < 3; ++d) {
+        const double a = cl->box_lo[d] - cl->pad * cl->spacing[d];
+        const double b = cl->box_lo[d] + (cl->gs[d] - cl->pad) * cl->spacing[d];
+        X = std::max(X, std::max(std::fabs(a), std::fabs(b)));
+    }
+    return X * (1.0 + 1e-6);
+}
 
-// pos_cs[k] = (pos[sorted[k]].xyz, bits(sorted[k]))
+// p32[k] = FP32 copy of pos[sorted[k]] with the original index in w: what the row
+// kernel stages, half the bytes of an FP64 record.  *wide is set when a coordinate
+// exceeds `bound` (or is NaN): the FP32 band then does not hold and the row kernel
+// decides every candidate in the position type.
 template <class T>
 __global__ void k_gather_cs(const typename V4<T>::type* __restrict__ pos, const int* __restrict__ sorted,
-                            const unsigned int* __restrict__ cs_end, typename V4<T>::type* __restrict__ out,
-                            long n_bound) {
+                            const unsigned int* __restrict__ cs_end, float4* __restrict__ out, long n_bound, T bound,
+                            unsigned int* __restrict__ wide) {
     long n = (long)*cs_end;
     if (n > n_bound) n = n_bound;
+    bool bad = false;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
-        int i = sorted[k];
-        typename V4<T>::type r = ld4(pos, i);
-        r.w = IdxBits<T>::enc(i);
-        st4(out, k, r);
+        const int i = sorted[k];
+        const typename V4<T>::type r = ld4(pos, i);
+        bad = bad || !(fabs(r.x) <= bound && fabs(r.y) <= bound && fabs(r.z) <= bound);
+        out[k] = make_float4((float)r.x, (float)r.y, (float)r.z, __int_as_float(i));
     }
+    if (bad) atomicOr(wide, 1u);
 }
 
 template <class T4> __device__ __forceinline__ bool lex_after(const T4& a, const T4& b) {
     return a.x > b.x || (a.x == b.x && (a.y > b.y || (a.y == b.y && a.z > b.z)));
 }
 
-template <class T>
-__global__ void __launch_bounds__(128) k_verlet_tile(const typename V4<T>::type* __restrict__ pcs, Grid<T> G, int TX,
-                                                     int ntx, const unsigned int* __restrict__ cs, long n_dom, T r2,
-                                                     int* __restrict__ nbr, int* __restrict__ nn, long stride,
-                                                     int max_nn, int smem_cap, int sym,
-                                                     unsigned int* __restrict__ ctrl_err,
-                                                     unsigned int* __restrict__ ctrl_nnmax) {
-    typedef typename V4<T>::type T4;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T4* sp = reinterpret_cast<T4*>(smem_raw);
-    __shared__ unsigned int row_beg[9], row_off[9];
-    __shared__ unsigned int cs_sm[9][40];
-    __shared__ int use_smem;
-
-    const int gx = G.gs[0];
-    const int ny = G.gs[1] - 2 * G.pad, nz = G.gs[2] - 2 * G.pad;
-    long t = blockIdx.x;
-    int tx = (int)(t % ntx);
-    long rest = t / ntx;
-    int y = (int)(rest % ny) + G.pad;
-    int z = (int)(rest / ny) + G.pad;
-    int x0 = G.pad + tx * TX;
-    int x1 = min(x0 + TX, gx - G.pad);  // exclusive
-    int ncol = x1 - x0 + 3;             // cells x0-1 .. x1 (x1 inclusive) + end marker
-
+// the 9 cell-row ranges of tile t in the cell-ordered array (no image ranges: real
+// particles and ghosts are sorted together)
+__device__ __forceinline__ void verlet_layout(const TileGeom& tg, long t, const unsigned int* __restrict__ cs,
+                                              TileSh& S) {
+    const int tx = (int)(t % tg.ntx);
+    const long rest = t / tg.ntx;
+    const int y = (int)(rest % tg.ny) + tg.pad, z = (int)(rest / tg.ny) + tg.pad;
+    const int x0 = tg.pad + tx * tg.TX, x1 = min(x0 + tg.TX, tg.gs0 - tg.pad);
+    const int ncol = x1 - x0 + 3;  // cells x0-1 .. x1 and the end of cell x1
     for (int e = threadIdx.x; e < 9 * ncol; e += blockDim.x) {
-        int r = e / ncol, j = e % ncol;
-        int dz = r / 3 - 1, dy = r % 3 - 1;
-        long c = (long)(x0 - 1 + j) + (long)gx * ((y + dy) + (long)G.gs[1] * (z + dz));
-        cs_sm[r][j] = cs[c];  // j == ncol-1 reads the start of cell x1+1 = end of cell x1
+        const int r = e / ncol, j = e % ncol;
+        const int dz = r / 3 - 1, dy = r % 3 - 1;
+        S.cR[r][j] = cs[(long)(x0 - 1 + j) + (long)tg.gs0 * ((y + dy) + (long)tg.gs1 * (z + dz))];
     }
+    if (threadIdx.x < 9) S.cI[threadIdx.x][0] = S.cI[threadIdx.x][ncol - 1] = 0;
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned int off = 0;
+        unsigned int o = 0;
         for (int r = 0; r < 9; ++r) {
-            row_beg[r] = cs_sm[r][0];
-            row_off[r] = off;
-            off += cs_sm[r][ncol - 1] - cs_sm[r][0];
+            S.oR[r] = S.oI[r] = o;
+            o += S.cR[r][ncol - 1] - S.cR[r][0];
         }
-        use_smem = (int)(off <= (unsigned int)smem_cap);
+        S.total = o;
+        S.ncol = ncol;
     }
     __syncthreads();
-    const bool sm = use_smem != 0;
-    if (sm) {
-        for (int r = 0; r < 9; ++r) {
-            unsigned int b = row_beg[r], len = cs_sm[r][ncol - 1] - b, o = row_off[r];
-            for (unsigned int k = threadIdx.x; k < len; k += blockDim.x) sp[o + k] = pcs[b + k];
-        }
-    }
-    __syncthreads();
+}
 
-    // domain particles of the centre row cells x0 .. x1-1 (row index 4: dy = dz = 0)
-    unsigned int ib = cs_sm[4][1], ie = cs_sm[4][ncol - 2];
-    for (unsigned int k = ib + threadIdx.x; k < ie; k += blockDim.x) {
-        T4 xi = pcs[k];
-        int i = IdxBits<T>::dec(xi.w);
-        if (i >= n_dom) continue;
-        // column of k's cell inside the tile: find j with cs_sm[4][j] <= k < cs_sm[4][j+1]
-        int j = 1;
-        while (j < ncol - 2 && cs_sm[4][j + 1] <= k) ++j;
-        int cnt = 0;
+// half-list rule: a domain partner q of i iff q > i, an image iff it lies after i
+template <class T>
+__device__ __forceinline__ bool sym_keep(const typename V4<T>::type* __restrict__ pos, int i, int q, long n_dom) {
+    if (q < n_dom) return q > i;
+    const typename V4<T>::type a = ld4(pos, (long)q), b = ld4(pos, (long)i);
+    return lex_after(a, b);
+}
+
+// Entries of particle i from the n candidates c4[0..n) appended to its row in
+// candidate order: accept masks of up to three chunks of 32 first, then one stream
+// of the accepted ones (see seg_rows).  Works on staged and on global records.
+template <class T, bool SYM>
+__device__ __forceinline__ void verlet_seg(const float4* __restrict__ c4, unsigned int n, const float4 x, int i,
+                                           const typename V4<T>::type* __restrict__ pos, T r2, float lo_thr,
+                                           float hi_thr, long n_dom, int* __restrict__ out, long stride, int max_nn,
+                                           int& c) {
 #pragma unroll 1
-        for (int r = 0; r < 9; ++r) {
-            unsigned int a = cs_sm[r][j - 1], e = cs_sm[r][j + 2];
-            const T4* base = sm ? (sp + row_off[r] - row_beg[r]) : pcs;
-#pragma unroll 4
-            for (unsigned int q = a; q < e; ++q) {
-                T4 xq = base[q];
-                T d2 = dist2(xi.x - xq.x, xi.y - xq.y, xi.z - xq.z);
-                if (d2 < r2) {
-                    const int qi = IdxBits<T>::dec(xq.w);
-                    if (sym && !(qi < n_dom ? qi > i : lex_after(xq, xi))) continue;
-                    if (cnt < max_nn) nbr[(long)cnt * stride + i] = qi;
-                    cnt++;
-                }
-            }
+    for (unsigned int q0 = 0; q0 < n; q0 += 96) {
+        const unsigned int m = min(96u, n - q0);
+        const unsigned int na = min(32u, m), nb = min(32u, m - na), nc = m - na - nb;
+        unsigned int ma = chunk_mask<T>(c4 + q0, na, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
+        unsigned int mb = chunk_mask<T>(c4 + q0 + 32, nb, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
+        unsigned int mc = chunk_mask<T>(c4 + q0 + 64, nc, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
+        // candidate of the highest bit of a mask: q + clz (modulo 2^32)
+        unsigned int qa = q0 + na - 32, qb = q0 + 32 + nb - 32, qc = q0 + 64 + nc - 32;
+        for (int rem = __popc(ma) + __popc(mb) + __popc(mc); rem > 0; --rem) {
+            if (ma == 0) { ma = mb; qa = qb; mb = mc; qb = qc; mc = 0; }
+            if (ma == 0) { ma = mb; qa = qb; mb = 0; }
+            const int z = __clz(ma);
+            ma ^= 0x80000000u >> z;
+            const int q = __float_as_int(c4[qa + (unsigned int)z].w);
+            if (SYM && !sym_keep<T>(pos, i, q, n_dom)) continue;
+            if (c < max_nn) out[(long)c * stride] = q;
+            ++c;
         }
-        if (cnt > max_nn) {
-            atomicOr(ctrl_err, ERR_NN_OVERFLOW);
-            atomicMax(ctrl_nnmax, (unsigned int)cnt);
-            cnt = max_nn;
-        }
-        nn[i] = cnt;
     }
 }
 
-static int choose_tx(pd_cl cl, long n_all, int& TX) {
-    double cells = (double)cl->div[0] * cl->div[1] * cl->div[2];
-    double occ = cells > 0 ? (double)n_all / cells : 1.0;
-    int tx = (int)(96.0 / (occ > 1e-3 ? occ : 1e-3));
-    int nxi = cl->gs[0] - 2 * cl->pad;
-    if (tx < 1) tx = 1;
-    if (tx > 32) tx = 32;
-    if (tx > nxi) tx = nxi;
-    TX = tx;
+// the same with every candidate decided in the position type (coordinates beyond the FP32 band's range)
+template <class T, bool SYM>
+__device__ __noinline__ void verlet_seg_wide(const float4* __restrict__ c4, unsigned int n, int i,
+                                             const typename V4<T>::type* __restrict__ pos, T r2, long n_dom,
+                                             int* __restrict__ out, long stride, int max_nn, int& c) {
+    for (unsigned int k = 0; k < n; ++k) {
+        const int q = __float_as_int(c4[k].w);
+        if (!exact_in<T>(pos, (unsigned int)i, q, r2)) continue;
+        if (SYM && !sym_keep<T>(pos, i, q, n_dom)) continue;
+        if (c < max_nn) out[(long)c * stride] = q;
+        ++c;
+    }
+}
+
+// Rows of the domain particles of one tile (TX cells of a cell row), global original
+// indices, column-major nbr[k*stride + i], in the walk order dz, dy, dx, in-cell.
+// Bound by the instructions of the candidate tests (27 cells hold about 6.4 times
+// the pairs kept), so: FP32 tests on 16-byte staged copies, sign bits shifted into
+// accept masks, the rare candidates within the rounding band decided exactly in the
+// position type (the scheme of the integrator's row build); one z-layer of three cell
+// rows staged at a time, so that nine CTAs fit an SM.  A layer beyond `pcap` records
+// is read from global memory instead.
+// Measured: 1,000,000 FP64 particles of a lattice (49 entries a row) 1198 -> 530 us, half
+// rows of 200,001 348 -> 171 us against FP64 records of all nine rows staged at once.
+template <class T, bool SYM>
+__global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>::type* __restrict__ pos,
+                                                        const float4* __restrict__ p32, TileGeom tg,
+                                                        const unsigned int* __restrict__ cs, long n_dom, T r2,
+                                                        float lo_thr, float hi_thr, int* __restrict__ nbr,
+                                                        int* __restrict__ nn, long stride, int max_nn,
+                                                        unsigned int pcap, const unsigned int* __restrict__ wide,
+                                                        unsigned int* __restrict__ ctrl_err,
+                                                        unsigned int* __restrict__ ctrl_nnmax) {
+    extern __shared__ __align__(128) unsigned char tile_raw[];
+    float4* sm = reinterpret_cast<float4*>(tile_raw);
+    __shared__ TileSh S;
+    verlet_layout(tg, blockIdx.x, cs, S);
+    const int ncol = S.ncol;
+    const unsigned int ib = S.cR[4][1], ie = S.cR[4][ncol - 2];
+    if (ib == ie) return;
+    if (threadIdx.x == 0) mbar_init(&S.bar, 1);
+    const bool exact_all = *wide != 0u;
+    unsigned int ph = 0;
+    // up to MAXI particles a thread and sweep; a denser tile takes further sweeps
+    constexpr int MAXI = 2;
+    const unsigned int sweep = (unsigned int)MAXI * blockDim.x;
+    for (unsigned int sb = ib; sb < ie; sb += sweep) {
+        float4 xi[MAXI];
+        int jcol[MAXI], cnt[MAXI];
+        bool dom = false;
+#pragma unroll
+        for (int m = 0; m < MAXI; ++m) {
+            const unsigned int k = sb + threadIdx.x + (unsigned int)m * blockDim.x;
+            xi[m] = k < ie ? p32[k] : make_float4(0.f, 0.f, 0.f, __int_as_float(-1));
+            cnt[m] = 0;
+            int j = 1;
+            while (j < ncol - 2 && S.cR[4][j + 1] <= k) ++j;
+            const int i = __float_as_int(xi[m].w);
+            jcol[m] = i >= 0 && i < n_dom ? j : 0;  // 0: no row (past the tile, or a ghost)
+            dom = dom || jcol[m] != 0;
+        }
+        if (!__syncthreads_or(dom ? 1 : 0)) continue;  // ghosts only; also covers the barrier's initialisation
+        for (int pass = 0; pass < 3; ++pass) {
+            const unsigned int base = S.oR[3 * pass];
+            const unsigned int tot = (pass < 2 ? S.oR[3 * pass + 3] : S.total) - base;
+            const bool staged = tot <= pcap && !exact_all;
+            if (staged && tot > 0) {
+                if (threadIdx.x < 32)
+                    stage_ranges_warp(S, 3 * pass, 3, sm, base, p32, p32, tot * (unsigned int)sizeof(float4), &S.bar);
+                const bool ok = mbar_wait_bounded(&S.bar, ph & 1u, 1u << 24);
+                if (!ok) {
+                    atomicOr(ctrl_err, ERR_TIMEOUT);
+                    mbar_wait_bounded(&S.bar, ph & 1u, 1u << 24);
+                }
+                ++ph;
+                if (!__syncthreads_and(ok ? 1 : 0)) return;
+            }
+#pragma unroll
+            for (int m = 0; m < MAXI; ++m) {
+                const int j = jcol[m];
+                if (j == 0) continue;
+                const int i = __float_as_int(xi[m].w);
+                int c = cnt[m];
+#pragma unroll 1
+                for (int r = 3 * pass; r < 3 * pass + 3; ++r) {
+                    const unsigned int a = S.cR[r][j - 1], n = S.cR[r][j + 2] - a;
+                    if (staged)
+                        verlet_seg<T, SYM>(sm + (S.oR[r] - base + (a - S.cR[r][0])), n, xi[m], i, pos, r2, lo_thr,
+                                           hi_thr, n_dom, nbr + i, stride, max_nn, c);
+                    else if (exact_all)
+                        verlet_seg_wide<T, SYM>(p32 + a, n, i, pos, r2, n_dom, nbr + i, stride, max_nn, c);
+                    else
+                        verlet_seg<T, SYM>(p32 + a, n, xi[m], i, pos, r2, lo_thr, hi_thr, n_dom, nbr + i, stride,
+                                           max_nn, c);
+                }
+                cnt[m] = c;
+            }
+            // every thread is done with this layer before the next one is copied over it
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
+#pragma unroll
+        for (int m = 0; m < MAXI; ++m) {
+            if (jcol[m] == 0) continue;
+            int c = cnt[m];
+            if (c > max_nn) {
+                atomicOr(ctrl_err, ERR_NN_OVERFLOW);
+                atomicMax(ctrl_nnmax, (unsigned int)c);
+                c = max_nn;
+            }
+            nn[__float_as_int(xi[m].w)] = c;
+        }
+    }
+}
+
+// Tile width: about a CTA's 128 threads of particles on average, at most 16 cells
+// (dense tiles of a sparse system otherwise outgrow the staging), narrower where
+// that leaves the GPU's 148 SMs with less than four tiles each.
+static int choose_tx(pd_cl cl, long n_all) {
+    const double cells = (double)cl->div[0] * cl->div[1] * cl->div[2];
+    const double occ = std::max(cells > 0 ? (double)n_all / cells : 1.0, 1e-3);
+    const long rows = (long)(cl->gs[1] - 2 * cl->pad) * (cl->gs[2] - 2 * cl->pad);
+    const int nxi = cl->gs[0] - 2 * cl->pad;
+    int tx = (int)std::min(16.0, 124.0 / occ);
+    const long want = 4 * 148;
+    if (rows * ((nxi + std::max(tx, 1) - 1) / std::max(tx, 1)) < want) tx = std::min(tx, (int)((long)nxi * rows / want));
+    return std::max(1, std::min(tx, nxi));
+}
+
+template <class T>
+static int verlet_rows(pd_vd h, pd_vl vl, const float4* p32, const TileGeom& tg, long ntiles, long n_dom, long stride,
+                       const unsigned int* wide, cudaStream_t st) {
+    typedef typename V4<T>::type T4;
+    pd_cl cl = vl->cl;
+    // staging of a z-layer: 1536 records (24 KB, nine CTAs per SM)
+    const unsigned int pcap = 1536;
+    const T rc = (T)vl->r_cut;
+    const T r2 = rc * rc;
+    // FP32 positions are staged as they are: their band is empty
+    const double band = sizeof(T) == 8 ? fp32_band_at(verlet_bound(cl), vl->r_cut) : 0.0;
+    const float lo_thr = sizeof(T) == 8 ? (float)((double)r2 - band) : (float)r2;
+    const float hi_thr = sizeof(T) == 8 ? (float)((double)r2 + band) : (float)r2;
+    auto go = [&](auto k) {
+        pd::launch(k, (unsigned)ntiles, TBLOCK, pcap * sizeof(float4), st, (const T4*)h->pos, p32, tg,
+                   (const unsigned int*)cl->cell_start.as<unsigned int>(), n_dom, r2, lo_thr, hi_thr, vl->nbr.as<int>(),
+                   vl->nn.as<int>(), stride, vl->max_nn, pcap, wide, &h->ctrl->err, &h->ctrl->nn_max);
+    };
+    if (vl->sym) go(k_verlet_rows<T, true>);
+    else go(k_verlet_rows<T, false>);
+    PD_LAUNCH_CHECK();
     return PD_OK;
 }
 
@@ -162,16 +293,18 @@ int verlet_build(pd_vd h, pd_vl vl, long n_dom, const unsigned int* n_img_dev, c
     pd_cl cl = vl->cl;
     long n_all_bound = n_img_dev ? h->cap : h->n_total;
     PD_TRY(cl_build(h, cl, n_all_bound, n_img_dev, st));
-    // cell-ordered positions with original indices
-    PD_TRY(h->tmp.ensure((size_t)(n_all_bound > 0 ? n_all_bound : 1) * h->pos_bytes));
+    // cell-ordered FP32 copies with original indices; the flag word of out-of-range
+    // coordinates lies behind the cell counts, which cl_build cleared
+    PD_TRY(h->tmp.ensure((size_t)(n_all_bound > 0 ? n_all_bound : 1) * sizeof(float4)));
     const unsigned int* cs_end = cl->cell_start.as<unsigned int>() + cl->ncells;
+    unsigned int* wide = cl->cell_cnt.as<unsigned int>() + cl->ncells + 1;
     unsigned g = grid_for(n_all_bound, 256);
     if (h->dtype == PD_F64)
         pd::launch(k_gather_cs<double>, g, 256, 0, st, (const double4*)h->pos, cl->sorted.as<int>(), cs_end,
-                                               h->tmp.as<double4>(), n_all_bound);
-    else
+                                               h->tmp.as<float4>(), n_all_bound, verlet_bound(cl), wide);
+    else  // staged as they are: nothing is out of range
         pd::launch(k_gather_cs<float>, g, 256, 0, st, (const float4*)h->pos, cl->sorted.as<int>(), cs_end,
-                                              h->tmp.as<float4>(), n_all_bound);
+                                              h->tmp.as<float4>(), n_all_bound, INFINITY, wide);
     PD_LAUNCH_CHECK();
     long stride = ((n_dom + 31) / 32) * 32;
     if (stride < 32) stride = 32;
@@ -189,55 +322,13 @@ int verlet_build(pd_vd h, pd_vl vl, long n_dom, const unsigned int* n_img_dev, c
         vl->stride = stride;
         vl->n_dom = n_dom;
         if (n_dom > 0) {
-            int TX;
-            choose_tx(cl, h->n_total > 0 ? h->n_total : h->n_real, TX);
-            int nxi = cl->gs[0] - 2 * cl->pad;
-            int ntx = (nxi + TX - 1) / TX;
-            long ntiles = (long)ntx * (cl->gs[1] - 2 * cl->pad) * (cl->gs[2] - 2 * cl->pad);
-            int smem_bytes = 64 * 1024;
-            int smem_cap = smem_bytes / h->pos_bytes;
-            if (h->dtype == PD_F64) {
-                static bool attr = false;
-                if (!attr) {
-                    cudaFuncSetAttribute(k_verlet_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-                    attr = true;
-                }
-                pd::launch(k_verlet_tile<double>, (unsigned)ntiles, 128, smem_bytes, st, 
-                    h->tmp.as<double4>(), [&] {
-                        Grid<double> G;
-                        for (int d = 0; d < 3; ++d) {
-                            G.lo[d] = cl->box_lo[d];
-                            G.sp[d] = cl->spacing[d];
-                            G.gs[d] = cl->gs[d];
-                        }
-                        G.pad = cl->pad;
-                        return G;
-                    }(),
-                    TX, ntx, cl->cell_start.as<unsigned int>(), n_dom, (double)(vl->r_cut * vl->r_cut),
-                    vl->nbr.as<int>(), vl->nn.as<int>(), stride, vl->max_nn, smem_cap, vl->sym ? 1 : 0,
-                    &h->ctrl->err, &h->ctrl->nn_max);
-            } else {
-                static bool attr = false;
-                if (!attr) {
-                    cudaFuncSetAttribute(k_verlet_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-                    attr = true;
-                }
-                float rc = (float)vl->r_cut;
-                pd::launch(k_verlet_tile<float>, (unsigned)ntiles, 128, smem_bytes, st, 
-                    h->tmp.as<float4>(), [&] {
-                        Grid<float> G;
-                        for (int d = 0; d < 3; ++d) {
-                            G.lo[d] = (float)cl->box_lo[d];
-                            G.sp[d] = (float)cl->spacing[d];
-                            G.gs[d] = cl->gs[d];
-                        }
-                        G.pad = cl->pad;
-                        return G;
-                    }(),
-                    TX, ntx, cl->cell_start.as<unsigned int>(), n_dom, rc * rc, vl->nbr.as<int>(), vl->nn.as<int>(),
-                    stride, vl->max_nn, smem_cap, vl->sym ? 1 : 0, &h->ctrl->err, &h->ctrl->nn_max);
-            }
-            PD_LAUNCH_CHECK();
+            // a particle outside the grid (never mapped) lies in no tile: its row is empty
+            PD_CUDA(cudaMemsetAsync(vl->nn.p, 0, sizeof(int) * (size_t)n_dom, st));
+            TileGeom tg;
+            long ntiles = 0;
+            PD_TRY(tile_plan(cl, n_dom, choose_tx(cl, h->n_total > 0 ? h->n_total : h->n_real), tg, ntiles));
+            if (h->dtype == PD_F64) PD_TRY(verlet_rows<double>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, wide, st));
+            else PD_TRY(verlet_rows<float>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, wide, st));
         }
         if (!check) return PD_OK;
         PD_TRY(read_ctrl(h, st));
