@@ -70,6 +70,23 @@ __device__ __forceinline__ float div_by(float a, float x) {
     return fmaf(e, ay, ay);
 }
 
+// 1/sqrt(x) of a normal positive x from the hardware approximation y0: with
+// e = 1 - x y0^2, x^-1/2 = y0 (1 - e)^-1/2 = y0 (1 + e/2 + 3/8 e^2 + ...) (binomial
+// series); e is below 2^-19 (FP64) and 2^-21 (FP32), so the terms kept leave an error
+// below the type's rounding.  An overflowed x keeps y0 = 0, as a division would give.
+__device__ __forceinline__ double rsqrt_series(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = x <= 1.7976931348623157e308 ? fma(-x * y, y, 1.0) : 0.0;
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float rsqrt_series(float x) {
+    float y;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float e = x <= 3.402823466e38f ? fmaf(-x * y, y, 1.0f) : 0.0f;
+    return fmaf(0.5f * y, e, y);
+}
+
 template <class T>
 __device__ __forceinline__ void lj_acc(const LJP<T>& P, T r2, T dx, T dy, T dz, T& fx, T& fy, T& fz, T& e, T& w) {
     T ir2 = recip(r2);
