@@ -140,7 +140,7 @@ int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cud
         PD_LAUNCH_CHECK();
     }
     PD_TRY(scan_u32(cl->cell_cnt.as<unsigned int>(), cl->cell_start.as<unsigned int>(), nc + 1, nullptr,
-                    h->scan_scratch, st));
+                    h->scan_scratch, st, &h->ctrl->err));
     if (n_part > 0) {
         unsigned g = grid_for(n_part, 256);
         pd::launch(k_cl_scatter, g, 256, 0, st, n_part, n_part_dev, n_add, cl->cell_of.as<unsigned int>(),
@@ -156,7 +156,7 @@ int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cud
     return PD_OK;
 }
 
-// reorder: dst[k] = src[sorted[k]] (gather, coalesced writes) for positions, gid and properties
+// gather: dst[k] = src[ids[k]] of one column
 template <class T>
 __global__ void k_gather4(const typename V4<T>::type* __restrict__ src, typename V4<T>::type* __restrict__ dst,
                           const int* __restrict__ ids, long n) {
@@ -209,58 +209,72 @@ __global__ void k_gather_cols(const int* __restrict__ ids, long n, GatherCols G)
     }
 }
 
-// restore: dst[sorted[k]] = src[k]
-template <class T>
-__global__ void k_scatter4(const typename V4<T>::type* __restrict__ src, typename V4<T>::type* __restrict__ dst,
-                           const int* __restrict__ ids, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        st4(dst, ids[k], ld4(src, k));
-}
-template <class E>
-__global__ void k_scatter(const E* __restrict__ src, E* __restrict__ dst, const int* __restrict__ ids, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        dst[ids[k]] = src[k];
+// Columns moved element by element: MODE 0 gather dst[k] = src[ids[k]], 1 scatter
+// dst[ids[k]] = src[k], 2 copy dst[k] = src[k] (columns need not start on 16 bytes, so
+// a copy moves elements too, coalesced all the same).
+template <int MODE> __global__ void k_move_cols(const int* __restrict__ ids, long n, GatherCols G) {
+    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
+        const long id = MODE == 2 ? k : (long)ids[k];
+        const long from = MODE == 1 ? k : id, to = MODE == 1 ? id : k;
+        for (int c = 0; c < G.ncol; ++c) {
+            const int es = G.esize[c];
+            if (es == 32) {
+                const double2* s2 = reinterpret_cast<const double2*>(G.src[c]) + 2 * from;
+                double2* d2 = reinterpret_cast<double2*>(G.dst[c]) + 2 * to;
+                const double2 a = __ldg(s2), b = __ldg(s2 + 1);
+                d2[0] = a;
+                d2[1] = b;
+            } else if (es == 16) {
+                reinterpret_cast<double2*>(G.dst[c])[to] = __ldg(reinterpret_cast<const double2*>(G.src[c]) + from);
+            } else if (es == 8) {
+                reinterpret_cast<long long*>(G.dst[c])[to] = __ldg(reinterpret_cast<const long long*>(G.src[c]) + from);
+            } else {
+                reinterpret_cast<int*>(G.dst[c])[to] = __ldg(reinterpret_cast<const int*>(G.src[c]) + from);
+            }
+        }
+    }
 }
 
+// Permutation in place (the storage keeps its addresses): up to GCOLS columns move into
+// scratch in one kernel and back in another.  A kernel and a copy for each column were
+// bound by their launches on small systems: 4,099 FP64 particles, reorder and
+// restoreOrder of four columns together 41 us of GPU time in 20 launches.
 static int permute(pd_vd h, const int* ids, long n, unsigned long prop_mask, bool with_pos, bool with_gid,
                    bool restore, cudaStream_t st) {
     if (n <= 0) return PD_OK;
-    unsigned g = grid_for(n, 256);
-    size_t maxb = (size_t)n * h->pos_bytes;
-    for (auto& P : h->props) maxb = std::max(maxb, (size_t)n * P.esize);
-    PD_TRY(h->tmp2.ensure(maxb));
-    if (with_pos) {
-        if (h->dtype == PD_F64) {
-            if (restore) pd::launch(k_scatter4<double>, g, 256, 0, st, (const double4*)h->pos, h->tmp2.as<double4>(), ids, n);
-            else pd::launch(k_gather4<double>, g, 256, 0, st, (const double4*)h->pos, h->tmp2.as<double4>(), ids, n);
-        } else {
-            if (restore) pd::launch(k_scatter4<float>, g, 256, 0, st, (const float4*)h->pos, h->tmp2.as<float4>(), ids, n);
-            else pd::launch(k_gather4<float>, g, 256, 0, st, (const float4*)h->pos, h->tmp2.as<float4>(), ids, n);
-        }
-        PD_LAUNCH_CHECK();
-        PD_CUDA(cudaMemcpyAsync(h->pos, h->tmp2.p, (size_t)n * h->pos_bytes, cudaMemcpyDeviceToDevice, st));
-    }
-    if (with_gid) {
-        if (restore) pd::launch(k_scatter<int>, g, 256, 0, st, h->gid, h->tmp2.as<int>(), ids, n);
-        else pd::launch(k_gather<int>, g, 256, 0, st, h->gid, h->tmp2.as<int>(), ids, n);
-        PD_LAUNCH_CHECK();
-        PD_CUDA(cudaMemcpyAsync(h->gid, h->tmp2.p, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-    }
+    struct Col {
+        char* p;
+        int es;
+    };
+    std::vector<Col> cols;
+    if (with_pos) cols.push_back({(char*)h->pos, (int)h->pos_bytes});
+    if (with_gid) cols.push_back({(char*)h->gid, 4});
     for (size_t p = 0; p < h->props.size(); ++p) {
         if (!(prop_mask & (1ul << p))) continue;
         Prop& P = h->props[p];
-        for (int c = 0; c < P.ncomp; ++c) {
-            char* base = P.d + (size_t)c * h->cap * P.esize;
-            if (P.esize == 8) {
-                if (restore) pd::launch(k_scatter<long long>, g, 256, 0, st, (const long long*)base, h->tmp2.as<long long>(), ids, n);
-                else pd::launch(k_gather<long long>, g, 256, 0, st, (const long long*)base, h->tmp2.as<long long>(), ids, n);
-            } else {
-                if (restore) pd::launch(k_scatter<int>, g, 256, 0, st, (const int*)base, h->tmp2.as<int>(), ids, n);
-                else pd::launch(k_gather<int>, g, 256, 0, st, (const int*)base, h->tmp2.as<int>(), ids, n);
-            }
-            PD_LAUNCH_CHECK();
-            PD_CUDA(cudaMemcpyAsync(base, h->tmp2.p, (size_t)n * P.esize, cudaMemcpyDeviceToDevice, st));
+        for (int c = 0; c < P.ncomp; ++c) cols.push_back({P.d + (size_t)c * h->cap * P.esize, P.esize});
+    }
+    const unsigned g = grid_for(n, 256);
+    auto room = [&](size_t c) { return ((size_t)n * cols[c].es + 255) & ~(size_t)255; };  // aligned scratch columns
+    for (size_t c0 = 0; c0 < cols.size(); c0 += GCOLS) {
+        const size_t c1 = std::min(cols.size(), c0 + (size_t)GCOLS);
+        size_t bytes = 0;
+        for (size_t c = c0; c < c1; ++c) bytes += room(c);
+        PD_TRY(h->tmp2.ensure(bytes));
+        GatherCols out{}, back{};
+        out.ncol = back.ncol = (int)(c1 - c0);
+        char* t = h->tmp2.as<char>();
+        for (size_t c = c0; c < c1; ++c) {
+            out.src[c - c0] = back.dst[c - c0] = cols[c].p;
+            out.dst[c - c0] = t;
+            back.src[c - c0] = t;
+            out.esize[c - c0] = back.esize[c - c0] = cols[c].es;
+            t += room(c);
         }
+        if (restore) pd::launch(k_move_cols<1>, g, 256, 0, st, ids, n, out);
+        else pd::launch(k_move_cols<0>, g, 256, 0, st, ids, n, out);
+        pd::launch(k_move_cols<2>, g, 256, 0, st, (const int*)nullptr, n, back);
+        PD_LAUNCH_CHECK();
     }
     return PD_OK;
 }
@@ -353,15 +367,11 @@ int cl_reorder(pd_vd h, pd_cl cl, long n_part, unsigned long prop_mask, bool wit
 }
 
 // sorted slots of the domain particles, in sorted order (getDomainSortIds)
-__global__ void k_dom_flags(const int* __restrict__ sorted, long n, long gm, unsigned int* __restrict__ f) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        f[k] = sorted[k] < gm ? 1u : 0u;
-}
-__global__ void k_dom_compact(const int* __restrict__ sorted, long n, long gm, const unsigned int* __restrict__ pos,
-                              int* __restrict__ out) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        if (sorted[k] < gm) out[pos[k]] = (int)k;
-}
+struct DomSlot {
+    const int* sorted;
+    long gm;
+    __device__ __forceinline__ bool operator()(long k) const { return sorted[k] < gm; }
+};
 
 // the reference's calculate_force / calculate_force_sort: L lanes share a particle and
 // take the candidates of its cell rows (2r + 1 cells along x, contiguous in the cell
@@ -479,7 +489,6 @@ int pd_celllist_destroy(pd_cl cl) {
     cl->cell_of.release();
     cl->slot.release();
     cl->dom_sort.release();
-    cl->flags.release();
     delete cl;
     return PD_OK;
 }
@@ -490,15 +499,14 @@ int pd_celllist_update(pd_vd h, pd_cl cl, unsigned long prop_mask, void* stream)
     long n = h->n_total;
     PD_TRY(cl_build(h, cl, n, nullptr, st));
     // getDomainSortIds: sorted slots holding domain particles
-    PD_TRY(cl->flags.ensure(sizeof(unsigned int) * (n + 1)));
     PD_TRY(cl->dom_sort.ensure(sizeof(int) * (n + 1)));
     if (n > 0) {
-        unsigned g = grid_for(n, 256);
-        pd::launch(k_dom_flags, g, 256, 0, st, cl->sorted.as<int>(), n, h->n_real, cl->flags.as<unsigned int>());
-        PD_LAUNCH_CHECK();
-        PD_TRY(scan_u32(cl->flags.as<unsigned int>(), cl->slot.as<unsigned int>(), n, nullptr, h->scan_scratch, st));
-        pd::launch(k_dom_compact, g, 256, 0, st, cl->sorted.as<int>(), n, h->n_real, cl->slot.as<unsigned int>(),
-                                         cl->dom_sort.as<int>());
+        const unsigned nt = (unsigned)((n + FT_TILE - 1) / FT_TILE);
+        PD_TRY(h->tile_cnt.ensure(sizeof(unsigned int) * nt));
+        const DomSlot f{cl->sorted.as<const int>(), h->n_real};
+        pd::launch(k_flag_count<DomSlot>, nt, FT_BLOCK, 0, st, f, n, h->tile_cnt.as<unsigned int>());
+        pd::launch(k_flag_fill<DomSlot>, nt, FT_BLOCK, 0, st, f, n, (const unsigned int*)h->tile_cnt.as<unsigned int>(),
+                   cl->dom_sort.as<unsigned int>(), (unsigned int*)nullptr);
         PD_LAUNCH_CHECK();
     }
     if (cl->opt & PD_CL_GPU_REORDER) {
@@ -511,6 +519,10 @@ int pd_celllist_update(pd_vd h, pd_cl cl, unsigned long prop_mask, void* stream)
         cl->reordered = false;
     }
     PD_TRY(read_ctrl(h, st));
+    if (h->ctrl_h->err & ERR_TIMEOUT) {
+        set_error("cell list: a device wait gave up");
+        return PD_ETIMEOUT;
+    }
     if (h->ctrl_h->err & ERR_CELL_RANGE) {
         unsigned int z = 0;
         cudaMemcpy(&h->ctrl->err, &z, sizeof(z), cudaMemcpyHostToDevice);

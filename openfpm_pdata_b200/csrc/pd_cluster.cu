@@ -332,7 +332,7 @@ template <class T> static int md_run_cluster_t(pd_md md, int steps, cudaStream_t
     PD_TRY(h->img_shift.ensure(img_cap));
     PD_TRY(md->kpart.ensure(sizeof(double) * 3 * CL_CTAS + sizeof(unsigned int) * 4));
     PD_TRY(md->E.ensure(sizeof(double) * 4 * (steps + 1)));
-    if (h->nbox == 0) PD_TRY(ghost_boxes_upload(h, st));
+    PD_TRY(ghost_boxes_upload(h, st));
     ClArgs<T> A;
     memset(&A, 0, sizeof(A));
     A.pos = (typename V4<T>::type*)h->pos;

@@ -188,6 +188,182 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* a, double 
 }
 
 // ---------------------------------------------------------------------------
+// Single-pass prefix sums over tiles (decoupled look-back: Merrill & Garland, "Single-
+// pass parallel prefix scan with decoupled look-back", 2016).  A tile publishes its own
+// sum, then adds up the sums of the tiles before it until it meets one that has already
+// published its running total; flag and value share one 64-bit word, so no fence is
+// needed.  Tiles are numbered by a ticket in the order in which their CTAs start, so
+// the tiles waited for have started; the wait is bounded all the same.  The last CTA to
+// finish clears the words, so the state is all zero between launches (also under graph
+// replay) and needs clearing only when it is allocated (lookback_ensure).
+struct Lookback {
+    unsigned int ticket, done, pad[2];
+    unsigned long long word[1];  // one per tile: flag (1 own sum, 2 running total) << 32 | value
+};
+__device__ __forceinline__ unsigned int lookback_tile(Lookback* L, unsigned int* sh) {
+    if (threadIdx.x == 0) *sh = atomicAdd(&L->ticket, 1u);
+    __syncthreads();
+    return *sh;
+}
+// By the whole CTA: the sum of all tiles before `tile`, whose own sum is `agg` (the same in
+// every thread); *ok is cleared in a thread whose wait gave up.  A step looks at BLOCK
+// tiles, one a thread: the CTAs of a wave all publish at about the same time, and a
+// warp's window of 32 took a step of an L2 round trip for each 32 of them (17 us for 500
+// tiles).
+template <int BLOCK>
+__device__ __forceinline__ unsigned int lookback_sum(Lookback* L, unsigned int tile, unsigned int agg, bool* ok) {
+    constexpr int NW = BLOCK / 32;
+    __shared__ unsigned int part[NW], ends[NW];
+    volatile unsigned long long* word = L->word;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned int excl = 0;
+    if (tile > 0) {
+        if (threadIdx.x == 0) word[tile] = (1ull << 32) | agg;
+        bool found = false;
+        for (long last = (long)tile - 1; !found; last -= BLOCK) {
+            const long idx = last - (long)threadIdx.x;
+            unsigned long long v = 2ull << 32;  // before the first tile: a running total of zero
+            if (idx >= 0) {
+                unsigned int it = 0;
+                while (((v = word[idx]) >> 32) == 0ull && ++it < (1u << 24)) {
+                }
+                if ((v >> 32) == 0ull) {
+                    *ok = false;
+                    v = 2ull << 32;
+                }
+            }
+            const unsigned int full = __ballot_sync(0xffffffffu, (v >> 32) == 2ull);
+            unsigned int add = lane <= (full ? __ffs(full) - 1 : 31) ? (unsigned int)v : 0u;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+            if (lane == 0) {
+                part[w] = add;
+                ends[w] = full;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < NW; ++j) {
+                if (!found) excl += part[j];
+                found = found || ends[j] != 0u;
+            }
+            __syncthreads();
+        }
+    }
+    if (threadIdx.x == 0) word[tile] = (2ull << 32) | (unsigned long long)(excl + agg);
+    return excl;
+}
+// by the whole CTA at its end: the last one clears the state of `nt` tiles
+__device__ __forceinline__ void lookback_finish(Lookback* L, unsigned int nt, unsigned int* sh) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        *sh = atomicAdd(&L->done, 1u);
+    }
+    __syncthreads();
+    if (*sh != nt - 1) return;
+    for (unsigned int i = threadIdx.x; i < nt; i += blockDim.x) L->word[i] = 0ull;
+    if (threadIdx.x == 0) L->ticket = L->done = 0u;
+}
+
+// ---------------------------------------------------------------------------
+// Stable compaction in two kernels: one counts each tile's elements, the other adds up
+// the counts of the tiles before its own (a few words a thread, from L2) and writes.
+// Where a pass needs thousands of tiles this beats a look-back: 1000 tiles of int marks
+// 31 us by look-back (the polling of a wave's CTAs congests the words they wait for).
+
+// by the whole CTA: the sum of cnt[0, tile), the same in every thread
+template <int BLOCK>
+__device__ __forceinline__ unsigned int tile_prefix(const unsigned int* __restrict__ cnt, unsigned int tile) {
+    __shared__ unsigned int part[BLOCK / 32];
+    unsigned int s = 0;
+    for (unsigned int j = threadIdx.x; j < tile; j += BLOCK) s += cnt[j];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    s = 0;
+#pragma unroll
+    for (int j = 0; j < BLOCK / 32; ++j) s += part[j];
+    __syncthreads();
+    return s;
+}
+
+// Offsets of a tile's flagged items: item k of thread t is element base + k * BLOCK + t,
+// flagged in bit k of `flags`; off[k] receives `excl` plus the number of flagged elements
+// of the tile before it, *total `excl` plus all of them.  Warp ballots, one scan of the
+// tile's ITEMS * BLOCK / 32 counts by the first warp.
+template <int BLOCK, int ITEMS>
+__device__ __forceinline__ void tile_offsets(unsigned int flags, unsigned int excl, unsigned int (&off)[ITEMS],
+                                             unsigned int* total) {
+    constexpr int NW = BLOCK / 32, NC = ITEMS * NW, PER = (NC + 31) / 32;
+    __shared__ unsigned int cnt[PER * 32], sum;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned int bal[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        bal[k] = __ballot_sync(0xffffffffu, flags >> k & 1u);
+        if (lane == 0) cnt[k * NW + w] = __popc(bal[k]);
+    }
+    __syncthreads();
+    if (w == 0) {
+        unsigned int v[PER], s = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            v[j] = lane * PER + j < NC ? cnt[lane * PER + j] : 0u;
+            s += v[j];
+        }
+        unsigned int incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) sum = incl;
+        unsigned int run = incl - s;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            cnt[lane * PER + j] = run;
+            run += v[j];
+        }
+    }
+    __syncthreads();
+    *total = excl + sum;
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) off[k] = excl + cnt[k * NW + w] + __popc(bal[k] & ((1u << lane) - 1u));
+}
+
+// ascending elements i < n with f(i): tile counts, then the elements at their offsets
+static constexpr int FT_BLOCK = 512, FT_ITEMS = 8;
+static constexpr long FT_TILE = (long)FT_BLOCK * FT_ITEMS;
+template <class F> __device__ __forceinline__ unsigned int tile_flags(const F& f, long n, long base) {
+    unsigned int flags = 0;
+#pragma unroll
+    for (int k = 0; k < FT_ITEMS; ++k) {
+        const long i = base + (long)k * FT_BLOCK + threadIdx.x;
+        if (i < n && f(i)) flags |= 1u << k;
+    }
+    return flags;
+}
+template <class F> __global__ void __launch_bounds__(FT_BLOCK) k_flag_count(F f, long n, unsigned int* __restrict__ cnt) {
+    const unsigned int c =
+        block_sum<unsigned int, FT_BLOCK>(__popc(tile_flags(f, n, (long)blockIdx.x * FT_TILE)));
+    if (threadIdx.x == 0) cnt[blockIdx.x] = c;
+}
+template <class F>
+__global__ void __launch_bounds__(FT_BLOCK) k_flag_fill(F f, long n, const unsigned int* __restrict__ cnt,
+                                                        unsigned int* __restrict__ out,
+                                                        unsigned int* __restrict__ total) {
+    const long base = (long)blockIdx.x * FT_TILE;
+    const unsigned int flags = tile_flags(f, n, base);
+    unsigned int off[FT_ITEMS], tot;
+    tile_offsets<FT_BLOCK, FT_ITEMS>(flags, tile_prefix<FT_BLOCK>(cnt, blockIdx.x), off, &tot);
+    if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1 && total) *total = tot;
+#pragma unroll
+    for (int k = 0; k < FT_ITEMS; ++k)
+        if (flags >> k & 1u) out[off[k]] = (unsigned int)(base + (long)k * FT_BLOCK + threadIdx.x);
+}
+
+// ---------------------------------------------------------------------------
 // 1-D bulk copies global -> shared through the TMA engine (cp.async.bulk, no
 // tensor map, no multicast) completing on an mbarrier.  Addresses and sizes must
 // be multiples of 16 bytes (positions are 16- or 32-byte records).

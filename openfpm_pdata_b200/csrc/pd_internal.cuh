@@ -17,6 +17,8 @@ void set_error(const char* fmt, ...);
 // PD_OK when p is device (or managed) memory of the current device; else PD_EINVAL
 // with a message naming `who` and `what`.  Neither allocates nor synchronises.
 int check_device_ptr(const void* p, const char* who, const char* what);
+// p is plain device memory of the current device (kernels may read and write it directly)
+bool on_this_device(const void* p);
 
 #define PD_CUDA(call)                                                                                   \
     do {                                                                                                \
@@ -102,11 +104,12 @@ inline int type_size(int t) {
     }
 }
 
-// exclusive scan, in place, of nb per-block partial counts (one block); the total to *total_dev
-int scan_partials(unsigned int* part, long nb, unsigned int* total_dev, cudaStream_t st);
-// exclusive scan of n uint32 values (in may equal out); writes the total to *total_dev
+// room for the look-back state of `nt` tiles in `b`, cleared when it is (re)allocated
+int lookback_ensure(Buf& b, long nt, cudaStream_t st);
+// exclusive scan of n uint32 values (in may equal out); writes the total to *total_dev;
+// ERR_TIMEOUT into *err if a wait gave up
 int scan_u32(const unsigned int* in, unsigned int* out, long n, unsigned int* total_dev, Buf& scratch,
-             cudaStream_t st);
+             cudaStream_t st, unsigned int* err);
 
 inline unsigned int grid_for(long n, int block, long cap_blocks = 148L * 64) {
     long g = (n + block - 1) / block;
@@ -143,8 +146,10 @@ struct pd_vd_s {
     std::vector<pd::Prop> props;
     // periodic images (o_part_loc): source slot and shift id of each ghost
     pd::Buf img_src, img_shift, img_cnt, img_start;
+    pd::Buf img_list;  // ghost_get: images found, (particle, box), tile by tile
     pd::Buf boxes, box_sv, shifts;  // device copies of the local ghost boxes
-    int nbox = 0;
+    int nbox = 0;            // boxes uploaded (0: no image can exist)
+    bool boxes_dom = false;  // boxes / shifts hold the domain's own ghost boxes
     long n_img = 0;
     bool img_valid = false;
     bool img_gen_order = false;  // images in generation order (ghost_put can fold them)
@@ -154,7 +159,7 @@ struct pd_vd_s {
     int pend_opt = 0;
     pd::Ctrl* ctrl = nullptr;    // device
     pd::Ctrl* ctrl_h = nullptr;  // pinned host mirror
-    pd::Buf scan_scratch, tmp, tmp2, red;
+    pd::Buf scan_scratch, tile_cnt, tmp, tmp2, red;
     // spare storage of the same capacity: a reorder gathers into it and swaps it in
     // (cl_reorder with swap); allocated on first use, freed with the storage
     void* spare_pos = nullptr;
@@ -183,7 +188,7 @@ struct pd_cl_s {
     int div[3], gs[3];
     double box_lo[3], spacing[3];
     long ncells = 0;
-    pd::Buf cell_start, cell_cnt, sorted, sorted_tmp, cell_of, slot, dom_sort, flags;
+    pd::Buf cell_start, cell_cnt, sorted, sorted_tmp, cell_of, slot, dom_sort;
     long n_part = 0;
     long ghost_marker = 0;
     bool reordered = false;  // the vector holds cell-ordered data until restore_order

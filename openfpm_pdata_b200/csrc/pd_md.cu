@@ -636,7 +636,7 @@ int md_rebuild(pd_md md, cudaStream_t st) {
     } else {
         PD_TRY(cl_reorder(h, sort_cl, h->n_real, md_reorder_mask(md), true, true, st, md->swap_reorder));
     }
-    if (h->nbox == 0) PD_TRY(ghost_boxes_upload(h, st));
+    PD_TRY(ghost_boxes_upload(h, st));
     PD_TRY(ghost_generate(h, 0, true, st));
     if (md->mp.use_cell_list) {
         PD_TRY(cl_build(h, md->cl, h->n_total, nullptr, st));
@@ -761,7 +761,8 @@ static std::vector<uintptr_t> cl_graph_key(pd_md md) {
                                 (uintptr_t)cl->cell_of.p, (uintptr_t)cl->slot.p, (uintptr_t)h->tmp.p,
                                 (uintptr_t)h->tmp2.p, (uintptr_t)h->img_src.p, (uintptr_t)h->img_shift.p,
                                 (uintptr_t)h->img_cnt.p, (uintptr_t)h->img_start.p, (uintptr_t)h->boxes.p,
-                                (uintptr_t)h->shifts.p, (uintptr_t)h->scan_scratch.p, (uintptr_t)md->gcl_img_cap};
+                                (uintptr_t)h->shifts.p, (uintptr_t)h->scan_scratch.p, (uintptr_t)h->tile_cnt.p,
+                                (uintptr_t)h->img_list.p, (uintptr_t)md->gcl_img_cap};
     for (auto& P : h->props) k.push_back((uintptr_t)P.d);
     return k;
 }

@@ -1426,7 +1426,7 @@ static int slot_reset(pd_srv s, SrvSlot& sl, SrvReq* r, const SrvShape& shape) {
             h->lo[d] = 0.0;
             h->hi[d] = r->L;
         }
-        h->nbox = 0;  // the ghost boxes of the new box are uploaded by the first build
+        h->boxes_dom = false;  // the ghost boxes of the new box are uploaded by the first build
         h->n_img = 0;
         PD_CUDA(cudaMemsetAsync(h->ctrl, 0, sizeof(Ctrl), s->as));
         memset(h->ctrl_h, 0, sizeof(Ctrl));
@@ -1609,6 +1609,7 @@ static int load_state(pd_srv s, SrvSlot& sl, SrvReq* r) {
     void* dst = nullptr;
     if (rc == PD_OK) {
         h->nbox = B->nb;
+        h->boxes_dom = true;
         if (!inbox) {
             memcpy(st + ox, r->x.data(), sizeof(double) * 3 * n);
             memcpy(st + ov, r->v.data(), sizeof(double) * 3 * n);

@@ -1,0 +1,147 @@
+"""The single-pass kernels (look-back between tiles) at the edges of their tiles: ghost
+images, compaction, index selection, sorted domain slots, multi-column reorders, and the
+device-array copies, all exact."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+F32, F64 = np.float32, np.float64
+
+
+@pytest.fixture(scope="module")
+def pd():
+    from openfpm_pdata_b200 import pd as _pd
+    _pd.lib()
+    return _pd
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("n,corner", [(1, True), (1023, False), (1024, False), (1025, True), (40000, False),
+                                      (20001, True)])
+def test_ghost_images(pd, orc, dtype, n, corner):
+    """Images, sources and shifts of several calls; with every particle in one corner (seven
+    images each) the first call finds far more images than it made room for."""
+    rng = np.random.default_rng(n)
+    L, g = 4.0, 0.25
+    lo, hi, bc = np.zeros(3), np.full(3, L), np.ones(3, np.int32)
+    vd = pd.VectorDist(n, lo, hi, bc, g, dtype=dtype, props=[(pd.PD_I32, 1), (pd.PD_F64, 2)])
+    a = np.arange(n, dtype=np.int32)
+    b = rng.normal(size=(n, 2))
+    for rep in range(3):
+        x = rng.uniform(0, 0.2 if corner and rep != 1 else L, size=(n, 3)).astype(dtype)
+        x = orc.wrap(x, lo.astype(dtype), hi.astype(dtype), bc)
+        vd.map()
+        vd.hostToDevicePos(x)
+        vd.hostToDeviceProp(0, a)
+        vd.hostToDeviceProp(1, b)
+        vd.ghost_get()
+        img, src, shf = orc.ghost_get(x, lo.astype(dtype), hi.astype(dtype), bc, g)
+        s, h = vd.ghost_records()
+        assert np.array_equal(s, src) and np.array_equal(h, shf)
+        assert np.array_equal(vd.deviceToHostPos()[n:], img)
+        assert np.array_equal(vd.deviceToHostProp(0)[n:], a[src])
+        assert np.array_equal(vd.deviceToHostProp(1)[n:], b[src])
+
+
+def test_ghost_boxes_after_user_boxes(pd, orc):
+    """The domain's boxes, uploaded once, come back after a call with other boxes."""
+    rng = np.random.default_rng(3)
+    lo, hi, bc = np.zeros(3), np.ones(3), np.ones(3, np.int32)
+    x = rng.random((5000, 3))
+    vd = pd.VectorDist(5000, lo, hi, bc, 0.1)
+    vd.hostToDevicePos(x)
+    vd.ghost_get()
+    _, src, _ = orc.ghost_get(x, lo, hi, bc, 0.1)
+    vd.ghost_count_boxes([[0, 0, 0]], [[0.5, 0.5, 0.5]], [0])
+    vd.ghost_get()
+    assert np.array_equal(vd.ghost_records()[0], src)
+
+
+@pytest.mark.parametrize("n", [1, 4095, 4096, 4097, 70001])
+@pytest.mark.parametrize("frac", [0.0, 0.3, 1.0])
+def test_remove_and_indexes(pd, orc, n, frac):
+    rng = np.random.default_rng(n)
+    lo, hi, bc = np.zeros(3), np.ones(3), np.ones(3, np.int32)
+    # 2 + 1 + 30 columns: more than one launch takes
+    vd = pd.VectorDist(n, lo, hi, bc, 0.1, props=[(pd.PD_I32, 1), (pd.PD_F32, 30)])
+    x, p = rng.random((n, 3)), rng.normal(size=(n, 30)).astype(F32)
+    mark = (rng.random(n) < frac).astype(np.int32)
+    vd.hostToDevicePos(x)
+    vd.hostToDeviceProp(0, mark)
+    vd.hostToDeviceProp(1, p)
+    want = np.nonzero(mark == 1)[0]
+    assert np.array_equal(vd.get_indexes_by_type(0, 1), want)
+    assert np.array_equal(vd.get_indexes_by_type(0, 1, device=True).cpu().numpy(), want)
+    assert np.array_equal(vd.get_indexes_by_type(0, 1, end=n // 2), want[want < n // 2])
+    vd.remove_marked(0)
+    keep = mark == 0
+    assert vd.size_local() == keep.sum()
+    assert np.array_equal(vd.deviceToHostPos(), x[keep])
+    assert np.array_equal(vd.deviceToHostProp(1), p[keep])
+    assert np.array_equal(vd.gid(), np.nonzero(keep)[0])
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("n", [1, 2047, 2049, 30011])
+def test_reorder_many_columns(pd, dtype, n):
+    """22 columns of 4 and 8 bytes there and back, with ghosts; the sorted domain slots."""
+    rng = np.random.default_rng(n)
+    vd = pd.VectorDist(n, np.zeros(3), np.ones(3), np.ones(3, np.int32), 0.1, dtype=dtype,
+                       props=[(pd.PD_F64, 13), (pd.PD_F32, 5), (pd.PD_I64, 2)])
+    x = rng.random((n, 3)).astype(dtype)
+    vals = [rng.normal(size=(n, 13)), rng.normal(size=(n, 5)).astype(F32), rng.integers(-9, 9, size=(n, 2))]
+    vd.hostToDevicePos(x)
+    for p, a in enumerate(vals):
+        vd.hostToDeviceProp(p, a)
+    vd.ghost_get()
+    before = [vd.deviceToHostPos(), vd.gid()] + [vd.deviceToHostProp(p) for p in range(3)]
+    cl = vd.getCellListGPU(0.1, opt=pd.CL_NON_SYMMETRIC | pd.CL_GPU_REORDER)
+    vd.updateCellListGPU(cl)
+    _, so = cl.get()
+    after = [vd.deviceToHostPos(), vd.gid()] + [vd.deviceToHostProp(p) for p in range(3)]
+    for a, b in zip(before, after):
+        assert np.array_equal(a[so], b)
+    import torch
+    view = cl.view()
+    dom = torch.empty(n, dtype=torch.int32, device="cuda")
+    import ctypes
+    ctypes.CDLL("libcudart.so.12").cudaMemcpy(ctypes.c_void_p(dom.data_ptr()), ctypes.c_void_p(view.dom_sort_ids),
+                                              ctypes.c_size_t(4 * n), ctypes.c_int(3))
+    assert np.array_equal(dom.cpu().numpy(), np.nonzero(so < n)[0])
+    vd.restoreOrder(cl)
+    for a, b in zip(before, [vd.deviceToHostPos(), vd.gid()] + [vd.deviceToHostProp(p) for p in range(3)]):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("n", [1, 1001])
+def test_device_arrays(pd, dtype, n):
+    """Device tensors in and out, whole, sliced, at offsets, strided and one element off."""
+    import torch
+    t = torch.float32 if dtype == F32 else torch.float64
+    pt = pd.PD_F32 if dtype == F32 else pd.PD_F64
+    vd = pd.VectorDist(n, np.zeros(3), np.ones(3), np.ones(3, np.int32), 0.1, dtype=dtype,
+                       props=[(pt, 3), (pd.PD_I32, 1), (pd.PD_I64, 2)])
+    g = torch.Generator(device="cuda").manual_seed(1)
+    flat = torch.rand(3 * n + 1, device="cuda", dtype=t, generator=g)
+    x = flat[1:].reshape(n, 3)  # starts one element past the allocation
+    wide = torch.rand((n, 6), device="cuda", dtype=t, generator=g)
+    v = wide[:, ::2]
+    i32 = torch.arange(n, device="cuda", dtype=torch.int32)
+    i64 = torch.arange(2 * n, device="cuda").reshape(n, 2) - n
+    vd.hostToDevicePos(x)
+    vd.hostToDeviceProp(0, v)
+    vd.hostToDeviceProp(1, i32)
+    vd.hostToDeviceProp(2, i64)
+    assert torch.equal(vd.deviceToHostPos(device=True), x)
+    assert torch.equal(vd.deviceToHostProp(0, device=True), v)
+    assert torch.equal(vd.deviceToHostProp(1, device=True), i32)
+    assert torch.equal(vd.deviceToHostProp(2, device=True), i64)
+    assert np.array_equal(vd.deviceToHostPos(), x.cpu().numpy())
+    assert np.array_equal(vd.deviceToHostProp(0), v.cpu().numpy())
+    if n > 1:
+        vd.hostToDeviceProp(0, v[:7] * 2, offset=3)
+        assert torch.equal(vd.deviceToHostProp(0, offset=2, count=9, device=True),
+                           torch.cat([v[2:3], v[:7] * 2, v[10:11]]))
+        assert torch.equal(vd.deviceToHostPos(offset=5, count=11, device=True), x[5:16])
