@@ -196,6 +196,13 @@ int pd_d2h_pos(pd_vd h, void* host_xyz, long offset, long count, void* stream);
 /* hostToDeviceProp<prp> / deviceToHostProp<prp>; host component-major [ncomp][count] */
 int pd_h2d_prop(pd_vd h, int prop, const void* host, long offset, long count, void* stream);
 int pd_d2h_prop(pd_vd h, int prop, void* host, long offset, long count, void* stream);
+/* hostToDeviceProp / deviceToHostProp / deviceToHostPos of rows [count][ncomp] in device
+ * memory of the current device, aligned to the element (PD_EINVAL otherwise): the layout
+ * of another library's device arrays, read and written in one pass.  Enqueued on
+ * `stream`, not waited for.  No counterpart in the reference. */
+int pd_h2d_prop_rows(pd_vd h, int prop, const void* dev, long offset, long count, void* stream);
+int pd_d2h_prop_rows(pd_vd h, int prop, void* dev, long offset, long count, void* stream);
+int pd_d2h_pos_rows(pd_vd h, void* dev, long offset, long count, void* stream);
 /* map(RUN_ON_DEVICE) on one process -- vector_dist.hpp:2158-2176 ->
  * vector_dist_comm.hpp:1405-1437 -> apply_bc_each_part (vector_dist_cuda_funcs.cuh:45-53):
  * drops the ghost and wraps every periodic coordinate with periodic_l. */

@@ -109,6 +109,9 @@ def lib():
             "pd_d2h_pos": ([vp, vp, lp, lp, vp], ip),
             "pd_h2d_prop": ([vp, ip, vp, lp, lp, vp], ip),
             "pd_d2h_prop": ([vp, ip, vp, lp, lp, vp], ip),
+            "pd_h2d_prop_rows": ([vp, ip, vp, lp, lp, vp], ip),
+            "pd_d2h_prop_rows": ([vp, ip, vp, lp, lp, vp], ip),
+            "pd_d2h_pos_rows": ([vp, vp, lp, lp, vp], ip),
             "pd_map": ([vp, ip, vp], ip),
             "pd_ghost_get": ([vp, ctypes.c_ulong, ip, vp], ip),
             "pd_ghost_records": ([vp, vp, vp, lp, P(ctypes.c_long)], ip),
@@ -217,6 +220,13 @@ def _check_tensor(a, dtype):
     want = torch.float64 if np.dtype(dtype) == np.float64 else torch.float32
     if a.dtype != want:
         raise TypeError("tensor of %s expected, got %s" % (want, a.dtype))
+
+
+def _finish_on_side_stream(torch):
+    """The library works on the default stream: what it has enqueued there is ordered before
+    later torch work on that stream, and waited for here when torch uses another one."""
+    if torch.cuda.current_stream().cuda_stream != 0:
+        torch.cuda.default_stream().synchronize()
 
 
 def launch_count():
@@ -397,7 +407,8 @@ class VectorDist:
             t = torch.empty((max(n, 0), 3), dtype=torch.float64 if self.dtype == np.float64 else torch.float32,
                             device="cuda")
             if n:
-                check(lib().pd_d2h_pos(self.h, ctypes.c_void_p(t.data_ptr()), int(offset), int(n), None))
+                check(lib().pd_d2h_pos_rows(self.h, ctypes.c_void_p(t.data_ptr()), int(offset), int(n), None))
+                _finish_on_side_stream(torch)
             return t
         if out is None:
             out = np.zeros((n, 3), self.dtype)
@@ -416,9 +427,15 @@ class VectorDist:
             want = getattr(torch, np.dtype(_NP[t]).name)
             if a.dtype != want:
                 raise TypeError(f"hostToDeviceProp: a {want} tensor is expected, got {a.dtype}")
-            cm = a.reshape(-1, nc).t().contiguous()
-            check(lib().pd_h2d_prop(self.h, int(p), ctypes.c_void_p(cm.data_ptr()), int(offset), int(cm.shape[1]),
-                                    None))
+            rows = a.reshape(-1, nc)
+            if a.device.index == torch.cuda.current_device():
+                rows = rows.contiguous()
+                check(lib().pd_h2d_prop_rows(self.h, int(p), ctypes.c_void_p(rows.data_ptr()), int(offset),
+                                             int(rows.shape[0]), None))
+            else:  # another device's memory is copied, not read by kernels
+                cm = rows.t().contiguous()
+                check(lib().pd_h2d_prop(self.h, int(p), ctypes.c_void_p(cm.data_ptr()), int(offset),
+                                        int(cm.shape[1]), None))
             return
         a = np.asarray(a, dtype=_NP[t]).reshape(-1, nc)
         cm = np.ascontiguousarray(a.T)
@@ -451,10 +468,13 @@ class VectorDist:
         n = (self.size_local_with_ghost() if with_ghost else self.size_local()) - offset if count is None else count
         if device:
             import torch
-            cm = torch.empty((nc, max(n, 0)), dtype=getattr(torch, np.dtype(_NP[t]).name), device="cuda")
+            shape = (max(n, 0), nc) if nc > 1 else (max(n, 0),)
+            rows = torch.empty(shape, dtype=getattr(torch, np.dtype(_NP[t]).name), device="cuda")
             if n:
-                check(lib().pd_d2h_prop(self.h, int(p), ctypes.c_void_p(cm.data_ptr()), int(offset), int(n), None))
-            return cm.t().contiguous() if nc > 1 else cm[0].clone()
+                check(lib().pd_d2h_prop_rows(self.h, int(p), ctypes.c_void_p(rows.data_ptr()), int(offset), int(n),
+                                             None))
+                _finish_on_side_stream(torch)
+            return rows
         cm = np.zeros((nc, n), _NP[t])
         if n:
             check(lib().pd_d2h_prop(self.h, int(p), _ptr(cm), int(offset), int(n), None))
