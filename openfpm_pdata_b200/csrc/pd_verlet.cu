@@ -152,11 +152,12 @@ __device__ __noinline__ void verlet_seg_wide(const float4* __restrict__ c4, unsi
 // Bound by the instructions of the candidate tests (27 cells hold about 6.4 times
 // the pairs kept), so: FP32 tests on 16-byte staged copies, sign bits shifted into
 // accept masks, the rare candidates within the rounding band decided exactly in the
-// position type (the scheme of the integrator's row build); one z-layer of three cell
-// rows staged at a time, so that nine CTAs fit an SM.  A layer beyond `pcap` records
-// is read from global memory instead.
-// Measured: 1,000,000 FP64 particles of a lattice (49 entries a row) 1198 -> 530 us, half
-// rows of 200,001 348 -> 171 us against FP64 records of all nine rows staged at once.
+// position type (the scheme of the integrator's row build).  The neighbourhood is staged
+// at once where it fits `pcap` records (eight CTAs per SM), so that a CTA's warps wait for
+// each other once; else one z-layer of three cell rows at a time; a layer beyond `pcap`
+// records is read from global memory instead.
+// Measured: 1,000,000 FP64 particles of a lattice (49 entries a row) 1198 -> 520 us, half
+// rows of 200,001 348 -> 165 us against FP64 records of all nine rows staged at once.
 template <class T, bool SYM>
 __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>::type* __restrict__ pos,
                                                         const float4* __restrict__ p32, TileGeom tg,
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
     if (threadIdx.x == 0) mbar_init(&S.bar, 1);
     const bool exact_all = *wide != 0u;
     unsigned int ph = 0;
+    bool held = false;  // the whole neighbourhood is staged
     // up to MAXI particles a thread and sweep; a denser tile takes further sweeps
     constexpr int MAXI = 2;
     const unsigned int sweep = (unsigned int)MAXI * blockDim.x;
@@ -195,19 +197,22 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
             dom = dom || jcol[m] != 0;
         }
         if (!__syncthreads_or(dom ? 1 : 0)) continue;  // ghosts only; also covers the barrier's initialisation
-        for (int pass = 0; pass < 3; ++pass) {
-            const unsigned int base = S.oR[3 * pass];
-            const unsigned int tot = (pass < 2 ? S.oR[3 * pass + 3] : S.total) - base;
+        // the whole neighbourhood in one pass where it fits the staging, else a z-layer a pass
+        const int layers = S.total <= pcap ? 9 : 3;  // rows a pass
+        for (int r0 = 0; r0 < 9; r0 += layers) {
+            const unsigned int base = S.oR[r0];
+            const unsigned int tot = (r0 + layers < 9 ? S.oR[r0 + layers] : S.total) - base;
             const bool staged = tot <= pcap && !exact_all;
-            if (staged && tot > 0) {
+            if (staged && tot > 0 && (layers < 9 || !held)) {
                 if (threadIdx.x < 32)
-                    stage_ranges_warp(S, 3 * pass, 3, sm, base, p32, p32, tot * (unsigned int)sizeof(float4), &S.bar);
+                    stage_ranges_warp(S, r0, layers, sm, base, p32, p32, tot * (unsigned int)sizeof(float4), &S.bar);
                 const bool ok = mbar_wait_bounded(&S.bar, ph & 1u, 1u << 24);
                 if (!ok) {
                     atomicOr(ctrl_err, ERR_TIMEOUT);
                     mbar_wait_bounded(&S.bar, ph & 1u, 1u << 24);
                 }
                 ++ph;
+                held = layers == 9;
                 if (!__syncthreads_and(ok ? 1 : 0)) return;
             }
 #pragma unroll
@@ -217,7 +222,7 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
                 const int i = __float_as_int(xi[m].w);
                 int c = cnt[m];
 #pragma unroll 1
-                for (int r = 3 * pass; r < 3 * pass + 3; ++r) {
+                for (int r = r0; r < r0 + layers; ++r) {
                     const unsigned int a = S.cR[r][j - 1], n = S.cR[r][j + 2] - a;
                     if (staged)
                         verlet_seg<T, SYM>(sm + (S.oR[r] - base + (a - S.cR[r][0])), n, xi[m], i, pos, r2, lo_thr,
@@ -230,9 +235,11 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
                 }
                 cnt[m] = c;
             }
-            // every thread is done with this layer before the next one is copied over it
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
+            if (layers < 9) {
+                // every thread is done with this layer before the next one is copied over it
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncthreads();
+            }
         }
 #pragma unroll
         for (int m = 0; m < MAXI; ++m) {
@@ -267,7 +274,7 @@ static int verlet_rows(pd_vd h, pd_vl vl, const float4* p32, const TileGeom& tg,
                        const unsigned int* wide, cudaStream_t st) {
     typedef typename V4<T>::type T4;
     pd_cl cl = vl->cl;
-    // staging of a z-layer: 1536 records (24 KB, nine CTAs per SM)
+    // staging: 1536 records (24 KB, eight CTAs per SM)
     const unsigned int pcap = 1536;
     const T rc = (T)vl->r_cut;
     const T r2 = rc * rc;
