@@ -555,12 +555,18 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         // images only).  A CTA of 256 threads at two lanes a particle takes 128 in a
         // first round; a second round of up to 64 runs at four lanes each, so most
         // lanes are busy in both while tiles stay below 192 (the rows are about
-        // equally long).
+        // equally long).  Fewer particles a tile, down to 40, where 184 would leave the
+        // 148 SMs with less than two tiles each: 30,000 FP64 particles, force 22 us at 6
+        // cells (101 a tile), 29 us at 12.
         double inner = 1;
         for (int d = 0; d < 3; ++d) inner *= std::max(1.0, (h->hi[d] - h->lo[d]) / cl->spacing[d]);
         const double occ = std::max((double)n / inner, 1e-3);
-        tx_req = std::max(1, std::min(TXMAX, (int)(184.0 / occ)));
+        const double want = std::min(184.0, std::max(40.0, (double)n / (2 * 148)));
+        tx_req = std::max(1, std::min(TXMAX, (int)(want / occ)));
     }
+    const bool narrow = md->tile_tx == 0 && md->physics == 0 && h->dtype == PD_F64;
+    const int tx_auto = tx_req;
+    if (narrow && md->fit_req == tx_auto) tx_req = md->fit_tx;  // as the build before found it
     PD_TRY(tile_plan(cl, n, tx_req, md->tg, md->ntiles));
     unsigned int tmax = 0, cmax = 0;
     for (;;) {
@@ -571,12 +577,35 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         if (md->tg.TX <= 1) return PD_OK;  // stays on global rows
         PD_TRY(tile_plan(cl, n, md->tg.TX / 2, md->tg, md->ntiles));
     }
+    if (narrow) {
+        // An uneven system: every tile's CTA takes the shared memory of the densest one, so
+        // a width from the mean occupancy costs residency.  Narrower tiles until the
+        // densest leaves the CTAs that the registers allow (four of the FP64 kernel's with
+        // 24-byte records; of the precision form's with 16 one more than its five, which
+        // measured best), but not below half
+        // the width: tiles of few particles cost more than residency.  The next build
+        // starts from the width found.  1,000,003 particles in clusters, mean width 32:
+        // precision form 494 us at 32 cells, 371 at 18, 408 at 11; FP64 315, 291, 377.
+        const long target = md->mixed ? (227 * 1024 / 6 - 4608) / 16 : (227 * 1024 / 4 - 4608) / 24;
+        int tx = md->tg.TX;
+        if ((long)tmax > target) tx = std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)tmax) - 2);
+        else if (tx < tx_auto && (long)tmax * 5 < target * 4) tx = tx_auto;  // the densest part thinned out
+        md->fit_req = tx_auto;
+        if (tx != md->tg.TX && tx >= 1 && tx <= tx_auto) {
+            PD_TRY(tile_plan(cl, n, tx, md->tg, md->ntiles));
+            PD_TRY(tile_sizes(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), tmax, cmax,
+                              st));
+        }
+        md->fit_tx = md->tg.TX;
+    }
     if (md->tile_tx == 0 && md->physics == 1 && md->tg.TX > 1) {
-        // automatic width for SPH: the densest tile's two staged records within about
-        // 60 KB in FP64 (tiles of two or more cells, three CTAs per SM) or 48 KB in
-        // FP32; the mean occupancy counts the empty part of the tank, so the width
-        // is rescaled from the measured largest tile
-        const long target = (h->dtype == PD_F64 ? 60L : 48L) * 1024 / (2L * h->pos_bytes);
+        // automatic width for SPH: the densest tile within about 1730 staged particles (two
+        // records each; five cells of a filled tank): fewer, wider tiles stage less per
+        // particle, which counts for more than residency.  FP64, dp = 1/128: rates 608 us
+        // at two cells (three CTAs per SM), 576 at five (two); FP32, dp = 1/180: 733 us at
+        // four cells, 659 at five, 754 at six.  The mean occupancy counts the empty part
+        // of the tank, so the width is rescaled from the measured largest tile
+        const long target = 1730;
         if ((long)tmax > target) {
             int tx = (int)((double)(md->tg.TX + 2) * (double)target / (double)tmax) - 2;
             if (tx < 1) tx = 1;

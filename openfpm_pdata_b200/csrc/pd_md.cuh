@@ -20,6 +20,7 @@ struct pd_md_s {
     bool ready = false;
     // tiled neighbour structure (pd_tile.cu)
     bool use_tiles = true;
+    int fit_req = 0, fit_tx = 0;  // width that the last build narrowed, and to what (md_tiles)
     int tile_tx = 0;  // cells per tile along x (0: from the mean occupancy)
     int tile_p = 2;   // threads per domain particle in the pair kernel
     int tile_block = pd::FBLOCK_T;  // threads per CTA of the precision form's pair kernel

@@ -538,6 +538,10 @@ int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR
         double vol = (h->hi[0] - h->lo[0]) * (h->hi[1] - h->lo[1]) * (h->hi[2] - h->lo[2]);
         double mean = (double)n / vol * 4.18879 * r_list * r_list * r_list;
         max_nn = (int)(mean * 1.5 + 32);
+        // an uneven system: rows as long as the densest tile's mean occupancy gives (its
+        // cells have the list's radius as side), so that the rows are not built twice
+        const double dense = (double)cap / (9.0 * (tg.TX + 2));
+        max_nn = std::max(max_nn, (int)(dense * 4.18879 * 1.1 + 16));
     }
     max_nn = (max_nn + 1) & ~1;  // whole 32-bit words
     // three z-layer passes with a third of the staging (more resident CTAs) when
