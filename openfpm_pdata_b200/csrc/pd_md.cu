@@ -213,7 +213,8 @@ __global__ void __launch_bounds__(FBLOCK) k_kick_drift(typename V4<T>::type* __r
                                                        const typename V4<T>::type* __restrict__ xb, T* __restrict__ v,
                                                        const T* __restrict__ f, long cap, long n, T half, T dt,
                                                        unsigned long long* __restrict__ maxd2, T* __restrict__ sxy,
-                                                       T* __restrict__ sz) {
+                                                       T* __restrict__ sz, StepGuard guard) {
+    if (step_skipped(guard)) return;
     double mx = 0;
     for (long i = blockIdx.x * (long)FBLOCK + threadIdx.x; i < n; i += (long)gridDim.x * FBLOCK) {
         typename V4<T>::type x = ld4(pos, i);
@@ -251,7 +252,8 @@ __global__ void __launch_bounds__(FBLOCK) k_kick_kick_drift(typename V4<T>::type
                                                             T half, T dt, double mass,
                                                             unsigned long long* __restrict__ maxd2,
                                                             double* __restrict__ part, T* __restrict__ sxy,
-                                                            T* __restrict__ sz) {
+                                                            T* __restrict__ sz, StepGuard guard) {
+    if (step_skipped(guard)) return;
     double ke = 0, mx = 0;
     for (long i = blockIdx.x * (long)FBLOCK + threadIdx.x; i < n; i += (long)gridDim.x * FBLOCK) {
         const T fx = f[i], fy = f[cap + i], fz = f[2 * cap + i];
@@ -321,85 +323,71 @@ template <class T> __global__ void k_recip_check(const T* __restrict__ x, T* __r
         y[i] = recip(x[i]);
 }
 
-// first stage of a fixed-order sum of (pe, vir) pairs: block b sums a fixed chunk
-__global__ void k_sum_pairs(const double* __restrict__ in, long n, long chunk, double* __restrict__ out) {
-    double a = 0, b = 0;
-    long beg = (long)blockIdx.x * chunk, end = min(beg + chunk, n);
-    for (long i = beg + threadIdx.x; i < end; i += 256) {
-        a += in[2 * i];
-        b += in[2 * i + 1];
-    }
-    a = block_sum<double, 256>(a);
-    b = block_sum<double, 256>(b);
-    if (threadIdx.x == 0) {
-        out[2 * blockIdx.x] = a;
-        out[2 * blockIdx.x + 1] = b;
-    }
-}
-
-// the same for (pe, vir, ke) triples: out[3b + q]
-__global__ void k_sum_triples(const double* __restrict__ in, long n, long chunk, double* __restrict__ out) {
+// E[s] = (KE, PE, virial, rebuilt) of a step: the nbf (pe, vir) pairs of its force kernel
+// and the nbk kinetic partials, added in a fixed order by one CTA (a staging kernel
+// before it cost more than the one CTA's extra rounds: 23,000 pairs are 23 a thread)
+__global__ void __launch_bounds__(1024) k_energy(const double* __restrict__ fpart, long nbf,
+                                                 const double* __restrict__ kpart, int nbk, double rebuilt,
+                                                 double* __restrict__ E) {
     double a = 0, b = 0, c = 0;
-    long beg = (long)blockIdx.x * chunk, end = min(beg + chunk, n);
-    for (long i = beg + threadIdx.x; i < end; i += 256) {
-        a += in[3 * i];
-        b += in[3 * i + 1];
-        c += in[3 * i + 2];
+    for (int i = threadIdx.x; i < nbk; i += 1024) a += kpart[i];
+    for (long i = threadIdx.x; i < nbf; i += 1024) {
+        b += fpart[2 * i];
+        c += fpart[2 * i + 1];
     }
-    a = block_sum<double, 256>(a);
-    b = block_sum<double, 256>(b);
-    c = block_sum<double, 256>(c);
-    if (threadIdx.x == 0) {
-        out[3 * blockIdx.x] = a;
-        out[3 * blockIdx.x + 1] = b;
-        out[3 * blockIdx.x + 2] = c;
-    }
-}
-
-// E = (KE, PE, virial, rebuilt) from nb (pe, vir, ke) triples
-__global__ void k_energy3(const double* __restrict__ part, int nb, const unsigned int* __restrict__ rebuilt,
-                          double* __restrict__ E) {
-    double a = 0, b = 0, c = 0;
-    for (int i = threadIdx.x; i < nb; i += 256) {
-        a += part[3 * i + 2];
-        b += part[3 * i];
-        c += part[3 * i + 1];
-    }
-    a = block_sum<double, 256>(a);
-    b = block_sum<double, 256>(b);
-    c = block_sum<double, 256>(c);
+    a = block_sum<double, 1024>(a);
+    b = block_sum<double, 1024>(b);
+    c = block_sum<double, 1024>(c);
     if (threadIdx.x == 0) {
         E[0] = a;
         E[1] = b;
         E[2] = c;
-        E[3] = rebuilt ? (double)*rebuilt : 0.0;
+        E[3] = rebuilt;
     }
 }
 
-// E[s] = (KE, PE, virial, rebuilt) from the fixed-order partials
-__global__ void k_energy(const double* __restrict__ fpart, int nbf, const double* __restrict__ kpart, int nbk,
-                         const unsigned int* __restrict__ rebuilt, double* __restrict__ E) {
-    __shared__ double sh[3][256];
+// the same for several steps at once, one CTA a step, from n (pe, vir, ke) triples each;
+// the first of the steps was rebuilt or not, the others were not
+__global__ void __launch_bounds__(1024) k_energy_steps(const double* __restrict__ part, long n, double rebuilt0,
+                                                       double* __restrict__ E) {
+    const double* in = part + 3 * n * (long)blockIdx.x;
     double a = 0, b = 0, c = 0;
-    for (int i = threadIdx.x; i < nbk; i += 256) a += kpart[i];
-    for (int i = threadIdx.x; i < nbf; i += 256) {
-        b += fpart[2 * i];
-        c += fpart[2 * i + 1];
+    for (long i = threadIdx.x; i < n; i += 1024) {
+        b += in[3 * i];
+        c += in[3 * i + 1];
+        a += in[3 * i + 2];
     }
-    sh[0][threadIdx.x] = a;
-    sh[1][threadIdx.x] = b;
-    sh[2][threadIdx.x] = c;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int q = 0; q < 3; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + s];
-        __syncthreads();
-    }
+    a = block_sum<double, 1024>(a);
+    b = block_sum<double, 1024>(b);
+    c = block_sum<double, 1024>(c);
     if (threadIdx.x == 0) {
-        E[0] = sh[0][0];
-        E[1] = sh[1][0];
-        E[2] = sh[2][0];
-        E[3] = rebuilt ? (double)*rebuilt : 0.0;
+        double* e = E + 4 * (long)blockIdx.x;
+        e[0] = a;
+        e[1] = b;
+        e[2] = c;
+        e[3] = blockIdx.x == 0 ? rebuilt0 : 0.0;
+    }
+}
+
+// the stored images from their sources (positions), and the FP64 pair kernel's staging
+// copies of them in the same pass
+template <class T>
+__global__ void k_md_images(typename V4<T>::type* __restrict__ pos, long n, const int* __restrict__ src,
+                            const unsigned char* __restrict__ shf, const T* __restrict__ shifts, long m_n,
+                            T* __restrict__ sxy, T* __restrict__ sz, StepGuard guard) {
+    if (step_skipped(guard)) return;
+    for (long m = blockIdx.x * (long)blockDim.x + threadIdx.x; m < m_n; m += (long)gridDim.x * blockDim.x) {
+        const int s = shf[m];
+        typename V4<T>::type r = ld4(pos, src[m]);
+        r.x -= shifts[3 * s];
+        r.y -= shifts[3 * s + 1];
+        r.z -= shifts[3 * s + 2];
+        st4(pos, n + m, r);
+        if (sxy) {
+            sxy[2 * (n + m)] = r.x;
+            sxy[2 * (n + m) + 1] = r.y;
+            sz[n + m] = r.z;
+        }
     }
 }
 
@@ -522,6 +510,11 @@ int force_blocks(long n) {
     return (int)want;
 }
 
+// the plain FP64 tiled LJ path (its pair kernel also kicks and drifts)
+static bool md_split_possible(pd_md md) {
+    return md->physics == 0 && !md->mixed && !md->mp.use_cell_list && md->h->dtype == PD_F64;
+}
+
 // Tiled structure: the real particles are already in cell order (sort_cl holds
 // their cell starts); sort the images by cell too, then build the tile-local rows.
 static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
@@ -619,7 +612,7 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
     md->tcap = tmax;
     PD_TRY(tile_build(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), md->tcap,
                       md->vl->r_cut, md->pos32, md->tnbr, md->tnn, md->tstride, md->tmax_nn, st));
-    PD_TRY(md->tpart.ensure(sizeof(double) * 3 * ((md->ntiles > 0 ? md->ntiles : 1) + 256)));
+    PD_TRY(md->tpart.ensure(sizeof(double) * 3 * (size_t)(md->ntiles > 0 ? md->ntiles : 1) * (md_split_possible(md) ? STEPS_AHEAD : 1)));
     md->tiles_active = true;
     return PD_OK;
 }
@@ -628,7 +621,7 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
 // the FP64 tiled pair kernel reads (x, y) / z copies of the positions, refreshed by
 // the rebuild, the drift (real particles) and the image replay
 static bool md_split(pd_md md) {
-    return md->physics == 0 && !md->mixed && md->tiles_active && !md->mp.use_cell_list && md->h->dtype == PD_F64;
+    return md->tiles_active && md_split_possible(md);
 }
 
 // The properties the cell-order reorder carries: all but those the step recomputes
@@ -709,22 +702,23 @@ int md_rebuild(pd_md md, cudaStream_t st) {
     return PD_OK;
 }
 
-int md_forces(pd_md md, cudaStream_t st, const DriftArgs* drift) {
+int md_forces(pd_md md, cudaStream_t st, const DriftArgs* drift, const StepGuard& guard, double* part) {
+    if (!part) part = md->tpart.as<double>();
     if (drift && !(md->tiles_active && md->physics == 0 && !md->mixed)) {
         set_error("md_forces: the fused drift is the plain tiled path's");
         return PD_EINVAL;
     }
     if (md->physics == 1)
         return sph_rates(md->h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->tcap, md->tnbr, md->tnn,
-                         md->tstride, md->aux, md->sp, md->mp.force_prop, md->tile_p, st);
+                         md->tstride, md->aux, md->sp, md->mp.force_prop, md->tile_p, st, guard);
     if (md->mixed)
         return mixed_lj(md->h, md->vl->cl, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(),
                         md->tcap, md->off, md->tnbr, md->tnn, md->tstride, md->lj, md->mp.force_prop,
-                        md->tpart.as<double>(), md->tile_p, md->tile_block, st);
+                        part, md->tile_p, md->tile_block, st, guard);
     if (md->tiles_active)
         return tile_lj(md->h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), md->tcap,
-                       md->tnbr, md->tnn, md->tstride, md->lj, md->mp.force_prop, md->tpart.as<double>(), true,
-                       md->tile_p, md->sxy, md->sz, st, drift);
+                       md->tnbr, md->tnn, md->tstride, md->lj, md->mp.force_prop, part, true, md->tile_p, md->sxy,
+                       md->sz, st, drift, guard);
     return lj_launch(md->h, md->mp.use_cell_list ? nullptr : md->vl, md->mp.use_cell_list ? md->cl : nullptr, md->lj,
                      md->mp.force_prop, md->fpart.as<double>(), md->nblk, st);
 }
@@ -750,7 +744,7 @@ static int md_step_cl(pd_md md, cudaStream_t st, long img_cap) {
     const T half = (T)(0.5 * md->mp.dt / md->mp.mass);
     PD_CUDA(cudaMemsetAsync(&h->ctrl->maxdisp2, 0, sizeof(unsigned long long), st));
     pd::launch(k_kick_drift<T>, md->nblk, FBLOCK, 0, st, (T4*)h->pos, md->xb.as<T4>(), (T*)V.d, (const T*)F.d, h->cap,
-               n, half, (T)md->mp.dt, &h->ctrl->maxdisp2, (T*)nullptr, (T*)nullptr);
+               n, half, (T)md->mp.dt, &h->ctrl->maxdisp2, (T*)nullptr, (T*)nullptr, StepGuard());
     PD_LAUNCH_CHECK();
     h->n_total = n;
     h->img_valid = false;
@@ -1058,6 +1052,8 @@ int pd_md_destroy(pd_md md) {
     md->aux.release();
     md->rpart.release();
     md->eidx.release();
+    md->slots.release();
+    if (md->slots_h) cudaFreeHost(md->slots_h);
     if (md->gcl) cudaGraphExecDestroy(md->gcl);
     if (md->gst) cudaStreamDestroy(md->gst);
     for (cudaEvent_t e : md->evp) cudaEventDestroy(e);
@@ -1065,38 +1061,13 @@ int pd_md_destroy(pd_md md) {
     return PD_OK;
 }
 
-// energies of step s of the plain LJ path (kinetic partials in kpart, pair partials
-// of that step's force launch, the rebuild flag in the control block)
-static int md_energy(pd_md md, int s, cudaStream_t st) {
-    pd_vd h = md->h;
-    if (md->physics == 1) {
-        // WCSPH: kinetic energy of the fluid, sum of densities
-        pd::launch(k_energy, 1, 256, 0, st, (const double*)md->rpart.as<double>(), md->nblk,
-                   (const double*)md->kpart.as<double>(), md->nblk, (const unsigned int*)&h->ctrl->rebuild,
-                   md->E.as<double>() + 4 * s);
-    } else if (md->tiles_active) {
-        const int nb2 = 256;
-        long chunk = (md->ntiles + nb2 - 1) / nb2;
-        double* stage = md->tpart.as<double>() + 2 * md->ntiles;
-        pd::launch(k_sum_pairs, nb2, 256, 0, st, (const double*)md->tpart.as<double>(), md->ntiles, chunk, stage);
-        pd::launch(k_energy, 1, 256, 0, st, (const double*)stage, nb2, (const double*)md->kpart.as<double>(),
-                   md->nblk, (const unsigned int*)&h->ctrl->rebuild, md->E.as<double>() + 4 * s);
-    } else {
-        pd::launch(k_energy, 1, 256, 0, st, (const double*)md->fpart.as<double>(), md->nblk,
-                   (const double*)md->kpart.as<double>(), md->nblk, (const unsigned int*)&h->ctrl->rebuild,
-                   md->E.as<double>() + 4 * s);
-    }
-    PD_LAUNCH_CHECK();
-    return PD_OK;
-}
-
-// energies of step s from the per-tile (pe, vir, ke) triples of a pair kernel that drifted
-static int md_energy_drift(pd_md md, int s, cudaStream_t st) {
-    const int nb2 = 256;
-    long chunk = (md->ntiles + nb2 - 1) / nb2;
-    double* stage = md->tpart.as<double>() + 3 * md->ntiles;
-    pd::launch(k_sum_triples, nb2, 256, 0, st, (const double*)md->tpart.as<double>(), md->ntiles, chunk, stage);
-    pd::launch(k_energy3, 1, 256, 0, st, (const double*)stage, nb2, (const unsigned int*)&md->h->ctrl->rebuild,
+// energies of step s from the kinetic partials in kpart and the pair partials of its force
+// launch (WCSPH: kinetic energy of the fluid and sum of densities)
+static int md_energy(pd_md md, int s, bool rebuilt, cudaStream_t st) {
+    const double* f = md->physics == 1 ? md->rpart.as<double>()
+                                       : (md->tiles_active ? md->tpart.as<double>() : md->fpart.as<double>());
+    const long nf = md->physics == 0 && md->tiles_active ? md->ntiles : md->nblk;
+    pd::launch(k_energy, 1, 1024, 0, st, f, nf, (const double*)md->kpart.as<double>(), md->nblk, rebuilt ? 1.0 : 0.0,
                md->E.as<double>() + 4 * s);
     PD_LAUNCH_CHECK();
     return PD_OK;
@@ -1119,6 +1090,79 @@ static void md_fold_timing(pd_md md) {
     md->ev_rebuilt.clear();
 }
 
+// the step's opening half kick and drift, after the closing half kick of the step before
+// where `closing`; largest displacement to *maxd2
+static int md_drift(pd_md md, bool closing, unsigned long long* maxd2, const StepGuard& guard, cudaStream_t st) {
+    pd_vd h = md->h;
+    const long n = h->n_real;
+    const double half = 0.5 * md->mp.dt / md->mp.mass;
+    const Prop& V = h->props[md->mp.vel_prop];
+    const Prop& F = h->props[md->mp.force_prop];
+    if (md->physics == 1) {
+        if (closing)
+            return sph_kick_kick_drift(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->xb, md->aux, md->nblk,
+                                       md->mp.dt, md->kpart.as<double>(), md->rpart.as<double>(), maxd2, guard, st);
+        return sph_kick_drift(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->xb, md->aux, md->nblk, md->mp.dt,
+                              maxd2, guard, st);
+    }
+    if (md->mixed) {
+        if (closing)
+            return mixed_kick_kick_drift(h, md->vl->cl, md->off, md->offb, md->mp.vel_prop, md->mp.force_prop,
+                                         md->nblk, half, md->mp.dt, md->mp.mass, md->kpart.as<double>(), maxd2, guard,
+                                         st);
+        return mixed_kick_drift(h, md->vl->cl, md->off, md->offb, md->mp.vel_prop, md->mp.force_prop, md->nblk, half,
+                                md->mp.dt, maxd2, guard, st);
+    }
+    const bool split = md_split(md);  // the drift also refreshes the pair kernel's staging copies
+    auto go = [&](auto zero) {
+        typedef decltype(zero) T;
+        typedef typename V4<T>::type T4;
+        T* sxy = split ? md->sxy.as<T>() : nullptr;
+        T* sz = split ? md->sz.as<T>() : nullptr;
+        if (closing)
+            pd::launch(k_kick_kick_drift<T>, md->nblk, FBLOCK, 0, st, (T4*)h->pos, (const T4*)md->xb.as<T4>(), (T*)V.d,
+                       (const T*)F.d, h->cap, n, (T)half, (T)md->mp.dt, md->mp.mass, maxd2, md->kpart.as<double>(), sxy,
+                       sz, guard);
+        else
+            pd::launch(k_kick_drift<T>, md->nblk, FBLOCK, 0, st, (T4*)h->pos, (const T4*)md->xb.as<T4>(), (T*)V.d,
+                       (const T*)F.d, h->cap, n, (T)half, (T)md->mp.dt, maxd2, sxy, sz, guard);
+    };
+    if (h->dtype == PD_F64) go(0.0);
+    else go(0.0f);
+    PD_LAUNCH_CHECK();
+    return PD_OK;
+}
+
+// the images between rebuilds
+static int md_images(pd_md md, const StepGuard& guard, cudaStream_t st) {
+    pd_vd h = md->h;
+    if (md->mixed) return mixed_replay(h, md->off, md->offK, guard, st);
+    const long m = h->n_img;
+    if (m <= 0) return PD_OK;
+    const bool split = md_split(md);
+    auto go = [&](auto zero) {
+        typedef decltype(zero) T;
+        pd::launch(k_md_images<T>, grid_for(m, 256), 256, 0, st, (typename V4<T>::type*)h->pos, h->n_real,
+                   (const int*)h->img_src.as<int>(), (const unsigned char*)h->img_shift.as<unsigned char>(),
+                   (const T*)h->shifts.as<T>(), m, split ? md->sxy.as<T>() : (T*)nullptr,
+                   split ? md->sz.as<T>() : (T*)nullptr, guard);
+    };
+    if (h->dtype == PD_F64) go(0.0);
+    else go(0.0f);
+    PD_LAUNCH_CHECK();
+    return PD_OK;
+}
+
+// A run goes in batches of steps.  A batch's first step may rebuild; the steps after it
+// are enqueued before their rebuild decision is known, each guarded by the squared
+// displacement its drift left in a device slot (StepGuard): from the first step above
+// skin/2 on, the batch's kernels do nothing.  The host then reads the slots once, rebuilds
+// for that step and goes on from it.  So a rebuild interval costs about one host round
+// trip instead of one a step, which is most of a small system's step (10 steps of 250,047
+// FP64 particles with a snapshot 1.88 -> 1.63 ms).  The batch's length is the
+// steps expected until the next rebuild (the last interval); a step too many costs two
+// launches that return at once.  The operations of each step and their order do not
+// depend on the batches.
 int pd_md_run(pd_md md, int steps, void* stream, double* E) {
     if (!md || steps < 0) return PD_EINVAL;
     if (md_cluster_eligible(md)) return md_run_cluster(md, steps, S(stream), E);
@@ -1126,22 +1170,22 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
         return md_run_cl_graph(md, steps, S(stream), E);
     pd_vd h = md->h;
     cudaStream_t st = S(stream);
-    long n = h->n_real;
     PD_TRY(md->E.ensure(sizeof(double) * 4 * (steps + 1)));
-    Prop& V = h->props[md->mp.vel_prop];
-    Prop& F = h->props[md->mp.force_prop];
+    PD_TRY(md->slots.ensure(sizeof(unsigned long long) * (STEPS_AHEAD + 1)));
+    unsigned long long* slots = md->slots.as<unsigned long long>();
+    if (!md->slots_h)
+        PD_CUDA(cudaMallocHost((void**)&md->slots_h, sizeof(unsigned long long) * (STEPS_AHEAD + 1)));
+    const Prop& V = h->props[md->mp.vel_prop];
     if (!md->ready) {
         PD_TRY(md_rebuild(md, st));
         PD_TRY(md_forces(md, st));
         md->ready = true;
+        md->since = 0;
     }
-    double half = 0.5 * md->mp.dt / md->mp.mass;
-    double lim = 0.5 * md->mp.skin;
-    double lim2 = lim * lim;
-    // a step's closing half kick is fused with the next step's kick-drift
-    // (k_kick_kick_drift, k_sph_kick_kick_drift); the step's energies follow it, the
-    // last step's closing kick runs after the loop
-    const bool fused = md->physics == 0 || md->physics == 1;
+    const double half = 0.5 * md->mp.dt / md->mp.mass;
+    const double lim = 0.5 * md->mp.skin;
+    const double lim2 = lim * lim;
+    const bool always = md->mp.skin <= 0 || md->mp.use_cell_list;  // rebuild every step
     // timing: six events per step, read after the run (no synchronisation in the loop)
     if (md->timing)
         while (md->evp.size() < (size_t)6 * steps) {
@@ -1153,160 +1197,153 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
     std::vector<unsigned char> rebuilt_at(md->timing ? steps : 0, 0);
 #define PD_EV(k) \
     if (md->timing) PD_CUDA(cudaEventRecord(md->evp[6 * (size_t)s + (k)], st))
-    for (int s = 0; s < steps; ++s) {
-        unsigned int rebuilt = 0;
-        const bool split = md_split(md);  // the drift also refreshes the pair kernel's staging copies
-        PD_EV(0);
-        if (md->drifted) {
-            // the previous step's pair kernel made this step's kick and drift (and the
-            // previous step's closing kick and energies)
-            md->drifted = false;
-        } else {
-            PD_CUDA(cudaMemsetAsync(&h->ctrl->maxdisp2, 0, sizeof(unsigned long long), st));
-            if (fused && s > 0 && md->physics == 1) {
-                PD_TRY(sph_kick_kick_drift(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->xb, md->aux, md->nblk,
-                                           md->mp.dt, md->kpart.as<double>(), md->rpart.as<double>(), st));
-                PD_TRY(md_energy(md, s - 1, st));
-            } else if (fused && s > 0 && md->mixed) {
-                PD_TRY(mixed_kick_kick_drift(h, md->vl->cl, md->off, md->offb, md->mp.vel_prop, md->mp.force_prop, md->nblk, half,
-                                             md->mp.dt, md->mp.mass, md->kpart.as<double>(), st));
-                PD_TRY(md_energy(md, s - 1, st));
-            } else if (fused && s > 0) {
-                if (h->dtype == PD_F64)
-                    pd::launch(k_kick_kick_drift<double>, md->nblk, FBLOCK, 0, st, (double4*)h->pos,
-                               (const double4*)md->xb.as<double4>(), (double*)V.d, (const double*)F.d, h->cap, n, half,
-                               md->mp.dt, md->mp.mass, &h->ctrl->maxdisp2, md->kpart.as<double>(), split ? md->sxy.as<double>() : nullptr,
-                               split ? md->sz.as<double>() : nullptr);
-                else
-                    pd::launch(k_kick_kick_drift<float>, md->nblk, FBLOCK, 0, st, (float4*)h->pos,
-                               (const float4*)md->xb.as<float4>(), (float*)V.d, (const float*)F.d, h->cap, n, (float)half,
-                               (float)md->mp.dt, md->mp.mass, &h->ctrl->maxdisp2, md->kpart.as<double>(), (float*)nullptr,
-                               (float*)nullptr);
-                PD_LAUNCH_CHECK();
-                PD_TRY(md_energy(md, s - 1, st));
-            } else if (md->physics == 1)
-                PD_TRY(sph_kick_drift(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->xb, md->aux, md->nblk,
-                                      md->mp.dt, st));
-            else if (md->mixed)
-                PD_TRY(mixed_kick_drift(h, md->vl->cl, md->off, md->offb, md->mp.vel_prop, md->mp.force_prop, md->nblk, half,
-                                        md->mp.dt, st));
-            else if (h->dtype == PD_F64)
-                pd::launch(k_kick_drift<double>, md->nblk, FBLOCK, 0, st, (double4*)h->pos, md->xb.as<double4>(), (double*)V.d,
-                                                                  (const double*)F.d, h->cap, n, half, md->mp.dt,
-                                                                  &h->ctrl->maxdisp2, split ? md->sxy.as<double>() : nullptr,
-                                                                  split ? md->sz.as<double>() : nullptr);
-            else
-                pd::launch(k_kick_drift<float>, md->nblk, FBLOCK, 0, st, (float4*)h->pos, md->xb.as<float4>(), (float*)V.d,
-                                                                 (const float*)F.d, h->cap, n, (float)half,
-                                                                 (float)md->mp.dt, &h->ctrl->maxdisp2, (float*)nullptr,
-                                                                 (float*)nullptr);
+    bool drifted = false;     // step s is drifted already
+    bool due = false;         // ... and its rebuild decision is known: this
+    bool closing = false;     // the step before s still lacks its closing half kick and energies
+    bool last_rebuilt = false;  // ... and was rebuilt
+    for (int s = 0; s < steps;) {
+        // the drift and the pair kernel in one (plain FP64 tiles); a rebuild may change it
+        bool fused = md_split(md);
+        const bool ahead = !always && !md->timing && (md->tiles_active || md->physics == 1);
+        int K = 1;
+        if (ahead) {
+            // one step more than the last interval leaves until the next rebuild
+            const long left = due ? md->since + 2 : (md->interval > 0 ? md->interval - md->since : 4);
+            K = (int)std::max(2L, std::min((long)STEPS_AHEAD, left));
+        }
+        K = std::min(K, steps - s);
+        PD_CUDA(cudaMemsetAsync(slots, 0, sizeof(unsigned long long) * (K + 1), st));
+        const bool known = drifted;
+        bool rb = due, rebuilt = false;
+        for (int b = 0; b < K; ++b) {
+            if (b == 0) {
+                PD_EV(0);
+                if (!drifted) {
+                    PD_TRY(md_drift(md, closing, slots, StepGuard(), st));
+                    if (closing) PD_TRY(md_energy(md, s - 1, last_rebuilt, st));
+                    rb = always;
+                    if (!always && K == 1) {
+                        PD_CUDA(cudaMemcpyAsync(md->slots_h, slots, sizeof(unsigned long long),
+                                                cudaMemcpyDeviceToHost, st));
+                        PD_CUDA(cudaStreamSynchronize(st));
+                        double d2;
+                        memcpy(&d2, md->slots_h, sizeof(double));
+                        rb = d2 > lim2;
+                    }
+                }
+                PD_EV(1);
+                PD_EV(2);
+                if (rb) {
+                    PD_TRY(md_rebuild(md, st));
+                    rebuilt = true;
+                    md->interval = md->since + 1;
+                    md->since = -1;  // this step makes it 0
+                    if (fused != md_split(md)) {  // the neighbour structure changed its kind
+                        fused = md_split(md);
+                        K = 1;
+                    }
+                } else {
+                    PD_TRY(md_images(md, known || K == 1 ? StepGuard() : StepGuard{slots, nullptr, lim2}, st));
+                }
+                PD_EV(3);
+            } else {
+                if (!fused) {
+                    PD_TRY(md_drift(md, true, slots + b, StepGuard{slots + b - 1, slots + b, lim2}, st));
+                    PD_TRY(md_energy(md, s + b - 1, b == 1 && rebuilt, st));
+                }
+                PD_TRY(md_images(md, StepGuard{slots + b, nullptr, lim2}, st));
+            }
+            const bool unguarded = b == 0 && (known || rb || K == 1);
+            if (fused) {
+                // this step's closing kick and, unless it is the run's last, the next
+                // step's kick and drift into the second pair of staging copies
+                const bool close = s + b + 1 == steps;
+                const size_t cap = (size_t)(h->cap > 0 ? h->cap : 1);
+                if (!close) {
+                    PD_TRY(md->sxy2.ensure(cap * sizeof(double2)));
+                    PD_TRY(md->sz2.ensure(cap * sizeof(double)));
+                }
+                DriftArgs D{close, (double4*)h->pos, md->xb.as<const double4>(), (double*)V.d, h->cap, half,
+                            md->mp.dt, md->mp.mass, md->sxy2.as<double2>(), md->sz2.as<double>(), slots + b + 1};
+                const StepGuard g = unguarded ? StepGuard() : StepGuard{slots + b, slots + b + 1, lim2};
+                PD_TRY(md_forces(md, st, &D, g, md->tpart.as<double>() + 3 * md->ntiles * (long)b));
+                if (!close) {
+                    std::swap(md->sxy, md->sxy2);
+                    std::swap(md->sz, md->sz2);
+                }
+            } else {
+                PD_TRY(md_forces(md, st, nullptr, unguarded ? StepGuard() : StepGuard{slots + b, nullptr, lim2}));
+            }
+            if (b == 0) PD_EV(4);
+        }
+        if (fused) {
+            // rows of steps that were not reached are written again when they are
+            pd::launch(k_energy_steps, (unsigned)K, 1024, 0, st, (const double*)md->tpart.as<double>(), md->ntiles,
+                       rebuilt ? 1.0 : 0.0, md->E.as<double>() + 4 * s);
             PD_LAUNCH_CHECK();
         }
-        PD_EV(1);
-        bool rb = md->mp.skin <= 0 || md->mp.use_cell_list;
-        if (!rb) {
-            PD_CUDA(cudaMemcpyAsync(&h->ctrl_h->maxdisp2, &h->ctrl->maxdisp2, sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, st));
+        PD_EV(5);
+        if (md->timing) rebuilt_at[s] = rebuilt ? 1 : 0;
+        // how far the batch came
+        int done = K;
+        drifted = due = false;
+        if (!always && (fused || K > 1)) {
+            PD_CUDA(cudaMemcpyAsync(md->slots_h, slots, sizeof(unsigned long long) * (K + 1), cudaMemcpyDeviceToHost,
+                                    st));
             PD_CUDA(cudaStreamSynchronize(st));
-            double d2;
-            memcpy(&d2, &h->ctrl_h->maxdisp2, sizeof(double));
-            rb = d2 > lim2;
+            auto over = [&](int b) {
+                double d2;
+                memcpy(&d2, md->slots_h + b, sizeof(double));
+                return d2 > lim2;
+            };
+            done = known || rb || K == 1 ? 1 : 0;
+            while (done < K && !(over(done))) ++done;
+            if (done < K) {  // step s + done is drifted and needs a rebuild first
+                drifted = due = true;
+            } else if (fused && s + K < steps) {
+                drifted = true;
+                due = over(K);
+            }
+        } else if (fused && s + K < steps) {
+            drifted = true;
+            due = always;
         }
-        PD_EV(2);
-        if (rb) {
-            PD_TRY(md_rebuild(md, st));
-            rebuilt = 1;
-        } else if (md->mixed) {
-            PD_TRY(mixed_replay(h, md->off, md->offK, st));
-        } else {
-            PD_TRY(ghost_replay(h, 0ul, true, nullptr, h->n_img, st));
-            if (split) PD_TRY(tile_split(h, md->sxy, md->sz, h->n_real, h->n_img, st));
+        if (fused && done < K) {
+            // the kernels of the steps not made left the staging copies as they were
+            const int swaps = (K - done) - (s + K == steps ? 1 : 0);
+            if (swaps & 1) {
+                std::swap(md->sxy, md->sxy2);
+                std::swap(md->sz, md->sz2);
+            }
         }
-        PD_EV(3);
-        // plain FP64 tiled steps with a next step in this run: the pair kernel also
-        // makes this step's closing kick and the next step's kick and drift, into the
-        // second pair of staging copies, which then become the current ones
-        const bool drift = fused && !md->mixed && md_split(md) && s + 1 < steps;
-        if (drift) {
-            const size_t cap = (size_t)(h->cap > 0 ? h->cap : 1);
-            PD_TRY(md->sxy2.ensure(cap * sizeof(double2)));
-            PD_TRY(md->sz2.ensure(cap * sizeof(double)));
-            PD_CUDA(cudaMemsetAsync(&h->ctrl->maxdisp2, 0, sizeof(unsigned long long), st));
-            DriftArgs D{(double4*)h->pos, md->xb.as<const double4>(), (double*)V.d, h->cap, half, md->mp.dt,
-                        md->mp.mass, md->sxy2.as<double2>(), md->sz2.as<double>(), &h->ctrl->maxdisp2};
-            PD_TRY(md_forces(md, st, &D));
-            std::swap(md->sxy, md->sxy2);
-            std::swap(md->sz, md->sz2);
-            md->drifted = true;
-        } else {
-            PD_TRY(md_forces(md, st));
-        }
-        PD_EV(4);
-        if (md->timing) rebuilt_at[s] = (unsigned char)rebuilt;
-        if (fused) {
-            // the rebuild flag of this step, read by its energies
-            h->ctrl_h->rebuild = rebuilt;
-            PD_CUDA(cudaMemcpyAsync(&h->ctrl->rebuild, &h->ctrl_h->rebuild, sizeof(unsigned int),
-                                    cudaMemcpyHostToDevice, st));
-            if (drift) PD_TRY(md_energy_drift(md, s, st));
-            md->steps++;
-            PD_EV(5);
-            continue;
-        }
+        s += done;
+        md->steps += done;
+        md->since += done;
+        // a step drifted by md_drift is closed by the next step's; one that stopped the
+        // batch was drifted, and the step before it closed, in the batch
+        closing = !fused && done > 0 && !drifted;
+        last_rebuilt = rebuilt && done == 1;
+    }
+#undef PD_EV
+    if (closing) {
+        // the last step's closing half kick and energies
         if (md->physics == 1)
-            PD_TRY(sph_kick(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->nblk, md->mp.dt,
-                            md->kpart.as<double>(), md->rpart.as<double>(), st));
+            PD_TRY(sph_kick(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->nblk, md->mp.dt, md->kpart.as<double>(),
+                            md->rpart.as<double>(), st));
         else if (md->mixed)
             PD_TRY(mixed_kick(h, md->mp.vel_prop, md->mp.force_prop, md->nblk, half, md->mp.mass,
                               md->kpart.as<double>(), st));
-        else if (h->dtype == PD_F64)
-            pd::launch(k_kick<double>, md->nblk, FBLOCK, 0, st, (double*)V.d, (const double*)F.d, h->cap, n, half,
-                                                        md->mp.mass, md->kpart.as<double>());
-        else
-            pd::launch(k_kick<float>, md->nblk, FBLOCK, 0, st, (float*)V.d, (const float*)F.d, h->cap, n, (float)half,
-                                                       md->mp.mass, md->kpart.as<double>());
-        PD_LAUNCH_CHECK();
-        h->ctrl_h->rebuild = rebuilt;
-        PD_CUDA(cudaMemcpyAsync(&h->ctrl->rebuild, &h->ctrl_h->rebuild, sizeof(unsigned int), cudaMemcpyHostToDevice, st));
-        if (md->physics == 1) {
-            pd::launch(k_energy, 1, 256, 0, st, (const double*)md->rpart.as<double>(), md->nblk,
-                       (const double*)md->kpart.as<double>(), md->nblk, (const unsigned int*)&h->ctrl->rebuild,
-                       md->E.as<double>() + 4 * s);
-        } else if (md->tiles_active) {
-            const int nb2 = 256;
-            long chunk = (md->ntiles + nb2 - 1) / nb2;
-            double* stage = md->tpart.as<double>() + 2 * md->ntiles;
-            pd::launch(k_sum_pairs, nb2, 256, 0, st, (const double*)md->tpart.as<double>(), md->ntiles, chunk, stage);
-            pd::launch(k_energy, 1, 256, 0, st, (const double*)stage, nb2, (const double*)md->kpart.as<double>(),
-                       md->nblk, (const unsigned int*)&h->ctrl->rebuild, md->E.as<double>() + 4 * s);
+        else {
+            const Prop& F = h->props[md->mp.force_prop];
+            if (h->dtype == PD_F64)
+                pd::launch(k_kick<double>, md->nblk, FBLOCK, 0, st, (double*)V.d, (const double*)F.d, h->cap,
+                           h->n_real, half, md->mp.mass, md->kpart.as<double>());
+            else
+                pd::launch(k_kick<float>, md->nblk, FBLOCK, 0, st, (float*)V.d, (const float*)F.d, h->cap, h->n_real,
+                           (float)half, md->mp.mass, md->kpart.as<double>());
+            PD_LAUNCH_CHECK();
         }
-        else
-            pd::launch(k_energy, 1, 256, 0, st, (const double*)md->fpart.as<double>(), md->nblk,
-                       (const double*)md->kpart.as<double>(), md->nblk, (const unsigned int*)&h->ctrl->rebuild,
-                       md->E.as<double>() + 4 * s);
-        PD_LAUNCH_CHECK();
-        md->steps++;
-        PD_EV(5);
-    }
-#undef PD_EV
-    if (fused && steps > 0 && md->physics == 1) {
-        PD_TRY(sph_kick(h, md->sp, md->mp.vel_prop, md->mp.force_prop, md->nblk, md->mp.dt, md->kpart.as<double>(),
-                        md->rpart.as<double>(), st));
-        PD_TRY(md_energy(md, steps - 1, st));
-    } else if (fused && steps > 0 && md->mixed) {
-        PD_TRY(mixed_kick(h, md->mp.vel_prop, md->mp.force_prop, md->nblk, half, md->mp.mass, md->kpart.as<double>(),
-                          st));
-        PD_TRY(md_energy(md, steps - 1, st));
-    } else if (fused && steps > 0) {
-        // the last step's closing half kick and energies
-        if (h->dtype == PD_F64)
-            pd::launch(k_kick<double>, md->nblk, FBLOCK, 0, st, (double*)V.d, (const double*)F.d, h->cap, n, half,
-                       md->mp.mass, md->kpart.as<double>());
-        else
-            pd::launch(k_kick<float>, md->nblk, FBLOCK, 0, st, (float*)V.d, (const float*)F.d, h->cap, n, (float)half,
-                       md->mp.mass, md->kpart.as<double>());
-        PD_LAUNCH_CHECK();
-        PD_TRY(md_energy(md, steps - 1, st));
+        PD_TRY(md_energy(md, steps - 1, last_rebuilt, st));
     }
     if (md->mixed) PD_TRY(mixed_to_positions(h, md->vl->cl, md->off, st));  // the vector's positions are current
     if (E && steps > 0) {

@@ -33,7 +33,6 @@ struct pd_md_s {
     pd::Buf csR, csI, tnbr, tnn, tpart, pos32;
     pd::Buf sxy, sz;  // FP64 tiled path: the pair kernel's (x, y) / z copies of the positions
     pd::Buf sxy2, sz2;  // the second pair, written by a pair kernel that also drifts
-    bool drifted = false;  // the last pair kernel made the next step's kick and drift
     // precision form: FP32 cell-local offsets (all particles), their value at the
     // last build (real particles) and the constant parts of the image offsets
     int physics = 0;  // 0: Lennard-Jones, 1: WCSPH
@@ -43,6 +42,11 @@ struct pd_md_s {
     bool off_valid = false;  // `off` holds the authoritative state (after the first build)
     pd::Buf off, offb, offK;
     long builds = 0, steps = 0;
+    // steps enqueued ahead of their rebuild decision: a squared displacement per step of a
+    // batch (device, pinned mirror), steps since the last rebuild, the interval before it
+    pd::Buf slots;
+    unsigned long long* slots_h = nullptr;
+    long since = 0, interval = 0;
     // cell-list mode: the captured step graph, its image capacity, the step counter
     cudaGraphExec_t gcl = nullptr;
     cudaStream_t gst = nullptr;
@@ -62,12 +66,14 @@ struct pd_md_s {
 };
 
 namespace pd {
+static constexpr int STEPS_AHEAD = 8;  // steps of a batch at most (pd_md_run)
 int force_blocks(long n);
 // wrap, sort, periodic images, neighbour structure (and the mixed-form offsets)
 int md_rebuild(pd_md md, cudaStream_t st);
 // forces of the current state into the force property (with `drift`, the plain FP64
 // tiled path's pair kernel also makes the next step's kick and drift instead)
-int md_forces(pd_md md, cudaStream_t st, const DriftArgs* drift = nullptr);
+int md_forces(pd_md md, cudaStream_t st, const DriftArgs* drift = nullptr, const StepGuard& guard = StepGuard(),
+              double* part = nullptr);
 // cell-list mode of a small system: every step of a run in one thread-block cluster (pd_cluster.cu)
 bool md_cluster_eligible(pd_md md);
 int md_run_cluster(pd_md md, int steps, cudaStream_t st, double* E);

@@ -91,7 +91,8 @@ __global__ void k_image_k(const double4* __restrict__ pos, const float4* __restr
 }
 
 __global__ void k_replay32(float4* __restrict__ off, long n_real, long m, const int* __restrict__ src,
-                           const float4* __restrict__ K) {
+                           const float4* __restrict__ K, StepGuard guard) {
+    if (step_skipped(guard)) return;
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < m; k += (long)gridDim.x * blockDim.x) {
         float4 o = off[src[k]], q = K[k];
         float4 r = off[n_real + k];
@@ -106,7 +107,8 @@ __global__ void k_replay32(float4* __restrict__ off, long n_real, long m, const 
 __global__ void __launch_bounds__(256) k_kick_drift32(float4* __restrict__ off, const float4* __restrict__ ob,
                                                       float* __restrict__ v, const float* __restrict__ f, long cap,
                                                       long n, float half, float dt, CellGeom C,
-                                                      unsigned long long* __restrict__ maxd2) {
+                                                      unsigned long long* __restrict__ maxd2, StepGuard guard) {
+    if (step_skipped(guard)) return;
     double mx = 0;
     for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
         float4 o = off[i];
@@ -134,7 +136,8 @@ __global__ void __launch_bounds__(256) k_kick_kick_drift32(float4* __restrict__ 
                                                            float* __restrict__ v, const float* __restrict__ f,
                                                            long cap, long n, float half, float dt, double mass,
                                                            CellGeom C, unsigned long long* __restrict__ maxd2,
-                                                           double* __restrict__ part) {
+                                                           double* __restrict__ part, StepGuard guard) {
+    if (step_skipped(guard)) return;
     double mx = 0, ke = 0;
     for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
         const float fx = f[i], fy = f[cap + i], fz = f[2 * cap + i];
@@ -187,7 +190,8 @@ __global__ void __launch_bounds__(BLOCK, 5 * FBLOCK_T / BLOCK) k_vtile_lj_mixed(
                                                              const int* __restrict__ nn, long stride, float sx,
                                                              float sy, float sz, LJP<float> Pr, float* __restrict__ f,
                                                              long fcap, double* __restrict__ part,
-                                                             unsigned int* __restrict__ err) {
+                                                             unsigned int* __restrict__ err, StepGuard guard) {
+    if (step_skipped(guard)) return;
     extern __shared__ __align__(128) unsigned char tile_raw[];
     float4* sm = reinterpret_cast<float4*>(tile_raw);
     __shared__ TileShM S;
@@ -270,32 +274,33 @@ int mixed_to_positions_by_id(pd_vd h, pd_cl cl, const Buf& off, double* out, cud
     return PD_OK;
 }
 
-int mixed_replay(pd_vd h, Buf& off, const Buf& K, cudaStream_t st) {
+int mixed_replay(pd_vd h, Buf& off, const Buf& K, const StepGuard& guard, cudaStream_t st) {
     long m = h->n_img;
     if (m > 0)
         pd::launch(k_replay32, grid_for(m, 256), 256, 0, st, off.as<float4>(), h->n_real, m,
-                   (const int*)h->img_src.as<int>(), (const float4*)K.as<float4>());
+                   (const int*)h->img_src.as<int>(), (const float4*)K.as<float4>(), guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
 
 int mixed_kick_drift(pd_vd h, pd_cl cl, Buf& off, const Buf& ob, int vel_prop, int force_prop, int nblk,
-                     double half, double dt, cudaStream_t st) {
+                     double half, double dt, unsigned long long* maxd2, const StepGuard& guard, cudaStream_t st) {
     Prop& V = h->props[vel_prop];
     Prop& F = h->props[force_prop];
     pd::launch(k_kick_drift32, nblk, 256, 0, st, off.as<float4>(), (const float4*)ob.as<float4>(), (float*)V.d,
-               (const float*)F.d, h->cap, h->n_real, (float)half, (float)dt, mixed_cell_geom(cl), &h->ctrl->maxdisp2);
+               (const float*)F.d, h->cap, h->n_real, (float)half, (float)dt, mixed_cell_geom(cl), maxd2, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
 
 int mixed_kick_kick_drift(pd_vd h, pd_cl cl, Buf& off, const Buf& ob, int vel_prop, int force_prop, int nblk,
-                          double half, double dt, double mass, double* kpart, cudaStream_t st) {
+                          double half, double dt, double mass, double* kpart, unsigned long long* maxd2,
+                          const StepGuard& guard, cudaStream_t st) {
     Prop& V = h->props[vel_prop];
     Prop& F = h->props[force_prop];
     pd::launch(k_kick_kick_drift32, nblk, 256, 0, st, off.as<float4>(), (const float4*)ob.as<float4>(), (float*)V.d,
-               (const float*)F.d, h->cap, h->n_real, (float)half, (float)dt, mass, mixed_cell_geom(cl),
-               &h->ctrl->maxdisp2, kpart);
+               (const float*)F.d, h->cap, h->n_real, (float)half, (float)dt, mass, mixed_cell_geom(cl), maxd2,
+               kpart, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
@@ -313,13 +318,14 @@ int mixed_kick(pd_vd h, int vel_prop, int force_prop, int nblk, double half, dou
 template <int P, int BLOCK>
 static int launch_mixed(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                         unsigned int cap, const Buf& off, const Buf& nbr, const Buf& nn, long stride, float sx,
-                        float sy, float sz, const LJP<float>& LP, float* f, double* part, cudaStream_t st) {
+                        float sy, float sz, const LJP<float>& LP, float* f, double* part, const StepGuard& guard,
+                        cudaStream_t st) {
     int smem = (int)(cap * sizeof(float4));
     if (smem < 16) smem = 16;
     PD_CUDA(cudaFuncSetAttribute(k_vtile_lj_mixed<P, BLOCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     pd::launch(k_vtile_lj_mixed<P, BLOCK>, (unsigned)ntiles, BLOCK, (size_t)smem, st, (const float4*)off.as<float4>(),
                h->n_real, tg, csR, csI, cap, (const unsigned int*)nbr.as<unsigned int>(), (const int*)nn.as<int>(),
-               stride, sx, sy, sz, LP, f, h->cap, part, &h->ctrl->err);
+               stride, sx, sy, sz, LP, f, h->cap, part, &h->ctrl->err, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
@@ -339,7 +345,7 @@ void mixed_cutoff(const pd_lj_params_t& lj, LJP<float>& P) {
 
 int mixed_lj(pd_vd h, pd_cl cl, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
              unsigned int cap, const Buf& off, const Buf& nbr, const Buf& nn, long stride, const pd_lj_params_t& lj,
-             int force_prop, double* part, int P, int block, cudaStream_t st) {
+             int force_prop, double* part, int P, int block, cudaStream_t st, const StepGuard& guard) {
     LJP<float> LP{};
     LP.eps24 = (float)(24.0 * lj.eps);
     LP.eps4 = (float)(4.0 * lj.eps);
@@ -350,7 +356,8 @@ int mixed_lj(pd_vd h, pd_cl cl, const TileGeom& tg, long ntiles, const unsigned 
     const float sx = (float)C.sp[0], sy = (float)C.sp[1], sz = (float)C.sp[2];  // exact: multiples of q
 #define PD_MIXED_CASE(PP, BB)                                                                                   \
     if (P == PP && block == BB)                                                                                 \
-        return launch_mixed<PP, BB>(h, tg, ntiles, csR, csI, cap, off, nbr, nn, stride, sx, sy, sz, LP, f, part, st);
+        return launch_mixed<PP, BB>(h, tg, ntiles, csR, csI, cap, off, nbr, nn, stride, sx, sy, sz, LP, f, part, guard, \
+                                    st);
     PD_MIXED_CASE(1, FBLOCK_T)
     PD_MIXED_CASE(2, FBLOCK_T)
     PD_MIXED_CASE(4, FBLOCK_T)

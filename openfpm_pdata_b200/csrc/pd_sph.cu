@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(256) k_sph_kick_drift(typename V4<T>::type* __
                                                         const T* __restrict__ a, T* __restrict__ rho,
                                                         const T* __restrict__ drho, const int* __restrict__ type,
                                                         long cap, long n, T half, T dt, SphK<T> P,
-                                                        unsigned long long* __restrict__ maxd2) {
+                                                        unsigned long long* __restrict__ maxd2, StepGuard guard) {
+    if (step_skipped(guard)) return;
     double mx = 0;
     for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
         typename V4<T>::type x = ld4(pos, i);
@@ -154,7 +155,9 @@ __global__ void __launch_bounds__(256) k_sph_kick_kick_drift(typename V4<T>::typ
                                                              const int* __restrict__ type, long cap, long n, T half,
                                                              T dt, SphK<T> P, double m,
                                                              unsigned long long* __restrict__ maxd2,
-                                                             double* __restrict__ kpart, double* __restrict__ rpart) {
+                                                             double* __restrict__ kpart, double* __restrict__ rpart,
+                                                             StepGuard guard) {
+    if (step_skipped(guard)) return;
     double mx = 0, ke = 0, rs = 0;
     for (long i = blockIdx.x * 256L + threadIdx.x; i < n; i += (long)gridDim.x * 256) {
         typename V4<T>::type x = ld4(pos, i);
@@ -219,8 +222,9 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
                                                         const int* __restrict__ nn, long stride, int mwords,
                                                         const int* __restrict__ type, SphK<T> K, T* __restrict__ acc,
                                                         T* __restrict__ drho, long cap_p,
-                                                        unsigned int* __restrict__ err) {
+                                                        unsigned int* __restrict__ err, StepGuard guard) {
     typedef typename V4<T>::type T4;
+    if (step_skipped(guard)) return;
     extern __shared__ __align__(128) unsigned char tile_raw[];
     T4* sp = reinterpret_cast<T4*>(tile_raw);
     T4* sa = sp + cap;
@@ -411,7 +415,7 @@ int sph_pack(pd_vd h, const pd_sph_params_t& sp, int vel_prop, Buf& aux, cudaStr
 }
 
 int sph_kick_drift(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int acc_prop, const Buf& xb, Buf& aux,
-                   int nblk, double dt, cudaStream_t st) {
+                   int nblk, double dt, unsigned long long* maxd2, const StepGuard& guard, cudaStream_t st) {
     long n = h->n_real;
     const Prop& V = h->props[vel_prop];
     const Prop& A = h->props[acc_prop];
@@ -421,11 +425,11 @@ int sph_kick_drift(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int acc_pro
     if (h->dtype == PD_F64)
         pd::launch(k_sph_kick_drift<double>, nblk, 256, 0, st, (double4*)h->pos, (const double4*)xb.as<double4>(),
                    aux.as<double4>(), (double*)V.d, (const double*)A.d, (double*)R.d, (const double*)D.d,
-                   (const int*)Ty.d, h->cap, n, 0.5 * dt, dt, sphk<double>(sp), &h->ctrl->maxdisp2);
+                   (const int*)Ty.d, h->cap, n, 0.5 * dt, dt, sphk<double>(sp), maxd2, guard);
     else
         pd::launch(k_sph_kick_drift<float>, nblk, 256, 0, st, (float4*)h->pos, (const float4*)xb.as<float4>(),
                    aux.as<float4>(), (float*)V.d, (const float*)A.d, (float*)R.d, (const float*)D.d,
-                   (const int*)Ty.d, h->cap, n, (float)(0.5 * dt), (float)dt, sphk<float>(sp), &h->ctrl->maxdisp2);
+                   (const int*)Ty.d, h->cap, n, (float)(0.5 * dt), (float)dt, sphk<float>(sp), maxd2, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
@@ -449,7 +453,8 @@ int sph_kick(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int acc_prop, int
 }
 
 int sph_kick_kick_drift(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int acc_prop, const Buf& xb, Buf& aux,
-                        int nblk, double dt, double* kpart, double* rpart, cudaStream_t st) {
+                        int nblk, double dt, double* kpart, double* rpart, unsigned long long* maxd2,
+                        const StepGuard& guard, cudaStream_t st) {
     long n = h->n_real;
     const Prop& V = h->props[vel_prop];
     const Prop& A = h->props[acc_prop];
@@ -460,12 +465,12 @@ int sph_kick_kick_drift(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int ac
         pd::launch(k_sph_kick_kick_drift<double>, nblk, 256, 0, st, (double4*)h->pos,
                    (const double4*)xb.as<double4>(), aux.as<double4>(), (double*)V.d, (const double*)A.d,
                    (double*)R.d, (const double*)D.d, (const int*)Ty.d, h->cap, n, 0.5 * dt, dt, sphk<double>(sp),
-                   sp.mass, &h->ctrl->maxdisp2, kpart, rpart);
+                   sp.mass, maxd2, kpart, rpart, guard);
     else
         pd::launch(k_sph_kick_kick_drift<float>, nblk, 256, 0, st, (float4*)h->pos, (const float4*)xb.as<float4>(),
                    aux.as<float4>(), (float*)V.d, (const float*)A.d, (float*)R.d, (const float*)D.d,
                    (const int*)Ty.d, h->cap, n, (float)(0.5 * dt), (float)dt, sphk<float>(sp), sp.mass,
-                   &h->ctrl->maxdisp2, kpart, rpart);
+                   maxd2, kpart, rpart, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
@@ -473,7 +478,7 @@ int sph_kick_kick_drift(pd_vd h, const pd_sph_params_t& sp, int vel_prop, int ac
 template <class T, int P>
 static int launch_sph(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, unsigned int cap,
                       const Buf& nbr, const Buf& nn, long stride, const Buf& aux, const pd_sph_params_t& sp,
-                      int acc_prop, cudaStream_t st) {
+                      int acc_prop, const StepGuard& guard, cudaStream_t st) {
     typedef typename V4<T>::type T4;
     int smem = (int)(2 * cap * sizeof(T4));
     if (smem < 32) smem = 32;
@@ -485,22 +490,22 @@ static int launch_sph(pd_vd h, const TileGeom& tg, long ntiles, const unsigned i
     pd::launch(k_vtile_sph<T, P>, (unsigned)ntiles, FBLOCK_T, (size_t)smem, st, (const T4*)h->pos,
                (const T4*)aux.as<T4>(), tg, csR, cap, (const unsigned int*)nbr.as<unsigned int>(),
                (const int*)nn.as<int>(), stride, mwords, (const int*)Ty.d, sphk<T>(sp), (T*)A.d, (T*)D.d, h->cap,
-               &h->ctrl->err);
+               &h->ctrl->err, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
 
 int sph_rates(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, unsigned int cap, const Buf& nbr,
               const Buf& nn, long stride, const Buf& aux, const pd_sph_params_t& sp, int acc_prop, int P,
-              cudaStream_t st) {
+              cudaStream_t st, const StepGuard& guard) {
     if (h->dtype == PD_F64) {
-        if (P == 4) return launch_sph<double, 4>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
-        if (P == 1) return launch_sph<double, 1>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
-        return launch_sph<double, 2>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
+        if (P == 4) return launch_sph<double, 4>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
+        if (P == 1) return launch_sph<double, 1>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
+        return launch_sph<double, 2>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
     }
-    if (P == 4) return launch_sph<float, 4>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
-    if (P == 1) return launch_sph<float, 1>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
-    return launch_sph<float, 2>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, st);
+    if (P == 4) return launch_sph<float, 4>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
+    if (P == 1) return launch_sph<float, 1>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
+    return launch_sph<float, 2>(h, tg, ntiles, csR, cap, nbr, nn, stride, aux, sp, acc_prop, guard, st);
 }
 
 bool sph_tile_fits(pd_vd h, unsigned int tmax) { return 2L * tmax * h->pos_bytes <= 200L * 1024 && tmax <= 65535u; }

@@ -131,8 +131,9 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_lj(const typename V4<T>::typ
                                                        const unsigned int* __restrict__ nbr,
                                                        const int* __restrict__ nn, long stride, LJP<T> Pr,
                                                        T* __restrict__ f, long fcap, double* __restrict__ part,
-                                                       unsigned int* __restrict__ err) {
+                                                       unsigned int* __restrict__ err, StepGuard guard) {
     typedef typename V4<T>::type T4;
+    if (step_skipped(guard)) return;
     extern __shared__ __align__(128) unsigned char tile_raw[];
     T4* sm = reinterpret_cast<T4*>(tile_raw);
     __shared__ TileSh S;
@@ -231,7 +232,9 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_lj(const typename V4<T>::typ
 // copies and z as 8-byte values loaded by the CTA (their ranges need not start on
 // a 16-byte boundary), 24 bytes a record instead of 32; (x, y) records of
 // consecutive slots fall on all eight 16-byte bank groups.
-template <bool ENERGY, int P, int MINB, bool DRIFT>
+// STEP 0: forces; 1: the step's closing kick and the next step's kick and drift; 2: the
+// closing kick and forces (DriftArgs)
+template <bool ENERGY, int P, int MINB, int STEP>
 __global__ void __launch_bounds__(FBLOCK_T, MINB) k_vtile_lj_xyz(const double2* __restrict__ xy,
                                                            const double* __restrict__ zz, long n_real, TileGeom tg,
                                                            const unsigned int* __restrict__ csR,
@@ -241,8 +244,10 @@ __global__ void __launch_bounds__(FBLOCK_T, MINB) k_vtile_lj_xyz(const double2* 
                                                            LJP<double> Pr,
                                                            double* __restrict__ f, long fcap,
                                                            double* __restrict__ part, unsigned int* __restrict__ err,
-                                                           DriftArgs D) {
-    static_assert(ENERGY || !DRIFT, "the drift's kinetic energy partials ride on the energy partials");
+                                                           DriftArgs D, StepGuard guard) {
+    static_assert(ENERGY || STEP == 0, "the kinetic energy partials ride on the energy partials");
+    constexpr bool DRIFT = STEP == 1;
+    if (step_skipped(guard)) return;
     extern __shared__ __align__(128) unsigned char tile_raw[];
     double2* sxy = reinterpret_cast<double2*>(tile_raw);
     double* sz = reinterpret_cast<double*>(tile_raw + (size_t)cap * sizeof(double2));
@@ -308,13 +313,15 @@ __global__ void __launch_bounds__(FBLOCK_T, MINB) k_vtile_lj_xyz(const double2* 
             unsigned int q2 = sub + 2 * Q < mwords ? __ldg(row + (long)(sub + 2 * Q) * stride) : 0u;
             unsigned int q3 = sub + 3 * Q < mwords ? __ldg(row + (long)(sub + 3 * Q) * stride) : 0u;
             const int words = active ? (nn[i] + 1) >> 1 : 0;
-            if (DRIFT && active && sub == 0) {
-                // the drift's operands into L2 while the row is computed
+            if (STEP != 0 && active && sub == 0) {
+                // the kick's and drift's operands into L2 while the row is computed
                 prefetch_l2(D.v + i);
                 prefetch_l2(D.v + D.vcap + i);
                 prefetch_l2(D.v + 2 * D.vcap + i);
-                prefetch_l2(D.pos + i);
-                prefetch_l2(D.xb + i);
+                if (DRIFT) {
+                    prefetch_l2(D.pos + i);
+                    prefetch_l2(D.xb + i);
+                }
             }
             double fx = 0, fy = 0, fz = 0, e = 0, w = 0;
             // one pair (rows hold the particle itself, as the reference's full list
@@ -358,6 +365,16 @@ __global__ void __launch_bounds__(FBLOCK_T, MINB) k_vtile_lj_xyz(const double2* 
                 }
             }
             if (active && sub == 0) {
+                if (STEP == 2) {
+                    const long vc = D.vcap;
+                    const double vx = D.v[i] + D.half * fx;
+                    const double vy = D.v[vc + i] + D.half * fy;
+                    const double vz = D.v[2 * vc + i] + D.half * fz;
+                    D.v[i] = vx;
+                    D.v[vc + i] = vy;
+                    D.v[2 * vc + i] = vz;
+                    ke += 0.5 * D.mass * (vx * vx + vy * vy + vz * vz);
+                }
                 if (DRIFT) {
                     const long vc = D.vcap;
                     double vx = D.v[i] + D.half * fx;
@@ -395,9 +412,9 @@ __global__ void __launch_bounds__(FBLOCK_T, MINB) k_vtile_lj_xyz(const double2* 
     if (ENERGY) {
         pe = block_sum<double, FBLOCK_T>(pe);
         vir = block_sum<double, FBLOCK_T>(vir);
-        if (DRIFT) ke = block_sum<double, FBLOCK_T>(ke);
+        if (STEP != 0) ke = block_sum<double, FBLOCK_T>(ke);
         if (threadIdx.x == 0) {
-            if (DRIFT) {
+            if (STEP != 0) {
                 part[3 * blockIdx.x] = pe;
                 part[3 * blockIdx.x + 1] = vir;
                 part[3 * blockIdx.x + 2] = ke;
@@ -606,18 +623,18 @@ int tile_split(pd_vd h, Buf& sxy, Buf& sz, long first, long n, cudaStream_t st) 
     return PD_OK;
 }
 
-template <bool E, int P, int MINB, bool DRIFT>
+template <bool E, int P, int MINB, int STEP>
 static int launch_lj_xyz_k(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                            unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const LJP<double>& LP,
                            double* f, double* part, const Buf& sxy, const Buf& sz, const DriftArgs& D,
-                           cudaStream_t st) {
+                           const StepGuard& guard, cudaStream_t st) {
     int smem = (int)(cap * 24);
     if (smem < 32) smem = 32;
     const int mwords = (int)std::min<long>((long)(nbr.bytes / (4 * (size_t)stride)), 1L << 30);
-    PD_TRY(allow_smem(k_vtile_lj_xyz<E, P, MINB, DRIFT>, smem));
-    pd::launch(k_vtile_lj_xyz<E, P, MINB, DRIFT>, (unsigned)ntiles, FBLOCK_T, (size_t)smem, st,
+    PD_TRY(allow_smem(k_vtile_lj_xyz<E, P, MINB, STEP>, smem));
+    pd::launch(k_vtile_lj_xyz<E, P, MINB, STEP>, (unsigned)ntiles, FBLOCK_T, (size_t)smem, st,
                (const double2*)sxy.as<double2>(), (const double*)sz.as<double>(), h->n_real, tg, csR, csI, cap,
-               nbr.as<unsigned int>(), nn.as<int>(), stride, mwords, LP, f, h->cap, part, &h->ctrl->err, D);
+               nbr.as<unsigned int>(), nn.as<int>(), stride, mwords, LP, f, h->cap, part, &h->ctrl->err, D, guard);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }
@@ -625,19 +642,22 @@ static int launch_lj_xyz_k(pd_vd h, const TileGeom& tg, long ntiles, const unsig
 template <bool E, int P, int MINB>
 static int launch_lj_xyz(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                          unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const LJP<double>& LP, double* f,
-                         double* part, const Buf& sxy, const Buf& sz, const DriftArgs* drift, cudaStream_t st) {
+                         double* part, const Buf& sxy, const Buf& sz, const DriftArgs* drift, const StepGuard& guard,
+                         cudaStream_t st) {
     if (!sxy.p || !sz.p) {
         set_error("tile_lj: the FP64 staging copies were not made");
         return PD_ESTATE;
     }
-    if (!drift) return launch_lj_xyz_k<E, P, MINB, false>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part,
-                                                          sxy, sz, DriftArgs{}, st);
-    if (!E || !drift->sxy_next || !drift->sz_next || drift->sxy_next == sxy.as<double2>()) {
+    if (!drift) return launch_lj_xyz_k<E, P, MINB, 0>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part,
+                                                      sxy, sz, DriftArgs{}, guard, st);
+    if (!E || (!drift->close && (!drift->sxy_next || !drift->sz_next || drift->sxy_next == sxy.as<double2>()))) {
         set_error("tile_lj: a drift needs the energy partials and a second pair of staging copies");
         return PD_EINVAL;
     }
-    return launch_lj_xyz_k<E, P, MINB, E>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part, sxy, sz, *drift,
-                                          st);
+    if (drift->close) return launch_lj_xyz_k<E, P, MINB, E ? 2 : 0>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP,
+                                                                    f, part, sxy, sz, *drift, guard, st);
+    return launch_lj_xyz_k<E, P, MINB, E ? 1 : 0>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part, sxy, sz,
+                                                  *drift, guard, st);
 }
 
 // FP32 storage: the 16-byte records
@@ -645,7 +665,8 @@ template <class T, bool E, int P>
 struct LjLaunch {
     static int run(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                    unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const LJP<T>& LP, T* f, double* part,
-                   const Buf& sxy, const Buf& sz, int smem, const DriftArgs* drift, cudaStream_t st) {
+                   const Buf& sxy, const Buf& sz, int smem, const DriftArgs* drift, const StepGuard& guard,
+                   cudaStream_t st) {
         (void)sxy;
         (void)sz;
         if (drift) {
@@ -655,7 +676,7 @@ struct LjLaunch {
         PD_TRY(allow_smem(k_vtile_lj<T, E, P>, smem));
         pd::launch(k_vtile_lj<T, E, P>, (unsigned)ntiles, FBLOCK_T, (size_t)smem, st,
                    (const typename V4<T>::type*)h->pos, h->n_real, tg, csR, csI, cap, nbr.as<unsigned int>(),
-                   nn.as<int>(), stride, LP, f, h->cap, part, &h->ctrl->err);
+                   nn.as<int>(), stride, LP, f, h->cap, part, &h->ctrl->err, guard);
         PD_LAUNCH_CHECK();
         return PD_OK;
     }
@@ -665,9 +686,11 @@ template <bool E, int P>
 struct LjLaunch<double, E, P> {
     static int run(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                    unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const LJP<double>& LP, double* f,
-                   double* part, const Buf& sxy, const Buf& sz, int smem, const DriftArgs* drift, cudaStream_t st) {
+                   double* part, const Buf& sxy, const Buf& sz, int smem, const DriftArgs* drift,
+                   const StepGuard& guard, cudaStream_t st) {
         (void)smem;
-        return launch_lj_xyz<E, P, 4>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part, sxy, sz, drift, st);
+        return launch_lj_xyz<E, P, 4>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part, sxy, sz, drift,
+                                      guard, st);
     }
 };
 
@@ -675,7 +698,7 @@ template <class T>
 static int tile_lj_t(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                      unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const pd_lj_params_t& lj, T* f,
                      double* part, bool energy, int P, const Buf& sxy, const Buf& sz, int smem,
-                     const DriftArgs* drift, cudaStream_t st) {
+                     const DriftArgs* drift, const StepGuard& guard, cudaStream_t st) {
     LJP<T> LP{};
     LP.eps24 = (T)(24.0 * lj.eps);
     LP.eps4 = (T)(4.0 * lj.eps);
@@ -685,7 +708,7 @@ static int tile_lj_t(pd_vd h, const TileGeom& tg, long ntiles, const unsigned in
 #define PD_LJ_CASE(E, PP)                                                                                         \
     if (energy == E && P == PP)                                                                                   \
         return LjLaunch<T, E, PP>::run(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, LP, f, part, sxy, sz, smem, \
-                                       drift, st);
+                                       drift, guard, st);
     PD_LJ_CASE(true, 1)
     PD_LJ_CASE(true, 2)
     PD_LJ_CASE(true, 4)
@@ -699,16 +722,16 @@ static int tile_lj_t(pd_vd h, const TileGeom& tg, long ntiles, const unsigned in
 
 int tile_lj(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
             unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const pd_lj_params_t& lj, int force_prop,
-            double* part, bool energy, int P, const Buf& sxy, const Buf& sz, cudaStream_t st,
-            const DriftArgs* drift) {
+            double* part, bool energy, int P, const Buf& sxy, const Buf& sz, cudaStream_t st, const DriftArgs* drift,
+            const StepGuard& guard) {
     Prop& F = h->props[force_prop];
     int smem = (int)(cap * h->pos_bytes);
     if (smem < 16) smem = 16;
     if (h->dtype == PD_F64)
         return tile_lj_t<double>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, lj, (double*)F.d, part, energy, P,
-                                 sxy, sz, smem, drift, st);
+                                 sxy, sz, smem, drift, guard, st);
     return tile_lj_t<float>(h, tg, ntiles, csR, csI, cap, nbr, nn, stride, lj, (float*)F.d, part, energy, P, sxy,
-                            sz, smem, drift, st);
+                            sz, smem, drift, guard, st);
 }
 
 int tile_translate(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,

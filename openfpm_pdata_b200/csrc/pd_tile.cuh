@@ -13,6 +13,22 @@ struct TileGeom {
     int TX, ntx, ny, nz;
 };
 
+// Steps enqueued ahead of their rebuild decision (pd_md_run): a kernel of a step whose
+// slot holds a squared displacement above lim2 does nothing but mark the next slot, so
+// that every later step of the batch does nothing either.  slot nullptr: always runs.
+struct StepGuard {
+    const unsigned long long* slot = nullptr;
+    unsigned long long* next = nullptr;
+    double lim2 = 0;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ bool step_skipped(const StepGuard& g) {
+    if (!g.slot || !(__longlong_as_double((long long)*g.slot) > g.lim2)) return false;
+    if (g.next && blockIdx.x == 0 && threadIdx.x == 0) *g.next = 0x7ff0000000000000ull;  // infinity
+    return true;
+}
+#endif
+
 int tile_plan(pd_cl cl, long n_real, int TX_req, TileGeom& tg, long& ntiles);
 int tile_sizes(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                unsigned int& tmax, unsigned int& cmax, cudaStream_t st);
@@ -34,8 +50,10 @@ int tile_split(pd_vd h, Buf& sxy, Buf& sz, long first, long n, cudaStream_t st);
 // kernel, in its order), the drifted position into the vector and into the other
 // pair of staging copies (the pair kernel still reads the current ones), and the
 // largest |x - x_build|^2 into *maxd2.  The force itself is not stored: the next
-// step recomputes it before anything reads it.
+// step recomputes it before anything reads it.  With `close` (a run's last step) only the
+// closing half kick is made and the force is stored.
 struct DriftArgs {
+    bool close;
     double4* pos;
     const double4* xb;
     double* v;
@@ -46,11 +64,11 @@ struct DriftArgs {
     unsigned long long* maxd2;
 };
 // LJ forces from the tiled rows (FP64: from the staging copies sxy / sz, which must be
-// current).  Per tile, part receives (pe, vir), or (pe, vir, ke) with a drift.
+// current).  Per tile, part receives (pe, vir), or (pe, vir, ke) with `drift`.
 int tile_lj(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
             unsigned int cap, const Buf& nbr, const Buf& nn, long stride, const pd_lj_params_t& lj, int force_prop,
             double* part, bool energy, int P, const Buf& sxy, const Buf& sz, cudaStream_t st,
-            const DriftArgs* drift = nullptr);
+            const DriftArgs* drift = nullptr, const StepGuard& guard = StepGuard());
 int tile_translate(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
                    const Buf& nbr, const Buf& nn, long stride, int max_nn, int* out_dev, cudaStream_t st);
 
