@@ -61,6 +61,7 @@ struct Ctrl {
     unsigned int tile_center_max;  // largest number of domain particles of a tile
     unsigned int tile_pass_max;    // largest staged z-layer (3 rows) of a tile (records)
     unsigned int n_keep;           // count of the last compaction / index selection
+    unsigned int run_done;         // steps made by the last bucket run (pd_cluster.cu)
 };
 
 // Allocation context: inside an AllocScope, device allocations of the library are

@@ -1053,6 +1053,7 @@ int pd_md_destroy(pd_md md) {
     md->rpart.release();
     md->eidx.release();
     md->slots.release();
+    md->buckets.release();
     if (md->slots_h) cudaFreeHost(md->slots_h);
     if (md->gcl) cudaGraphExecDestroy(md->gcl);
     if (md->gst) cudaStreamDestroy(md->gst);

@@ -1,0 +1,84 @@
+"""The cell-list driver's bucket kernel against the FP64 oracle and the one-cluster kernel
+it hands over to: the smallest systems, a box of few cells, open boundaries, FP32 storage,
+and a system whose densest cell overflows a bucket.  A run equals runs of one step and a
+second identical run bit for bit (the order in which buckets fill does not matter)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+F32, F64 = np.float32, np.float64
+
+
+@pytest.fixture(scope="module")
+def pd():
+    from openfpm_pdata_b200 import pd as _pd
+    _pd.lib()
+    return _pd
+
+
+def _md(pd, x, v, L, bc, dtype, dt=0.002):
+    t = pd.PD_F64 if dtype == F64 else pd.PD_F32
+    vd = pd.VectorDist(x.shape[0], np.zeros(3), np.full(3, L), np.asarray(bc, np.int32), 2.5, dtype=dtype,
+                       props=[(t, 3), (t, 3), (pd.PD_I32, 1)])
+    vd.hostToDevicePos(x.astype(dtype))
+    vd.hostToDeviceProp(0, v)
+    vd.hostToDeviceProp(2, np.arange(x.shape[0]))
+    return vd, pd.MD(vd, 0, 1, dt=dt, skin=0.0, use_cell_list=True)
+
+
+def _by_id(vd):
+    i = vd.deviceToHostProp(2, with_ghost=False)
+    x, v = vd.deviceToHostPos(with_ghost=False), vd.deviceToHostProp(0, with_ghost=False)
+    xo, vo = np.empty_like(x), np.empty_like(v)
+    xo[i], vo[i] = x, v
+    return xo, vo
+
+
+def _system(kind):
+    from openfpm_pdata_b200 import workloads
+    if kind == "one":
+        return np.array([[1.0, 7.9, 0.1]]), np.array([[3.0, 2.0, -4.0]]), 8.0
+    if kind == "clump":  # 1728 particles at spacing 1.0 in a corner of a box of 30: 15.6 a cell there, 0.2 on average
+        x, v, _ = workloads.lj_lattice(12, 0.98, 0.03, seed=4)
+        return x + 0.5, v * 0.3, 60.0
+    side, sp = {"few cells": (8, 1.02), "c1": (16, 1.0), "many": (33, 1.05)}[kind]
+    return workloads.lj_lattice(side, sp, 0.05, seed=5)
+
+
+@pytest.mark.parametrize("kind", ["one", "few cells", "c1", "many", "clump"])
+def test_follows_the_oracle(pd, orc, kind):
+    x, v, L = _system(kind)
+    steps = 6 if kind == "many" else 25
+    lo, hi, bc = np.zeros(3), np.full(3, L), np.ones(3, np.int32)
+    vd, md = _md(pd, x, v, L, bc, F64)
+    E = np.concatenate([md.run(2), md.run(steps - 2)])
+    xo, vo, Eo = orc.md_lj(x, v, lo, hi, bc, 2.5, 2.5, 0.0, 1.0, 1.0, 0.002, 1.0, steps)
+    np.testing.assert_allclose(E[:, :3], Eo[1:, :3], rtol=1e-9, atol=1e-9)
+    gx, gv = _by_id(vd)
+    d = gx - xo
+    d -= L * np.round(d / L)
+    assert np.abs(d).max() < 1e-9
+    # the images belong to the last positions, with their properties
+    n = vd.size_local()
+    pos = vd.deviceToHostPos()
+    img, src, _ = orc.ghost_get(pos[:n], lo, hi, bc, 2.5)
+    assert np.array_equal(pos[n:], img)
+    assert np.array_equal(vd.deviceToHostProp(0)[n:], vd.deviceToHostProp(0)[:n][src])
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("kind", ["few cells", "c1", "clump"])
+@pytest.mark.parametrize("bc", [(1, 1, 1), (1, 0, 1)])
+def test_run_equals_single_steps(pd, dtype, kind, bc):
+    x, v, L = _system(kind)
+    if bc != (1, 1, 1):
+        v = v * [1.0, 0.1, 1.0]
+    runs = []
+    for parts in ([17], [17], [1] * 17):
+        vd, md = _md(pd, x, v, L, bc, dtype)
+        E = np.concatenate([md.run(k) for k in parts])
+        runs.append((E,) + _by_id(vd))
+    assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[1]))
+    if kind != "clump":  # (there the two kernels share the runs differently)
+        assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[2]))
