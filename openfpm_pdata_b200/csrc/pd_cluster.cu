@@ -567,7 +567,7 @@ __device__ __forceinline__ void cb_advance(const CbArgs<T>& A, const BoxSet<T>& 
 }
 
 template <class T>
-__global__ void __launch_bounds__(CB_THREADS) k_md_buckets(CbArgs<T> A) {
+__global__ void __launch_bounds__(CB_THREADS, 3) k_md_buckets(CbArgs<T> A) {
     typedef typename V4<T>::type T4;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char cb_raw[];
@@ -575,6 +575,7 @@ __global__ void __launch_bounds__(CB_THREADS) k_md_buckets(CbArgs<T> A) {
     __shared__ BoxSet<T> B;
     __shared__ unsigned int num[27], off[28], cellid[27];
     __shared__ int keys[CB_THREADS / 32][CB_MAXCAP];
+    __shared__ double esum[3][CB_THREADS / 32];
     for (int i = threadIdx.x; i < (int)(sizeof(BoxSet<T>) / 4); i += blockDim.x)
         reinterpret_cast<int*>(&B)[i] = reinterpret_cast<const int*>(A.boxes)[i];
     __syncthreads();
@@ -666,13 +667,20 @@ __global__ void __launch_bounds__(CB_THREADS) k_md_buckets(CbArgs<T> A) {
             const unsigned int me = oc + (active ? (unsigned int)q : 0u);
             const T4 xi = sp[me];
             T fx = 0, fy = 0, fz = 0, e = 0, w = 0;
-            if (active)
+            // (v, f) of the particle while the pairs are computed
+            const int i = idx_of<T>(xi.w);
+            T vx = 0, vy = 0, vz = 0;
+            if (active) {
+                vx = __ldcg(A.v + i) + A.half * __ldcg(A.f + i);
+                vy = __ldcg(A.v + A.cap + i) + A.half * __ldcg(A.f + A.cap + i);
+                vz = __ldcg(A.v + 2 * A.cap + i) + A.half * __ldcg(A.f + 2 * A.cap + i);
                 for (unsigned int k = sub; k < M; k += L) {
                     const T4 xq = sp[k];
                     const T dx = xi.x - xq.x, dy = xi.y - xq.y, dz = xi.z - xq.z;
                     const T r2 = dist2(dx, dy, dz);
                     if (r2 < A.P.rc2 && k != me) lj_acc(A.P, r2, dx, dy, dz, fx, fy, fz, e, w);
                 }
+            }
             for (int o = 1; o < L; o <<= 1) {
                 fx += __shfl_xor_sync(0xffffffffu, fx, o);
                 fy += __shfl_xor_sync(0xffffffffu, fy, o);
@@ -682,10 +690,6 @@ __global__ void __launch_bounds__(CB_THREADS) k_md_buckets(CbArgs<T> A) {
             }
             const unsigned int group = __ballot_sync(0xffffffffu, active);
             if (active) {
-                const int i = idx_of<T>(xi.w);
-                T vx = __ldcg(A.v + i) + A.half * __ldcg(A.f + i);
-                T vy = __ldcg(A.v + A.cap + i) + A.half * __ldcg(A.f + A.cap + i);
-                T vz = __ldcg(A.v + 2 * A.cap + i) + A.half * __ldcg(A.f + 2 * A.cap + i);
                 vx = vx + A.half * fx;
                 vy = vy + A.half * fy;
                 vz = vz + A.half * fz;
@@ -705,17 +709,23 @@ __global__ void __launch_bounds__(CB_THREADS) k_md_buckets(CbArgs<T> A) {
             }
             __syncthreads();
         }
-        pe = block_sum<double, CB_THREADS>(pe);
-        vir = block_sum<double, CB_THREADS>(vir);
-        ke = block_sum<double, CB_THREADS>(ke);
-        if (threadIdx.x == 0) {
-            double* pt = A.part + 3 * ((long)(s & 1) * gridDim.x + blockIdx.x);
-            pt[0] = pe;
-            pt[1] = vir;
-            pt[2] = ke;
+        pe = warp_sum(pe);
+        vir = warp_sum(vir);
+        ke = warp_sum(ke);
+        if (lane == 0) {
+            esum[0][warp] = pe;
+            esum[1][warp] = vir;
+            esum[2][warp] = ke;
+        }
+        __syncthreads();
+        if (threadIdx.x < 3) {
+            double t = 0;
+            for (int k = 0; k < CB_THREADS / 32; ++k) t += esum[threadIdx.x][k];
+            A.part[3 * ((long)(s & 1) * gridDim.x + blockIdx.x) + threadIdx.x] = t;
         }
         alive = grid_barrier(cluster, A.bar, target += nclusters, A.err);
-        if (blockIdx.x == 0) {  // the step's energies, while the other CTAs go on
+        // the step's energies while the other CTAs go on, by the last CTA (of the fewest cells)
+        if (blockIdx.x == gridDim.x - 1) {
             const double* pt = A.part + 3 * (long)(s & 1) * gridDim.x;
             double a = 0, b = 0, c = 0;
             for (unsigned int r = threadIdx.x; r < gridDim.x; r += CB_THREADS) {
