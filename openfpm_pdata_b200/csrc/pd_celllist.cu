@@ -156,19 +156,7 @@ int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cud
     return PD_OK;
 }
 
-// gather: dst[k] = src[ids[k]] of one column
-template <class T>
-__global__ void k_gather4(const typename V4<T>::type* __restrict__ src, typename V4<T>::type* __restrict__ dst,
-                          const int* __restrict__ ids, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        st4(dst, k, ld4(src, ids[k]));
-}
-template <class E>
-__global__ void k_gather(const E* __restrict__ src, E* __restrict__ dst, const int* __restrict__ ids, long n) {
-    for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x)
-        dst[k] = src[ids[k]];
-}
-// the same for up to GCOLS columns at once (positions, global ids, property components):
+// gather dst[k] = src[ids[k]] of up to GCOLS columns (positions, global ids, property components):
 // each permutation entry read once; a column's element is 4, 8, 16 or 32 bytes
 static constexpr int GCOLS = 16;
 struct GatherCols {
@@ -228,8 +216,10 @@ template <int MODE> __global__ void k_move_cols(const int* __restrict__ ids, lon
                 reinterpret_cast<double2*>(G.dst[c])[to] = __ldg(reinterpret_cast<const double2*>(G.src[c]) + from);
             } else if (es == 8) {
                 reinterpret_cast<long long*>(G.dst[c])[to] = __ldg(reinterpret_cast<const long long*>(G.src[c]) + from);
-            } else {
+            } else if (es == 4) {
                 reinterpret_cast<int*>(G.dst[c])[to] = __ldg(reinterpret_cast<const int*>(G.src[c]) + from);
+            } else {
+                G.dst[c][to] = __ldg(G.src[c] + from);
             }
         }
     }
@@ -239,36 +229,23 @@ template <int MODE> __global__ void k_move_cols(const int* __restrict__ ids, lon
 // scratch in one kernel and back in another.  A kernel and a copy for each column were
 // bound by their launches on small systems: 4,099 FP64 particles, reorder and
 // restoreOrder of four columns together 41 us of GPU time in 20 launches.
-static int permute(pd_vd h, const int* ids, long n, unsigned long prop_mask, bool with_pos, bool with_gid,
-                   bool restore, cudaStream_t st) {
+int permute_columns(pd_vd h, const MoveCol* cols, int ncols, const int* ids, long n, bool restore, cudaStream_t st) {
     if (n <= 0) return PD_OK;
-    struct Col {
-        char* p;
-        int es;
-    };
-    std::vector<Col> cols;
-    if (with_pos) cols.push_back({(char*)h->pos, (int)h->pos_bytes});
-    if (with_gid) cols.push_back({(char*)h->gid, 4});
-    for (size_t p = 0; p < h->props.size(); ++p) {
-        if (!(prop_mask & (1ul << p))) continue;
-        Prop& P = h->props[p];
-        for (int c = 0; c < P.ncomp; ++c) cols.push_back({P.d + (size_t)c * h->cap * P.esize, P.esize});
-    }
     const unsigned g = grid_for(n, 256);
-    auto room = [&](size_t c) { return ((size_t)n * cols[c].es + 255) & ~(size_t)255; };  // aligned scratch columns
-    for (size_t c0 = 0; c0 < cols.size(); c0 += GCOLS) {
-        const size_t c1 = std::min(cols.size(), c0 + (size_t)GCOLS);
+    auto room = [&](int c) { return ((size_t)n * cols[c].esize + 255) & ~(size_t)255; };  // aligned scratch columns
+    for (int c0 = 0; c0 < ncols; c0 += GCOLS) {
+        const int c1 = std::min(ncols, c0 + GCOLS);
         size_t bytes = 0;
-        for (size_t c = c0; c < c1; ++c) bytes += room(c);
+        for (int c = c0; c < c1; ++c) bytes += room(c);
         PD_TRY(h->tmp2.ensure(bytes));
         GatherCols out{}, back{};
-        out.ncol = back.ncol = (int)(c1 - c0);
+        out.ncol = back.ncol = c1 - c0;
         char* t = h->tmp2.as<char>();
-        for (size_t c = c0; c < c1; ++c) {
-            out.src[c - c0] = back.dst[c - c0] = cols[c].p;
+        for (int c = c0; c < c1; ++c) {
+            out.src[c - c0] = back.dst[c - c0] = (char*)cols[c].p;
             out.dst[c - c0] = t;
             back.src[c - c0] = t;
-            out.esize[c - c0] = back.esize[c - c0] = cols[c].es;
+            out.esize[c - c0] = back.esize[c - c0] = cols[c].esize;
             t += room(c);
         }
         if (restore) pd::launch(k_move_cols<1>, g, 256, 0, st, ids, n, out);
@@ -279,19 +256,17 @@ static int permute(pd_vd h, const int* ids, long n, unsigned long prop_mask, boo
     return PD_OK;
 }
 
-int gather_bytes(const void* src, void* dst, const int* ids, long n, int esize, cudaStream_t st) {
-    if (n <= 0) return PD_OK;
-    unsigned g = grid_for(n, 256);
-    switch (esize) {
-        case 1: pd::launch(k_gather<unsigned char>, g, 256, 0, st, (const unsigned char*)src, (unsigned char*)dst, ids, n); break;
-        case 4: pd::launch(k_gather<int>, g, 256, 0, st, (const int*)src, (int*)dst, ids, n); break;
-        case 8: pd::launch(k_gather<long long>, g, 256, 0, st, (const long long*)src, (long long*)dst, ids, n); break;
-        case 16: pd::launch(k_gather4<float>, g, 256, 0, st, (const float4*)src, (float4*)dst, ids, n); break;
-        case 32: pd::launch(k_gather4<double>, g, 256, 0, st, (const double4*)src, (double4*)dst, ids, n); break;
-        default: set_error("gather_bytes: element size %d", esize); return PD_EINVAL;
+static int permute(pd_vd h, const int* ids, long n, unsigned long prop_mask, bool with_pos, bool with_gid,
+                   bool restore, cudaStream_t st) {
+    std::vector<MoveCol> cols;
+    if (with_pos) cols.push_back({h->pos, (int)h->pos_bytes});
+    if (with_gid) cols.push_back({h->gid, 4});
+    for (size_t p = 0; p < h->props.size(); ++p) {
+        if (!(prop_mask & (1ul << p))) continue;
+        Prop& P = h->props[p];
+        for (int c = 0; c < P.ncomp; ++c) cols.push_back({P.d + (size_t)c * h->cap * P.esize, P.esize});
     }
-    PD_LAUNCH_CHECK();
-    return PD_OK;
+    return permute_columns(h, cols.data(), (int)cols.size(), ids, n, restore, st);
 }
 
 // The gather of a reorder straight into the vector's spare storage, which then

@@ -223,8 +223,13 @@ int read_ctrl(pd_vd h, cudaStream_t st);
 int cl_geometry(pd_cl cl, pd_vd h, double r_cut, double enlarge, int nn_box);
 // counting sort of the particles [first, first + n_part) (ids relative to `first`)
 int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cudaStream_t st, long first = 0);
-// gather src[ids[k]] -> dst[k] for k < n of 4/8/16/32-byte elements (dst may not alias src)
-int gather_bytes(const void* src, void* dst, const int* ids, long n, int esize, cudaStream_t st);
+// columns of n elements of 1, 4, 8, 16 or 32 bytes permuted in place: element k from ids[k],
+// or with `restore` to ids[k]
+struct MoveCol {
+    void* p;
+    int esize;
+};
+int permute_columns(pd_vd h, const MoveCol* cols, int ncols, const int* ids, long n, bool restore, cudaStream_t st);
 // Further outputs of the reorder of FP64 positions into spare storage: the reordered
 // records also to `xb` and as (x, y) / z copies to `sxy` / `sz` (room for n_part);
 // *done tells whether they were written (not by the in-place reorder)

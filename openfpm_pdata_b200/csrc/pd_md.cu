@@ -510,6 +510,13 @@ int force_blocks(long n) {
     return (int)want;
 }
 
+int md_auto_width(pd_vd h, pd_cl cl, long n, double want) {
+    double inner = 1;
+    for (int d = 0; d < 3; ++d) inner *= std::max(1.0, (h->hi[d] - h->lo[d]) / cl->spacing[d]);
+    const double occ = std::max((double)n / inner, 1e-3);
+    return std::max(1, std::min(TXMAX, (int)(want / occ)));
+}
+
 // the plain FP64 tiled LJ path (its pair kernel also kicks and drifts)
 static bool md_split_possible(pd_md md) {
     return md->physics == 0 && !md->mixed && !md->mp.use_cell_list && md->h->dtype == PD_F64;
@@ -519,28 +526,19 @@ static bool md_split_possible(pd_md md) {
 // their cell starts); sort the images by cell too, then build the tile-local rows.
 static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
     pd_vd h = md->h;
-    long nc1 = cl->ncells + 1;
-    PD_TRY(md->csR.ensure(sizeof(unsigned int) * nc1));
-    PD_TRY(md->csI.ensure(sizeof(unsigned int) * nc1));
-    PD_CUDA(cudaMemcpyAsync(md->csR.p, cl->cell_start.p, sizeof(unsigned int) * nc1, cudaMemcpyDeviceToDevice, st));
+    // the cell starts of the real particles, then of the images: the list's buffer and the
+    // driver's change places
+    std::swap(md->csR, cl->cell_start);
     long m = h->n_img, n = h->n_real;
     PD_TRY(cl_build(h, cl, m, nullptr, st, n));
-    PD_CUDA(cudaMemcpyAsync(md->csI.p, cl->cell_start.p, sizeof(unsigned int) * nc1, cudaMemcpyDeviceToDevice, st));
+    std::swap(md->csI, cl->cell_start);
     h->img_gen_order = false;  // the images are sorted into cell order below
-    if (m > 0) {
-        const int* ids = cl->sorted.as<int>();
-        size_t need = std::max((size_t)m * h->pos_bytes, (size_t)m * sizeof(int));
-        PD_TRY(h->tmp2.ensure(need));
-        char* pos_img = (char*)h->pos + (size_t)n * h->pos_bytes;
-        PD_TRY(gather_bytes(pos_img, h->tmp2.p, ids, m, h->pos_bytes, st));
-        PD_CUDA(cudaMemcpyAsync(pos_img, h->tmp2.p, (size_t)m * h->pos_bytes, cudaMemcpyDeviceToDevice, st));
-        PD_TRY(gather_bytes(h->gid + n, h->tmp2.p, ids, m, 4, st));
-        PD_CUDA(cudaMemcpyAsync(h->gid + n, h->tmp2.p, sizeof(int) * m, cudaMemcpyDeviceToDevice, st));
-        PD_TRY(gather_bytes(h->img_src.p, h->tmp2.p, ids, m, 4, st));
-        PD_CUDA(cudaMemcpyAsync(h->img_src.p, h->tmp2.p, sizeof(int) * m, cudaMemcpyDeviceToDevice, st));
-        PD_TRY(gather_bytes(h->img_shift.p, h->tmp2.p, ids, m, 1, st));
-        PD_CUDA(cudaMemcpyAsync(h->img_shift.p, h->tmp2.p, (size_t)m, cudaMemcpyDeviceToDevice, st));
-    }
+    const MoveCol cols[4] = {{(char*)h->pos + (size_t)n * h->pos_bytes, (int)h->pos_bytes},
+                             {h->gid + n, 4},
+                             {h->img_src.p, 4},
+                             {h->img_shift.p, 1}};
+    PD_TRY(permute_columns(h, cols, 4, cl->sorted.as<int>(), m, false, st));
+    const unsigned int *csR = md->csR.as<unsigned int>(), *csI = md->csI.as<unsigned int>();
     int tx_req = md->tile_tx;
     if (tx_req == 0 && md->physics == 0) {
         // LJ: the widest tile with at most about 184 domain particles on average, from
@@ -551,68 +549,86 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         // equally long).  Fewer particles a tile, down to 40, where 184 would leave the
         // 148 SMs with less than two tiles each: 30,000 FP64 particles, force 22 us at 6
         // cells (101 a tile), 29 us at 12.
-        double inner = 1;
-        for (int d = 0; d < 3; ++d) inner *= std::max(1.0, (h->hi[d] - h->lo[d]) / cl->spacing[d]);
-        const double occ = std::max((double)n / inner, 1e-3);
-        const double want = std::min(184.0, std::max(40.0, (double)n / (2 * 148)));
-        tx_req = std::max(1, std::min(TXMAX, (int)(want / occ)));
+        tx_req = md_auto_width(h, cl, n, std::min(184.0, std::max(40.0, (double)n / (2 * 148))));
     }
     const bool narrow = md->tile_tx == 0 && md->physics == 0 && h->dtype == PD_F64;
     const int tx_auto = tx_req;
     if (narrow && md->fit_req == tx_auto) tx_req = md->fit_tx;  // as the build before found it
-    PD_TRY(tile_plan(cl, n, tx_req, md->tg, md->ntiles));
-    unsigned int tmax = 0, cmax = 0;
-    for (;;) {
-        PD_TRY(tile_sizes(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), tmax, cmax,
-                          st));
-        if (md->physics == 1 ? sph_tile_fits(h, tmax) : tile_fits(h, tmax)) break;
-        // the densest tile does not fit: narrower tiles (the width is a performance choice only)
-        if (md->tg.TX <= 1) return PD_OK;  // stays on global rows
-        PD_TRY(tile_plan(cl, n, md->tg.TX / 2, md->tg, md->ntiles));
-    }
-    if (narrow) {
-        // An uneven system: every tile's CTA takes the shared memory of the densest one, so
-        // a width from the mean occupancy costs residency.  Narrower tiles until the
-        // densest leaves the CTAs that the registers allow (four of the FP64 kernel's with
-        // 24-byte records; of the precision form's with 16 one more than its five, which
-        // measured best), but not below half
-        // the width: tiles of few particles cost more than residency.  The next build
-        // starts from the width found.  1,000,003 particles in clusters, mean width 32:
-        // precision form 494 us at 32 cells, 371 at 18, 408 at 11; FP64 315, 291, 377.
-        const long target = md->mixed ? (227 * 1024 / 6 - 4608) / 16 : (227 * 1024 / 4 - 4608) / 24;
+    // what the densest tile's staging should stay within, for the automatic widths:
+    //  - LJ, FP64 vectors: every tile's CTA takes the shared memory of the densest one, so
+    //    on an uneven system a width from the mean occupancy costs residency.  The CTAs
+    //    that the registers allow: four of the FP64 kernel's with 24-byte records, five of
+    //    the precision form's with 16 and 9 KB of lists; but not below half the width
+    //    (tiles of few particles cost more than residency).  1,000,003 particles in
+    //    clusters, mean width 32: precision form 494 us at 32 cells, 371 at 18, 408 at 11;
+    //    FP64 315, 291, 377.
+    //  - SPH: about 1730 staged particles (two records each; five cells of a filled tank):
+    //    fewer, wider tiles stage less per particle, which counts for more than residency.
+    //    FP64, dp = 1/128: rates 608 us at two cells (three CTAs per SM), 576 at five
+    //    (two); FP32, dp = 1/180: 733 us at four cells, 659 at five, 754 at six.  The mean
+    //    occupancy counts the empty part of the tank.
+    const long target = md->physics == 1 ? 1730 : (md->mixed ? (227 * 1024 / 5 - 10752) / 16 : (227 * 1024 / 4 - 4608) / 24);
+    const bool sph_auto = md->tile_tx == 0 && md->physics == 1;
+    // the width for a densest tile of `t` records at the current one
+    auto fit = [&](long t) {
         int tx = md->tg.TX;
-        if ((long)tmax > target) tx = std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)tmax) - 2);
-        else if (tx < tx_auto && (long)tmax * 5 < target * 4) tx = tx_auto;  // the densest part thinned out
-        md->fit_req = tx_auto;
-        if (tx != md->tg.TX && tx >= 1 && tx <= tx_auto) {
+        if (narrow && t > target)
+            tx = std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)t) - 2);
+        else if (narrow && tx < tx_auto && t * 5 < target * 4)
+            tx = tx_auto;  // the densest part thinned out
+        else if (sph_auto && tx > 1 && t > target)
+            tx = std::min(tx, std::max(1, (int)((double)(tx + 2) * (double)target / (double)t) - 2));
+        return narrow ? std::min(tx, tx_auto) : tx;
+    };
+    auto fits = [&](unsigned int t) { return md->physics == 1 ? sph_tile_fits(h, t) : tile_fits(h, t); };
+    const TileGeom before = md->tg;
+    const bool again = md->tiles_sized;
+    md->tiles_sized = false;
+    PD_TRY(tile_plan(cl, n, tx_req, md->tg, md->ntiles));
+    bool small = false;
+    if (again && (narrow || md->tile_tx != 0) && memcmp(&before, &md->tg, sizeof(TileGeom)) == 0) {
+        // The plan of the build before: its sizes with a margin, the real ones read with the
+        // build's own read-back (one synchronisation less, about 15 us of a small system's
+        // rebuild).  A tile that grew beyond the margin sends the build back.
+        PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, false, st));
+        const unsigned int most = 200u * 1024u / (unsigned int)sizeof(float4);  // staged FP32 records at most
+        const unsigned int cap = std::min(most, md->tcap + md->tcap / 8 + 32);
+        const unsigned int pcap = std::min(most, md->tpcap + md->tpcap / 8 + 32);
+        const int rc = tile_build(h, md->tg, md->ntiles, csR, csI, cap, pcap, md->vl->r_cut, md->pos32, md->tnbr,
+                                  md->tnn, md->tstride, md->tmax_nn, &small, st);
+        if (rc != PD_OK && !small) return rc;
+        if (rc == PD_OK && !fits(h->ctrl_h->tile_max)) small = true;
+    } else {
+        small = true;
+    }
+    if (small) {
+        for (;;) {
+            PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, true, st));
+            if (fits(h->ctrl_h->tile_max)) break;
+            // the densest tile does not fit: narrower tiles (the width is a performance choice only)
+            if (md->tg.TX <= 1) return PD_OK;  // stays on global rows
+            PD_TRY(tile_plan(cl, n, md->tg.TX / 2, md->tg, md->ntiles));
+        }
+        const int tx = fit(h->ctrl_h->tile_max);
+        if (tx != md->tg.TX && tx >= 1) {
             PD_TRY(tile_plan(cl, n, tx, md->tg, md->ntiles));
-            PD_TRY(tile_sizes(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), tmax, cmax,
-                              st));
+            PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, true, st));
         }
-        md->fit_tx = md->tg.TX;
-    }
-    if (md->tile_tx == 0 && md->physics == 1 && md->tg.TX > 1) {
-        // automatic width for SPH: the densest tile within about 1730 staged particles (two
-        // records each; five cells of a filled tank): fewer, wider tiles stage less per
-        // particle, which counts for more than residency.  FP64, dp = 1/128: rates 608 us
-        // at two cells (three CTAs per SM), 576 at five (two); FP32, dp = 1/180: 733 us at
-        // four cells, 659 at five, 754 at six.  The mean occupancy counts the empty part
-        // of the tank, so the width is rescaled from the measured largest tile
-        const long target = 1730;
-        if ((long)tmax > target) {
-            int tx = (int)((double)(md->tg.TX + 2) * (double)target / (double)tmax) - 2;
-            if (tx < 1) tx = 1;
-            if (tx < md->tg.TX) {
-                PD_TRY(tile_plan(cl, n, tx, md->tg, md->ntiles));
-                PD_TRY(tile_sizes(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), tmax,
-                                  cmax, st));
-            }
+        if (narrow) {
+            md->fit_req = tx_auto;
+            md->fit_tx = md->tg.TX;
         }
+        PD_TRY(tile_build(h, md->tg, md->ntiles, csR, csI, h->ctrl_h->tile_max, h->ctrl_h->tile_pass_max,
+                          md->vl->r_cut, md->pos32, md->tnbr, md->tnn, md->tstride, md->tmax_nn, &small, st));
+    } else if (narrow) {
+        md->fit_req = tx_auto;
+        md->fit_tx = fit(h->ctrl_h->tile_max);  // for the next build's plan
     }
-    md->tcap = tmax;
-    PD_TRY(tile_build(h, md->tg, md->ntiles, md->csR.as<unsigned int>(), md->csI.as<unsigned int>(), md->tcap,
-                      md->vl->r_cut, md->pos32, md->tnbr, md->tnn, md->tstride, md->tmax_nn, st));
-    PD_TRY(md->tpart.ensure(sizeof(double) * 3 * (size_t)(md->ntiles > 0 ? md->ntiles : 1) * (md_split_possible(md) ? STEPS_AHEAD : 1)));
+    md->tcap = h->ctrl_h->tile_max;
+    md->tpcap = h->ctrl_h->tile_pass_max;
+    md->tiles_sized = true;
+    PD_TRY(md->tpart.ensure(sizeof(double) * 3 * (size_t)(md->ntiles > 0 ? md->ntiles : 1) *
+                            (md_split_possible(md) ? STEPS_AHEAD : 1)));
     md->tiles_active = true;
     return PD_OK;
 }

@@ -27,7 +27,8 @@ struct pd_md_s {
     bool tiles_active = false;
     pd::TileGeom tg;
     long ntiles = 0;
-    unsigned int tcap = 0;
+    unsigned int tcap = 0, tpcap = 0;  // records of the last build's largest neighbourhood and layer
+    bool tiles_sized = false;          // ... of the plan in tg
     long tstride = 0;
     int tmax_nn = 0;
     pd::Buf csR, csI, tnbr, tnn, tpart, pos32;
@@ -70,6 +71,8 @@ struct pd_md_s {
 namespace pd {
 static constexpr int STEPS_AHEAD = 8;  // steps of a batch at most (pd_md_run)
 int force_blocks(long n);
+// cells per tile for `want` domain particles a tile at the mean occupancy of the cells inside the box
+int md_auto_width(pd_vd h, pd_cl cl, long n, double want);
 // wrap, sort, periodic images, neighbour structure (and the mixed-form offsets)
 int md_rebuild(pd_md md, cudaStream_t st);
 // forces of the current state into the force property (with `drift`, the plain FP64

@@ -500,14 +500,12 @@ int tile_plan(pd_cl cl, long n_real, int TX_req, TileGeom& tg, long& ntiles) {
 }
 
 int tile_sizes(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
-               unsigned int& tmax, unsigned int& cmax, cudaStream_t st) {
+               bool read, cudaStream_t st) {
     PD_CUDA(cudaMemsetAsync(&h->ctrl->tile_max, 0, 3 * sizeof(unsigned int), st));
     pd::launch(k_tile_sizes, grid_for(ntiles, 256), 256, 0, st, tg, ntiles, csR, csI, &h->ctrl->tile_max,
                &h->ctrl->tile_center_max, &h->ctrl->tile_pass_max);
     PD_LAUNCH_CHECK();
-    PD_TRY(read_ctrl(h, st));
-    tmax = h->ctrl_h->tile_max;
-    cmax = h->ctrl_h->tile_center_max;
+    if (read) PD_TRY(read_ctrl(h, st));
     return PD_OK;
 }
 
@@ -537,8 +535,9 @@ double fp32_band_at(double X, double r) {
 }
 
 int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
-               unsigned int cap, double r_list, Buf& pos32, Buf& nbr, Buf& nn, long& stride, int& max_nn,
-               cudaStream_t st) {
+               unsigned int cap, unsigned int pcap, double r_list, Buf& pos32, Buf& nbr, Buf& nn, long& stride,
+               int& max_nn, bool* small, cudaStream_t st) {
+    *small = false;
     long n = h->n_real;
     stride = ((n + 31) / 32) * 32;
     if (stride < 32) stride = 32;
@@ -562,10 +561,8 @@ int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR
     }
     max_nn = (max_nn + 1) & ~1;  // whole 32-bit words
     // three z-layer passes with a third of the staging (more resident CTAs) when
-    // the largest layer is well below the whole tile (the sizes of the tile_sizes
-    // call before); a tile of more than two domain particles a thread takes the
-    // passes again for the rest
-    const unsigned int pcap = h->ctrl_h->tile_pass_max;
+    // the largest layer is well below the whole tile; a tile of more than two domain
+    // particles a thread takes the passes again for the rest
     const bool layers = pcap > 0 && 2 * pcap < cap;
     for (int attempt = 0; attempt < 3; ++attempt) {
         int smem = (int)((layers ? pcap : cap) * sizeof(float4));
@@ -598,6 +595,15 @@ int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR
         }
         PD_LAUNCH_CHECK();
         PD_TRY(read_ctrl(h, st));
+        if ((h->ctrl_h->err & (ERR_TILE_CAP | ERR_TIMEOUT)) == ERR_TILE_CAP &&
+            (layers ? h->ctrl_h->tile_pass_max > pcap : h->ctrl_h->tile_max > cap)) {
+            // the sizes were an estimate; the control block holds the real ones now
+            h->ctrl_h->err &= ~(ERR_TILE_CAP | ERR_NN_OVERFLOW);
+            h->ctrl_h->nn_max = 0;
+            PD_CUDA(cudaMemcpyAsync(&h->ctrl->err, &h->ctrl_h->err, sizeof(unsigned int) * 2, cudaMemcpyHostToDevice, st));
+            *small = true;
+            return PD_ESTATE;
+        }
         if (h->ctrl_h->err & (ERR_TILE_CAP | ERR_TIMEOUT)) {
             set_error("tiled Verlet build failed (err=0x%x)", h->ctrl_h->err);
             return PD_EOVERFLOW;

@@ -30,16 +30,20 @@ __device__ __forceinline__ bool step_skipped(const StepGuard& g) {
 #endif
 
 int tile_plan(pd_cl cl, long n_real, int TX_req, TileGeom& tg, long& ntiles);
+// the largest staged neighbourhood, centre count and staged layer of the tiles into the
+// control block, and with `read` on to the host (one synchronisation)
 int tile_sizes(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
-               unsigned int& tmax, unsigned int& cmax, cudaStream_t st);
+               bool read, cudaStream_t st);
 bool tile_fits(pd_vd h, unsigned int tmax);  // FP64/FP32 staging of the pair kernel fits
 // bound on |d2_f32 - d2| for pairs near r in the vector's box (FP32 prefilter band of the build)
 double fp32_band(pd_vd h, double r);
 // the same for coordinates of magnitude up to X
 double fp32_band_at(double X, double r);
+// Rows of the tiles; `cap` and `pcap`: records of the largest neighbourhood and layer.
+// PD_ESTATE with *small set (and nothing else wrong) when a layer was larger than pcap.
 int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR, const unsigned int* csI,
-               unsigned int cap, double r_list, Buf& pos32, Buf& nbr, Buf& nn, long& stride, int& max_nn,
-               cudaStream_t st);
+               unsigned int cap, unsigned int pcap, double r_list, Buf& pos32, Buf& nbr, Buf& nn, long& stride,
+               int& max_nn, bool* small, cudaStream_t st);
 // The FP64 pair kernel stages (x, y) and z from copies of the positions: those of
 // the slots [first, first + n) refreshed from the records (room for the vector's capacity)
 int tile_split(pd_vd h, Buf& sxy, Buf& sz, long first, long n, cudaStream_t st);
