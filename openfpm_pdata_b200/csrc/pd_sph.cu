@@ -213,6 +213,58 @@ struct TileShS {
     unsigned long long bar;
 };
 
+// One round of a pair kernel's CTA over its tile's particles [first, ie): P lanes per row
+// while a round is full, more lanes per row (up to a warp) in the last, partial round.
+// Every thread takes part in every round (the shuffles need whole warps).
+struct TileRound {
+    unsigned int q, cnt, i;  // lanes a row, particles of the round, this thread's particle
+    int sub;                 // this thread's lane of its row
+    bool active;
+};
+template <int P, int BLOCK>
+__device__ __forceinline__ TileRound tile_round(unsigned int first, unsigned int ie) {
+    TileRound R;
+    const unsigned int left = ie - first;
+    R.q = P;
+    while (R.q < 32u && left * (R.q << 1) <= (unsigned int)BLOCK) R.q <<= 1;
+    R.cnt = min(left, (unsigned int)BLOCK / R.q);
+    R.sub = (int)(threadIdx.x % R.q);
+    R.active = threadIdx.x / R.q < R.cnt;
+    R.i = first + (R.active ? threadIdx.x / R.q : 0u);
+    return R;
+}
+
+// A row's words are read four iterations ahead of the pair loop (a register shift ring).
+// The first four are read together with the row length (within the buffer's mwords words
+// per particle), and before the round begins: the first round's while the tile's records
+// are still being staged, a later round's before the sums of the round before it (FP64,
+// 2,097,152 particles: rates 582 -> 561 us a step, FP32, 5,832,000: 665 -> 652; the FP64
+// LJ and precision-form pair kernels at 64 and 48 registers spill with it: 929 -> 1,174
+// and 244 -> 257 us).
+struct RowAhead {
+    unsigned int q0, q1, q2, q3;
+    int words;
+    __device__ __forceinline__ void open(const TileRound& R, const unsigned int* __restrict__ nbr,
+                                         const int* __restrict__ nn, long stride, int mwords) {
+        const unsigned int* row = nbr + R.i;
+        const int sub = R.sub, Q = (int)R.q;
+        q0 = sub < mwords ? __ldg(row + (long)sub * stride) : 0u;
+        q1 = sub + Q < mwords ? __ldg(row + (long)(sub + Q) * stride) : 0u;
+        q2 = sub + 2 * Q < mwords ? __ldg(row + (long)(sub + 2 * Q) * stride) : 0u;
+        q3 = sub + 3 * Q < mwords ? __ldg(row + (long)(sub + 3 * Q) * stride) : 0u;
+        words = R.active ? (__ldg(nn + R.i) + 1) >> 1 : 0;
+    }
+    // the word of iteration k, and the one four iterations on in its place
+    __device__ __forceinline__ unsigned int take(int k, int Q, const unsigned int* __restrict__ row, long stride) {
+        const unsigned int pair = q0;
+        q0 = q1;
+        q1 = q2;
+        q2 = q3;
+        q3 = k + 4 * Q < words ? __ldg(row + (long)(k + 4 * Q) * stride) : 0u;
+        return pair;
+    }
+};
+
 // rates of every particle of a tile; no periodic images in this configuration
 template <class T, int P>
 __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::type* __restrict__ pos,
@@ -245,14 +297,19 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
             S.cR[r][j] = csR[c];
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int o = 0;
-            for (int r = 0; r < 9; ++r) {
-                S.oR[r] = o;
-                o += S.cR[r][ncol - 1] - S.cR[r][0];
+        // staging offsets of the nine rows: a scan of their lengths across the first warp
+        if (threadIdx.x < 32) {
+            const int r = (int)threadIdx.x;
+            const unsigned int len = r < 9 ? S.cR[r][ncol - 1] - S.cR[r][0] : 0u;
+            unsigned int inc = len;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1) {
+                const unsigned int v = __shfl_up_sync(0xffffffffu, inc, o);
+                if (r >= o) inc += v;
             }
-            S.total = o;
-            S.ncol = ncol;
+            if (r < 9) S.oR[r] = inc - len;
+            if (r == 8) S.total = inc;
+            if (r == 0) S.ncol = ncol;
         }
         __syncthreads();
     }
@@ -279,6 +336,10 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
             }
         }
     }
+    TileRound R = tile_round<P, FBLOCK_T>(ib, ie);
+    RowAhead A;
+    A.open(R, nbr, nn, stride, mwords);
+    int ty = __ldg(type + R.i);
     bool waited = mbar_wait_bounded(&S.bar, 0, 1u << 24);
     if (!waited) {
         atomicOr(err, ERR_TIMEOUT);
@@ -287,38 +348,18 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
     if (!__syncthreads_and(waited ? 1 : 0)) return;
 
     const unsigned int base = S.oR[4] - S.cR[4][0];
-    // rounds of the whole CTA over the tile's particles: P lanes per row while a
-    // round is full, more lanes per row (up to a warp) in the last, partial round;
-    // every thread takes part in every round (the shuffles need whole warps)
     unsigned int first = ib;
-    while (first < ie) {
-        const unsigned int left = ie - first;
-        unsigned int q = P;
-        while (q < 32u && left * (q << 1) <= (unsigned int)FBLOCK_T) q <<= 1;
-        const unsigned int cnt = min(left, (unsigned int)FBLOCK_T / q);
-        const int sub = (int)(threadIdx.x % q);
-        const int Q = (int)q;
-        const bool active = threadIdx.x / q < cnt;
-        const unsigned int i = first + (active ? threadIdx.x / q : 0u);
+    for (;;) {
+        const unsigned int i = R.i;
         const unsigned int li = base + i;
         const T4 xi = sp[li];
         const T4 ai = sa[li];
         const T pa_r = xi.w;
         const unsigned int* row = nbr + i;
-        // row words read four iterations ahead (register shift ring); the first four
-        // together with the row length (within the buffer's mwords words per particle)
-        unsigned int q0 = sub < mwords ? __ldg(row + (long)sub * stride) : 0u;
-        unsigned int q1 = sub + Q < mwords ? __ldg(row + (long)(sub + Q) * stride) : 0u;
-        unsigned int q2 = sub + 2 * Q < mwords ? __ldg(row + (long)(sub + 2 * Q) * stride) : 0u;
-        unsigned int q3 = sub + 3 * Q < mwords ? __ldg(row + (long)(sub + 3 * Q) * stride) : 0u;
-        const int words = active ? (nn[i] + 1) >> 1 : 0;
+        const int Q = (int)R.q;
         T ax = 0, ay = 0, az = 0, dr = 0;
-        for (int k = sub; k < words; k += Q) {
-            const unsigned int pair = q0;
-            q0 = q1;
-            q1 = q2;
-            q2 = q3;
-            q3 = k + 4 * Q < words ? __ldg(row + (long)(k + 4 * Q) * stride) : 0u;
+        for (int k = R.sub; k < A.words; k += Q) {
+            const unsigned int pair = A.take(k, Q, row, stride);
 #pragma unroll
             for (int hh = 0; hh < 2; ++hh) {
                 const unsigned int l = hh ? (pair >> 16) : (pair & 0xffffu);
@@ -360,20 +401,29 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
                 }
             }
         }
-        for (unsigned int o = 1; o < q; o <<= 1) {
+        const bool fluid = ty == 0;
+        const unsigned int next = first + R.cnt;
+        TileRound N = R;
+        if (next < ie) {
+            N = tile_round<P, FBLOCK_T>(next, ie);
+            A.open(N, nbr, nn, stride, mwords);
+            ty = __ldg(type + N.i);
+        }
+        for (unsigned int o = 1; o < R.q; o <<= 1) {
             ax += __shfl_xor_sync(0xffffffffu, ax, o);
             ay += __shfl_xor_sync(0xffffffffu, ay, o);
             az += __shfl_xor_sync(0xffffffffu, az, o);
             dr += __shfl_xor_sync(0xffffffffu, dr, o);
         }
-        if (active && sub == 0) {
-            const bool fluid = type[i] == 0;
+        if (R.active && R.sub == 0) {
             acc[i] = fluid ? ax : T(0);
             acc[cap_p + i] = fluid ? ay : T(0);
             acc[2 * cap_p + i] = fluid ? az + K.gz : T(0);
             drho[i] = dr;
         }
-        first += cnt;
+        if (next >= ie) break;
+        first = next;
+        R = N;
     }
 }
 
