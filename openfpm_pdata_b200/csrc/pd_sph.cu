@@ -237,8 +237,8 @@ __device__ __forceinline__ TileRound tile_round(unsigned int first, unsigned int
 // A row's words are read four iterations ahead of the pair loop (a register shift ring).
 // The first four are read together with the row length (within the buffer's mwords words
 // per particle), and before the round begins: the first round's while the tile's records
-// are still being staged, a later round's before the sums of the round before it (FP64,
-// 2,097,152 particles: rates 582 -> 561 us a step, FP32, 5,832,000: 665 -> 652; the FP64
+// are still being staged, a later round's before the sums of the round before it (dam break,
+// FP64, dp = 1/128: rates 582 -> 561 us a step, FP32, dp = 1/180: 665 -> 652; the FP64
 // LJ and precision-form pair kernels at 64 and 48 registers spill with it: 929 -> 1,174
 // and 244 -> 257 us).
 struct RowAhead {

@@ -95,9 +95,14 @@ __global__ void __launch_bounds__(TBLOCK) k_vtile_build(const typename V4<T>::ty
 }
 
 // List build in three passes of one z-layer each (tile_rows_layers in
-// pd_tile_dev.cuh): a third of the full staging, more resident CTAs.
+// pd_tile_dev.cuh): a third of the full staging, more resident CTAs.  Bound by the
+// instructions of the candidate tests (about 460 a particle) and of the entries written
+// out: with the tests in packed FP32 pairs and two masks a stream instead of three, 1,760 ->
+// 1,621 us for 4,096,000 FP64 particles (69 entries a row), 369 -> 338 us for 1,000,000 in
+// droplets.  FP64 at eight CTAs per SM (64 registers; at nine 1,627, and 150 against 141 us
+// for 250,000 particles), FP32 at nine (eight: 1,267 against 1,229 us, 1,898,748 particles).
 template <class T>
-__global__ void __launch_bounds__(TBLOCK, 9) k_vtile_build3(const typename V4<T>::type* __restrict__ pos,
+__global__ void __launch_bounds__(TBLOCK, sizeof(T) == 8 ? 8 : 9) k_vtile_build3(const typename V4<T>::type* __restrict__ pos,
                                                          const float4* __restrict__ pos32, long n_real,
                                                          TileGeom tg, const unsigned int* __restrict__ csR,
                                                          const unsigned int* __restrict__ csI, unsigned int pcap,

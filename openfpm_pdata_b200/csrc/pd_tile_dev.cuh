@@ -148,6 +148,31 @@ __device__ __forceinline__ void tile_segb(const TileSh& S, unsigned int (*segb)[
     }
 }
 
+// t = |x - q|^2 - lo for a staged candidate: the x and y components in one packed
+// instruction each (two FP32 operations an issue slot), -lo riding on the squares.  Near
+// the threshold its rounding is at most 3 u r^2 (the square less lo, the other square, their
+// sum; the last sum is small), within the 4 u r^2 the band allows for.
+__device__ __forceinline__ unsigned long long pack_f32x2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b,
+                                                        unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float d2_less(unsigned long long n_xy, float z, const float4& q, unsigned long long m_lo) {
+    unsigned long long d;  // q - x, rounded once
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pack_f32x2(q.x, q.y)), "l"(n_xy));
+    const unsigned long long s = fma_f32x2(d, d, m_lo);
+    float sx, sy;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(sx), "=f"(sy) : "l"(s));
+    const float dz = z - q.z;
+    return fmaf(dz, dz, sx + sy);
+}
+
 // Accept mask of one chunk of n <= 32 staged candidates (c4[0..n)) for the
 // particle at x: the sign of t = d2 - lo_thr (surely in) shifted in, the first
 // candidate ending in the highest bit: bit n-1-k stands for c4[k] (fl(a - b) < 0
@@ -162,20 +187,19 @@ __device__ __forceinline__ unsigned int chunk_mask(const float4* __restrict__ c4
                                                    unsigned int i, const typename V4<T>::type* __restrict__ pos,
                                                    T r2, float lo_thr, float hi_thr) {
     unsigned int m = 0, umin = 0xffffffffu;
+    const unsigned long long n_xy = pack_f32x2(-x.x, -x.y), m_lo = pack_f32x2(-lo_thr, 0.f);
 #pragma unroll 4
     for (unsigned int k = 0; k < n; ++k) {
-        const float4 xq = c4[k];
-        const float d2 = dist2(x.x - xq.x, x.y - xq.y, x.z - xq.z);
-        const unsigned int t = __float_as_uint(d2 - lo_thr);
+        const unsigned int t = __float_as_uint(d2_less(n_xy, x.z, c4[k], m_lo));
         m = __funnelshift_l(t, m, 1);
         umin = min(umin, t);
     }
-    if (umin <= __float_as_uint(hi_thr - lo_thr)) {
+    const unsigned int band = __float_as_uint(hi_thr - lo_thr);
+    if (umin <= band) {
         for (unsigned int k = 0; k < n; ++k) {
             const float4 xq = c4[k];
-            const float d2 = dist2(x.x - xq.x, x.y - xq.y, x.z - xq.z);
-            if (!(d2 < lo_thr) && d2 < hi_thr && exact_in<T>(pos, i, __float_as_int(xq.w), r2))
-                m |= 1u << (n - 1 - k);
+            const unsigned int t = __float_as_uint(d2_less(n_xy, x.z, xq, m_lo));
+            if (t <= band && exact_in<T>(pos, i, __float_as_int(xq.w), r2)) m |= 1u << (n - 1 - k);
         }
     }
     return m;
@@ -183,7 +207,7 @@ __device__ __forceinline__ unsigned int chunk_mask(const float4* __restrict__ c4
 
 // Row entries of particle i (global index; FP32 copy x) from the staged candidates
 // [qb, qe), staging indices, candidate q at sm[q - base], appended in ascending q
-// (the entries of the candidate-by-candidate walk, in its order).  Up to three
+// (the entries of the candidate-by-candidate walk, in its order).  Two
 // chunks of 32 are tested into masks first; their accepted candidates then leave
 // as one stream, two entries (one 32-bit word) at a time, so a lane's loop runs
 // about half its accept count rather than the sum of the chunks' largest counts
@@ -196,27 +220,24 @@ __device__ __forceinline__ void seg_rows(const float4* __restrict__ sm, unsigned
                                          float hi_thr, unsigned int* __restrict__ out, long stride, int max_nn,
                                          int& c, unsigned int& pend) {
 #pragma unroll 1
-    for (unsigned int q0 = qb; q0 < qe; q0 += 96) {
-        const unsigned int n = min(96u, qe - q0);
-        const unsigned int na = min(32u, n), nb = min(32u, n - na), nc = n - na - nb;
+    for (unsigned int q0 = qb; q0 < qe; q0 += 64) {
+        const unsigned int n = min(64u, qe - q0);
+        const unsigned int na = min(32u, n), nb = n - na;
         const float4* c4 = sm + (q0 - base);
         unsigned int ma = chunk_mask<T>(c4, na, x, i, pos, r2, lo_thr, hi_thr);
         unsigned int mb = chunk_mask<T>(c4 + 32, nb, x, i, pos, r2, lo_thr, hi_thr);
-        unsigned int mc = chunk_mask<T>(c4 + 64, nc, x, i, pos, r2, lo_thr, hi_thr);
-        // candidate of bit b of a mask: qt - 31 + clz position, qt = last q of the chunk
-        unsigned int qa = q0 + na - 32, qb_ = q0 + 32 + nb - 32, qc = q0 + 64 + nc - 32;
-        int rem = __popc(ma) + __popc(mb) + __popc(mc);
+        int rem = __popc(ma) + __popc(mb);
         if (rem == 0) continue;
-        // the stream: ma first; an emptied mask takes the next one's place
-        if (ma == 0) { ma = mb; qa = qb_; mb = mc; qb_ = qc; mc = 0; }
-        if (ma == 0) { ma = mb; qa = qb_; mb = 0; }
-        if (mb == 0) { mb = mc; qb_ = qc; mc = 0; }
+        // the highest bit of each mask for its chunk's first candidate
+        ma <<= 32 - na;
+        mb = __funnelshift_lc(0u, mb, 32 - nb);
+        // the stream: ma first; mb takes an emptied ma's place (an entry is left in one of them)
+        unsigned int qa = q0;
         auto next = [&]() -> unsigned int {
+            if (ma == 0) { ma = mb; qa += 32; }
             const int z = __clz(ma);
-            const unsigned int q = qa + (unsigned int)z;
             ma ^= 0x80000000u >> z;
-            if (ma == 0) { ma = mb; qa = qb_; mb = mc; qb_ = qc; mc = 0; }
-            return q;
+            return qa + (unsigned int)z;
         };
         if (c & 1) {  // complete the pending word
             const unsigned int q = next();

@@ -104,7 +104,7 @@ __device__ __forceinline__ bool sym_keep(const typename V4<T>::type* __restrict_
 }
 
 // Entries of particle i from the n candidates c4[0..n) appended to its row in
-// candidate order: accept masks of up to three chunks of 32 first, then one stream
+// candidate order: accept masks of two chunks of 32 first, then one stream
 // of the accepted ones (see seg_rows).  Works on staged and on global records.
 template <class T, bool SYM>
 __device__ __forceinline__ void verlet_seg(const float4* __restrict__ c4, unsigned int n, const float4 x, int i,
@@ -112,17 +112,17 @@ __device__ __forceinline__ void verlet_seg(const float4* __restrict__ c4, unsign
                                            float hi_thr, long n_dom, int* __restrict__ out, long stride, int max_nn,
                                            int& c) {
 #pragma unroll 1
-    for (unsigned int q0 = 0; q0 < n; q0 += 96) {
-        const unsigned int m = min(96u, n - q0);
-        const unsigned int na = min(32u, m), nb = min(32u, m - na), nc = m - na - nb;
+    for (unsigned int q0 = 0; q0 < n; q0 += 64) {
+        const unsigned int m = min(64u, n - q0);
+        const unsigned int na = min(32u, m), nb = m - na;
         unsigned int ma = chunk_mask<T>(c4 + q0, na, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
         unsigned int mb = chunk_mask<T>(c4 + q0 + 32, nb, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
-        unsigned int mc = chunk_mask<T>(c4 + q0 + 64, nc, x, (unsigned int)i, pos, r2, lo_thr, hi_thr);
-        // candidate of the highest bit of a mask: q + clz (modulo 2^32)
-        unsigned int qa = q0 + na - 32, qb = q0 + 32 + nb - 32, qc = q0 + 64 + nc - 32;
-        for (int rem = __popc(ma) + __popc(mb) + __popc(mc); rem > 0; --rem) {
-            if (ma == 0) { ma = mb; qa = qb; mb = mc; qb = qc; mc = 0; }
-            if (ma == 0) { ma = mb; qa = qb; mb = 0; }
+        int rem = __popc(ma) + __popc(mb);
+        // the highest bit of each mask for its chunk's first candidate
+        ma <<= 32 - na;
+        mb = __funnelshift_lc(0u, mb, 32 - nb);
+        for (unsigned int qa = q0; rem > 0; --rem) {
+            if (ma == 0) { ma = mb; qa += 32; }
             const int z = __clz(ma);
             ma ^= 0x80000000u >> z;
             const int q = __float_as_int(c4[qa + (unsigned int)z].w);
@@ -156,8 +156,8 @@ __device__ __noinline__ void verlet_seg_wide(const float4* __restrict__ c4, unsi
 // at once where it fits `pcap` records (eight CTAs per SM), so that a CTA's warps wait for
 // each other once; else one z-layer of three cell rows at a time; a layer beyond `pcap`
 // records is read from global memory instead.
-// Measured: 1,000,000 FP64 particles of a lattice (49 entries a row) 1198 -> 520 us, half
-// rows of 200,001 348 -> 165 us against FP64 records of all nine rows staged at once.
+// Measured: 1,000,000 FP64 particles of a lattice (49 entries a row) 1198 -> 421 us, half
+// rows of 200,001 348 -> 144 us against FP64 records of all nine rows staged at once.
 template <class T, bool SYM>
 __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>::type* __restrict__ pos,
                                                         const float4* __restrict__ p32, TileGeom tg,
@@ -278,10 +278,10 @@ static int verlet_rows(pd_vd h, pd_vl vl, const float4* p32, const TileGeom& tg,
     const unsigned int pcap = 1536;
     const T rc = (T)vl->r_cut;
     const T r2 = rc * rc;
-    // FP32 positions are staged as they are: their band is empty
-    const double band = sizeof(T) == 8 ? fp32_band_at(verlet_bound(cl), vl->r_cut) : 0.0;
-    const float lo_thr = sizeof(T) == 8 ? (float)((double)r2 - band) : (float)r2;
-    const float hi_thr = sizeof(T) == 8 ? (float)((double)r2 + band) : (float)r2;
+    // FP32 positions are staged as they are: their band covers the rounding of the sums only
+    // (the test adds in another order than the predicate), down to a few subnormal steps
+    const double band = fp32_band_at(sizeof(T) == 8 ? verlet_bound(cl) : 0.0, vl->r_cut) + std::ldexp(1.0, -146);
+    const float lo_thr = (float)((double)r2 - band), hi_thr = (float)((double)r2 + band);
     auto go = [&](auto k) {
         pd::launch(k, (unsigned)ntiles, TBLOCK, pcap * sizeof(float4), st, (const T4*)h->pos, p32, tg,
                    (const unsigned int*)cl->cell_start.as<unsigned int>(), n_dom, r2, lo_thr, hi_thr, vl->nbr.as<int>(),

@@ -72,3 +72,26 @@ def test_particle_far_outside_the_grid(pd, dtype):
         else:
             want = near[i] < r * r
             assert np.array_equal(row[sure[i]], want[sure[i]])
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+def test_pairs_at_the_cutoff(pd, orc, dtype):
+    """Pairs whose distance is r up to a few roundings: many on a jittered shell of each of
+    some centres, decided as the exact predicate decides them."""
+    rng = np.random.default_rng(23)
+    L, r, n = 12.0, 1.3, 6000
+    lo, hi, bc = np.zeros(3), np.full(3, L), np.ones(3, np.int32)
+    c = rng.uniform(2, L - 2, size=(20, 3))
+    u = rng.normal(size=(n, 3))
+    u *= (r * (1.0 + rng.integers(-4, 5, size=(n, 1)) * np.finfo(dtype).eps)) / np.linalg.norm(u, axis=1)[:, None]
+    x = orc.wrap(np.concatenate([c, c[rng.integers(0, 20, n)] + u]).astype(dtype), lo.astype(dtype),
+                 hi.astype(dtype), bc)
+    vd = pd.VectorDist(len(x), lo, hi, bc, r, dtype=dtype)
+    vd.hostToDevicePos(x)
+    vd.map()
+    vd.ghost_get()
+    g = orc.cl_geometry(lo, hi, np.full(3, r), r, dtype=dtype, verlet=True)
+    off, idx = orc.verlet(vd.deviceToHostPos(), len(x), g, r)
+    got_off, got = vd.getVerlet(r).get()
+    assert np.array_equal(got_off, off)
+    assert np.array_equal(got, idx)
