@@ -1006,7 +1006,9 @@ struct CopyPool {
     std::vector<CopyJob> pieces;
     size_t next = 0, left = 0;
     bool stop = false, tried = false;
+    std::mutex use;  // held by the call whose copy the workers share; another call copies by itself
 
+    CopyPool() { pieces.reserve(16); }  // a copy has at most 4 + 2 pieces: no allocation later
     ~CopyPool() {
         {
             std::lock_guard<std::mutex> lk(mu);
@@ -1042,7 +1044,8 @@ struct CopyPool {
     void copy(const CopyJob* jobs, int nj) {
         size_t total = 0;
         for (int j = 0; j < nj; ++j) total += jobs[j].bytes;
-        if (total < ((size_t)1 << 20)) {
+        std::unique_lock<std::mutex> mine(use, std::try_to_lock);
+        if (total < ((size_t)1 << 20) || !mine.owns_lock()) {
             for (int j = 0; j < nj; ++j) memcpy(jobs[j].dst, jobs[j].src, jobs[j].bytes);
             return;
         }
@@ -1118,7 +1121,7 @@ struct pd_srv_s {
     // pinned outbox: a finished system's positions and energies are copied here by
     // the GPU and read by pd_srv_result; regions are freed at pd_srv_release
     PinnedFifo outbox;
-    std::unique_ptr<CopyPool> copier;  // submissions' copies into the inbox
+    CopyPool copier;  // submissions' copies into the inbox, results' out of the outbox
     bool adm_pending = false;
     cudaGraphExec_t gstep[4] = {nullptr, nullptr, nullptr, nullptr};  // 1, 2, 4, 8 steps per launch
     bool dirty = true;
@@ -2032,8 +2035,7 @@ int pd_srv_submit(pd_srv s, long n, double box, const double* x_host, const doub
     if (char* p = s->inbox.take(r->ticket, half + sizeof(double) * 3 * n, r->in_lo, s->ev_free)) {
         const CopyJob jobs[2] = {{p, reinterpret_cast<const char*>(x_host), sizeof(double) * 3 * n},
                                  {p + half, reinterpret_cast<const char*>(v_host), sizeof(double) * 3 * n}};
-        if (!s->copier) s->copier.reset(new CopyPool());
-        s->copier->copy(jobs, 2);
+        s->copier.copy(jobs, 2);
     } else {
         r->x.assign(x_host, x_host + 3 * n);
         r->v.assign(v_host, v_host + 3 * n);
@@ -2168,8 +2170,7 @@ int pd_srv_result(pd_srv s, long ticket, double* x_out, double* E_out, double* t
         const size_t ox = sizeof(double) * 3 * r->n, oe = (ox + 63) & ~(size_t)63;
         if (x_out) {
             const CopyJob job{reinterpret_cast<char*>(x_out), b, ox};
-            if (!s->copier) s->copier.reset(new CopyPool());
-            s->copier->copy(&job, 1);
+            s->copier.copy(&job, 1);
         }
         if (E_out) memcpy(E_out, b + oe, sizeof(double) * 4 * r->steps);
     } else {
