@@ -205,6 +205,13 @@ __global__ void __launch_bounds__(256) k_sph_kick_kick_drift(typename V4<T>::typ
     }
 }
 
+// Threads per tile CTA of the rates.  The tile width is chosen for about 1,730 staged
+// particles: 110 KB in FP64, two CTAs per SM, which at 256 threads leave the SM with 16
+// warps; 384 threads (74 registers) make them 24.  Dam break, FP64, dp = 1/128: 561 -> 521 us
+// a step, dp = 1/70: 179 -> 147, dp = 1/40: 56 -> 47 (512 threads at 64 registers: 615, 173,
+// 58).  FP32 has four CTAs of 256 (384 threads: 652 -> 717 us at dp = 1/180).
+template <class T> static constexpr int SPH_BLOCK = sizeof(T) == 8 ? 384 : FBLOCK_T;
+
 struct TileShS {
     unsigned int cR[9][TXMAX + 3];
     unsigned int oR[9];
@@ -267,7 +274,7 @@ struct RowAhead {
 
 // rates of every particle of a tile; no periodic images in this configuration
 template <class T, int P>
-__global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::type* __restrict__ pos,
+__global__ void __launch_bounds__(SPH_BLOCK<T>) k_vtile_sph(const typename V4<T>::type* __restrict__ pos,
                                                         const typename V4<T>::type* __restrict__ aux, TileGeom tg,
                                                         const unsigned int* __restrict__ csR, unsigned int cap,
                                                         const unsigned int* __restrict__ nbr,
@@ -336,7 +343,7 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
             }
         }
     }
-    TileRound R = tile_round<P, FBLOCK_T>(ib, ie);
+    TileRound R = tile_round<P, SPH_BLOCK<T>>(ib, ie);
     RowAhead A;
     A.open(R, nbr, nn, stride, mwords);
     int ty = __ldg(type + R.i);
@@ -405,7 +412,7 @@ __global__ void __launch_bounds__(FBLOCK_T) k_vtile_sph(const typename V4<T>::ty
         const unsigned int next = first + R.cnt;
         TileRound N = R;
         if (next < ie) {
-            N = tile_round<P, FBLOCK_T>(next, ie);
+            N = tile_round<P, SPH_BLOCK<T>>(next, ie);
             A.open(N, nbr, nn, stride, mwords);
             ty = __ldg(type + N.i);
         }
@@ -537,7 +544,7 @@ static int launch_sph(pd_vd h, const TileGeom& tg, long ntiles, const unsigned i
     const Prop& A = h->props[acc_prop];
     const Prop& D = h->props[sp.drho_prop];
     const Prop& Ty = h->props[sp.type_prop];
-    pd::launch(k_vtile_sph<T, P>, (unsigned)ntiles, FBLOCK_T, (size_t)smem, st, (const T4*)h->pos,
+    pd::launch(k_vtile_sph<T, P>, (unsigned)ntiles, SPH_BLOCK<T>, (size_t)smem, st, (const T4*)h->pos,
                (const T4*)aux.as<T4>(), tg, csR, cap, (const unsigned int*)nbr.as<unsigned int>(),
                (const int*)nn.as<int>(), stride, mwords, (const int*)Ty.d, sphk<T>(sp), (T*)A.d, (T*)D.d, h->cap,
                &h->ctrl->err, guard);
