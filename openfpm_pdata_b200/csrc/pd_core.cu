@@ -549,6 +549,7 @@ int pd_create(int dim, int dtype, long n, const double* lo, const double* hi, co
 
 int pd_destroy(pd_vd h) {
     if (!h) return PD_EINVAL;
+    *h->alive = false;
     dev_free(h->pos);
     dev_free(h->gid);
     for (auto& P : h->props) dev_free(P.d);

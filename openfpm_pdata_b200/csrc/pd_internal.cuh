@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -167,6 +168,8 @@ struct pd_vd_s {
     int* spare_gid = nullptr;
     std::vector<char*> spare_props;
     long spare_cap = 0;
+    // false once the vector is destroyed; shared with its drivers, which may be destroyed later
+    std::shared_ptr<bool> alive = std::make_shared<bool>(true);
     long epoch = 0;
     // slab decomposition (pd_slab.cu): the rows of the last labelling, in send
     // order (slot of each row, shift code of each halo row), and the halo

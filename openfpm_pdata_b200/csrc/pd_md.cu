@@ -963,6 +963,7 @@ int pd_md_create(pd_vd h, const pd_lj_params_t* lj, const pd_md_params_t* mp, pd
         }
     pd_md md = new pd_md_s();
     md->h = h;
+    md->alive = h->alive;
     md->lj = *lj;
     md->mp = *mp;
     md->mixed = mp->precision == PD_PREC_MIXED;
@@ -1011,6 +1012,7 @@ int pd_sph_create(pd_vd h, const pd_sph_params_t* sp, const pd_md_params_t* mp, 
         return PD_EINVAL;
     pd_md md = new pd_md_s();
     md->h = h;
+    md->alive = h->alive;
     md->mp = *mp;
     md->sp = *sp;
     md->physics = 1;
@@ -1037,8 +1039,9 @@ int pd_sph_create(pd_vd h, const pd_sph_params_t* sp, const pd_md_params_t* mp, 
 
 int pd_md_destroy(pd_md md) {
     if (!md) return PD_EINVAL;
-    if (md->swap_reorder && md->h) {
-        // the reorder's spare storage lives with the vector; without a driver it has no use
+    if (md->swap_reorder && *md->alive) {
+        // the reorder's spare storage lives with the vector; without a driver it has no use.
+        // A vector destroyed before its driver (a garbage collector's order) took it along.
         pd_vd h = md->h;
         free_storage(h->spare_pos, h->spare_gid, h->spare_props);
         h->spare_pos = nullptr;

@@ -8,6 +8,7 @@
 
 struct pd_md_s {
     pd_vd h = nullptr;
+    std::shared_ptr<bool> alive;  // of the vector: h may be used while true
     // the rebuild's reorder swaps the vector's spare storage in (single-system driver;
     // off where device pointers are kept in tables, the serving loop)
     bool swap_reorder = true;
