@@ -569,11 +569,12 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
     //    occupancy counts the empty part of the tank.
     const long target = md->physics == 1 ? 1730 : (md->mixed ? (227 * 1024 / 5 - 10752) / 16 : (227 * 1024 / 4 - 4608) / 24);
     const bool sph_auto = md->tile_tx == 0 && md->physics == 1;
-    // the width for a densest tile of `t` records at the current one
+    // the width for a densest tile of `t` records at the current one (narrower, or the
+    // automatic one again)
     auto fit = [&](long t) {
         int tx = md->tg.TX;
         if (narrow && t > target)
-            tx = std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)t) - 2);
+            tx = std::min(tx, std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)t) - 2));
         else if (narrow && tx < tx_auto && t * 5 < target * 4)
             tx = tx_auto;  // the densest part thinned out
         else if (sph_auto && tx > 1 && t > target)
@@ -581,6 +582,17 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         return narrow ? std::min(tx, tx_auto) : tx;
     };
     auto fits = [&](unsigned int t) { return md->physics == 1 ? sph_tile_fits(h, t) : tile_fits(h, t); };
+    // the plan of width tx or, where its densest tile does not fit the staging, of half of it and so on
+    // (the width is a performance choice only); its sizes are in the control block's mirror.  *ok: one fits.
+    auto plan = [&](int tx, bool* ok) {
+        PD_TRY(tile_plan(cl, n, tx, md->tg, md->ntiles));
+        for (;;) {
+            PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, true, st));
+            *ok = fits(h->ctrl_h->tile_max);
+            if (*ok || md->tg.TX <= 1) return (int)PD_OK;
+            PD_TRY(tile_plan(cl, n, md->tg.TX / 2, md->tg, md->ntiles));
+        }
+    };
     const TileGeom before = md->tg;
     const bool again = md->tiles_sized;
     md->tiles_sized = false;
@@ -602,17 +614,13 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         small = true;
     }
     if (small) {
-        for (;;) {
-            PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, true, st));
-            if (fits(h->ctrl_h->tile_max)) break;
-            // the densest tile does not fit: narrower tiles (the width is a performance choice only)
-            if (md->tg.TX <= 1) return PD_OK;  // stays on global rows
-            PD_TRY(tile_plan(cl, n, md->tg.TX / 2, md->tg, md->ntiles));
-        }
+        bool ok = false;
+        PD_TRY(plan(md->tg.TX, &ok));
+        if (!ok) return PD_OK;  // stays on global rows
         const int tx = fit(h->ctrl_h->tile_max);
         if (tx != md->tg.TX && tx >= 1) {
-            PD_TRY(tile_plan(cl, n, tx, md->tg, md->ntiles));
-            PD_TRY(tile_sizes(h, md->tg, md->ntiles, csR, csI, true, st));
+            PD_TRY(plan(tx, &ok));
+            if (!ok) return PD_OK;
         }
         if (narrow) {
             md->fit_req = tx_auto;

@@ -1,0 +1,49 @@
+"""Automatic tile widths on a system whose densest tiles fit the staging only after the width
+was halved several times: a dense rod along x in a box of vapour, long cutoff (88 particles a
+cell in the rod, fewer than two on average, so the mean occupancy asks for the widest tile).
+The run keeps a width that fits, from one rebuild to the next, and follows the oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+F32, F64 = np.float32, np.float64
+
+
+@pytest.fixture(scope="module")
+def pd():
+    from openfpm_pdata_b200 import pd as _pd
+    _pd.lib()
+    return _pd
+
+
+def _rod():
+    sp, k = 1.08, (89, 14, 14)
+    box = np.array([89 * sp, 110.0, 110.0])
+    g = np.stack(np.meshgrid(*[np.arange(c) for c in k], indexing="ij"), -1).reshape(-1, 3)
+    rng = np.random.default_rng(11)
+    x = (g + 0.5) * sp + rng.uniform(-0.03, 0.03, size=(len(g), 3)) + [0.0, 45.0, 47.0]
+    v = rng.normal(size=x.shape) * 1.5
+    return x, v - v.mean(0), box
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_dense_rod_in_a_thin_box(pd, orc, mixed):
+    x, v, box = _rod()
+    lo, bc, rc, skin, dt, steps = np.zeros(3), np.ones(3, np.int32), 4.5, 0.3, 0.004, 30
+    t = pd.PD_F32 if mixed else pd.PD_F64
+    vd = pd.VectorDist(len(x), lo, box, bc, rc + skin, dtype=F64, props=[(t, 3), (t, 3)])
+    vd.hostToDevicePos(x)
+    vd.hostToDeviceProp(0, v.astype(F32 if mixed else F64))
+    md = pd.MD(vd, 0, 1, dt=dt, skin=skin, r_cut=rc, precision=pd.PREC_MIXED if mixed else pd.PREC_FP64)
+    E = np.concatenate([md.run(k) for k in (1, 14, 15)])
+    tx = md.launch_shape()["tile_tx"]
+    assert 1 <= tx <= 5  # (5 + 2 cells) * 9 * 88 records of 32 bytes are the most that fit 200 KB
+    builds = E[:, 3].sum()
+    assert builds >= 2  # the width was chosen again at rebuilds
+    _, _, Eo = orc.md_lj(x, v, lo, box, bc, rc + skin, rc, skin, 1.0, 1.0, dt, 1.0, steps)
+    if mixed:
+        tot, toto = E[:, 0] + E[:, 1], Eo[1:, 0] + Eo[1:, 1]
+        assert np.max(np.abs(tot - toto) / np.abs(toto)) < 2e-5
+    else:
+        np.testing.assert_allclose(E[:, :3], Eo[1:, :3], rtol=1e-9)
