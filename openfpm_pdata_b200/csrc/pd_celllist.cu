@@ -140,7 +140,7 @@ int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cud
         PD_LAUNCH_CHECK();
     }
     PD_TRY(scan_u32(cl->cell_cnt.as<unsigned int>(), cl->cell_start.as<unsigned int>(), nc + 1, nullptr,
-                    h->scan_scratch, st, &h->ctrl->err));
+                    h->scan_scratch, st));
     if (n_part > 0) {
         unsigned g = grid_for(n_part, 256);
         pd::launch(k_cl_scatter, g, 256, 0, st, n_part, n_part_dev, n_add, cl->cell_of.as<unsigned int>(),
@@ -480,8 +480,10 @@ int pd_celllist_update(pd_vd h, pd_cl cl, unsigned long prop_mask, void* stream)
         PD_TRY(h->tile_cnt.ensure(sizeof(unsigned int) * nt));
         const DomSlot f{cl->sorted.as<const int>(), h->n_real};
         pd::launch(k_flag_count<DomSlot>, nt, FT_BLOCK, 0, st, f, n, h->tile_cnt.as<unsigned int>());
+        bool scanned;
+        PD_TRY(prefix_tiles(h->tile_cnt.as<unsigned int>(), nt, st, &scanned));
         pd::launch(k_flag_fill<DomSlot>, nt, FT_BLOCK, 0, st, f, n, (const unsigned int*)h->tile_cnt.as<unsigned int>(),
-                   cl->dom_sort.as<unsigned int>(), (unsigned int*)nullptr);
+                   scanned, cl->dom_sort.as<unsigned int>(), (unsigned int*)nullptr);
         PD_LAUNCH_CHECK();
     }
     if (cl->opt & PD_CL_GPU_REORDER) {
@@ -494,10 +496,6 @@ int pd_celllist_update(pd_vd h, pd_cl cl, unsigned long prop_mask, void* stream)
         cl->reordered = false;
     }
     PD_TRY(read_ctrl(h, st));
-    if (h->ctrl_h->err & ERR_TIMEOUT) {
-        set_error("cell list: a device wait gave up");
-        return PD_ETIMEOUT;
-    }
     if (h->ctrl_h->err & ERR_CELL_RANGE) {
         unsigned int z = 0;
         cudaMemcpy(&h->ctrl->err, &z, sizeof(z), cudaMemcpyHostToDevice);

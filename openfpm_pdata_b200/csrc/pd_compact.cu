@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(CT_BLOCK) k_flip_mark(E* __restrict__ m, long 
 // with eight loads a thread at 64 registers).
 template <class E>
 __global__ void __launch_bounds__(CT_BLOCK, 4) k_compact(const E* __restrict__ flipped, ColSet C, long n,
-                                                      const unsigned int* __restrict__ part,
+                                                      const unsigned int* __restrict__ part, bool scanned,
                                                       unsigned int* __restrict__ n_keep) {
     const long i0 = (long)blockIdx.x * CT_TILE + threadIdx.x;
     unsigned int kept = 0;
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(CT_BLOCK, 4) k_compact(const E* __restrict__ f
         if (i < n && flipped[i] != E(0)) kept |= 1u << k;
     }
     unsigned int d[CT_ITEMS], total;  // (n < 2^32)
-    tile_offsets<CT_BLOCK, CT_ITEMS>(kept, tile_prefix<CT_BLOCK>(part, blockIdx.x), d, &total);
+    tile_offsets<CT_BLOCK, CT_ITEMS>(kept, tile_before<CT_BLOCK>(part, blockIdx.x, scanned), d, &total);
     if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1) *n_keep = total;
     for (int k = 0; k < CT_ITEMS; ++k) {
         if (!(kept >> k & 1u)) continue;
@@ -185,7 +185,8 @@ int pd_remove_marked(pd_vd h, int prop, void* stream) {
     typed([&](auto* m) {
         pd::launch(k_flip_mark<std::decay_t<decltype(*m)>>, (unsigned)nt, CT_BLOCK, 0, st, m, n, part);
     });
-    int rc = PD_OK;
+    bool scanned = false;
+    int rc = prefix_tiles(part, nt, st, &scanned);
     for (size_t c0 = 0; c0 < cols.size() && rc == PD_OK; c0 += CMAXC) {
         const size_t c1 = std::min(cols.size(), c0 + (size_t)CMAXC);
         ColSet C;
@@ -199,7 +200,7 @@ int pd_remove_marked(pd_vd h, int prop, void* stream) {
         typed([&](auto* m) {
             typedef std::decay_t<decltype(*m)> E;
             pd::launch(k_compact<E>, (unsigned)nt, CT_BLOCK, 0, st, (const E*)m, C, n, (const unsigned int*)part,
-                       &h->ctrl->n_keep);
+                       scanned, &h->ctrl->n_keep);
         });
         if (cudaGetLastError() != cudaSuccess) rc = PD_ECUDA;
     }
@@ -247,10 +248,15 @@ int pd_get_indexes_by_type(pd_vd h, int prop, int cmp, long long value, long end
     const unsigned nt = (unsigned)((n + FT_TILE - 1) / FT_TILE);
     PD_TRY(h->tile_cnt.ensure(sizeof(unsigned int) * nt));
     unsigned int* cnt = h->tile_cnt.as<unsigned int>();
+    int rc = PD_OK;
     auto go = [&](auto f) {
         typedef decltype(f) F;
+        bool scanned;
         pd::launch(k_flag_count<F>, nt, FT_BLOCK, 0, st, f, n, cnt);
-        pd::launch(k_flag_fill<F>, nt, FT_BLOCK, 0, st, f, n, (const unsigned int*)cnt, out, &h->ctrl->n_keep);
+        rc = prefix_tiles(cnt, nt, st, &scanned);
+        if (rc == PD_OK)
+            pd::launch(k_flag_fill<F>, nt, FT_BLOCK, 0, st, f, n, (const unsigned int*)cnt, scanned, out,
+                       &h->ctrl->n_keep);
     };
     switch (P.type) {
         case PD_F64: go(CmpFlag<double>{(const double*)P.d, (double)value, cmp}); break;
@@ -260,6 +266,7 @@ int pd_get_indexes_by_type(pd_vd h, int prop, int cmp, long long value, long end
         case PD_I64: go(CmpFlag<long long>{(const long long*)P.d, value, cmp}); break;
         default: return PD_EINVAL;
     }
+    PD_TRY(rc);
     PD_LAUNCH_CHECK();
     PD_TRY(read_ctrl(h, st));
     const long m = h->ctrl_h->n_keep;
@@ -302,8 +309,8 @@ int pd_slab_halo(const double* x, long n, int axis, double lo_thr, double hi_thr
     const unsigned g = grid_for(n, 256);
     pd::launch(k_slab_mark, g, 256, 0, st, x, n, axis, lo_thr, hi_thr, f0, f1);
     PD_LAUNCH_CHECK();
-    PD_TRY(scan_u32(f0, o0, n, tot, scratch, st, nullptr));
-    PD_TRY(scan_u32(f1, o1, n, tot + 1, scratch, st, nullptr));
+    PD_TRY(scan_u32(f0, o0, n, tot, scratch, st));
+    PD_TRY(scan_u32(f1, o1, n, tot + 1, scratch, st));
     pd::launch(k_fill_indexes, g, 256, 0, st, (const unsigned int*)f0, (const unsigned int*)o0, n, l0);
     pd::launch(k_fill_indexes, g, 256, 0, st, (const unsigned int*)f1, (const unsigned int*)o1, n, l1);
     PD_LAUNCH_CHECK();

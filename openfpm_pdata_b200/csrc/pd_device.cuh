@@ -188,88 +188,15 @@ __device__ __forceinline__ void atomic_max_nonneg(unsigned long long* a, double 
 }
 
 // ---------------------------------------------------------------------------
-// Single-pass prefix sums over tiles (decoupled look-back: Merrill & Garland, "Single-
-// pass parallel prefix scan with decoupled look-back", 2016).  A tile publishes its own
-// sum, then adds up the sums of the tiles before it until it meets one that has already
-// published its running total; flag and value share one 64-bit word, so no fence is
-// needed.  Tiles are numbered by a ticket in the order in which their CTAs start, so
-// the tiles waited for have started; the wait is bounded all the same.  The last CTA to
-// finish clears the words, so the state is all zero between launches (also under graph
-// replay) and needs clearing only when it is allocated (lookback_ensure).
-struct Lookback {
-    unsigned int ticket, done, pad[2];
-    unsigned long long word[1];  // one per tile: flag (1 own sum, 2 running total) << 32 | value
-};
-__device__ __forceinline__ unsigned int lookback_tile(Lookback* L, unsigned int* sh) {
-    if (threadIdx.x == 0) *sh = atomicAdd(&L->ticket, 1u);
-    __syncthreads();
-    return *sh;
-}
-// By the whole CTA: the sum of all tiles before `tile`, whose own sum is `agg` (the same in
-// every thread); *ok is cleared in a thread whose wait gave up.  A step looks at BLOCK
-// tiles, one a thread: the CTAs of a wave all publish at about the same time, and a
-// warp's window of 32 took a step of an L2 round trip for each 32 of them (17 us for 500
-// tiles).
-template <int BLOCK>
-__device__ __forceinline__ unsigned int lookback_sum(Lookback* L, unsigned int tile, unsigned int agg, bool* ok) {
-    constexpr int NW = BLOCK / 32;
-    __shared__ unsigned int part[NW], ends[NW];
-    volatile unsigned long long* word = L->word;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    unsigned int excl = 0;
-    if (tile > 0) {
-        if (threadIdx.x == 0) word[tile] = (1ull << 32) | agg;
-        bool found = false;
-        for (long last = (long)tile - 1; !found; last -= BLOCK) {
-            const long idx = last - (long)threadIdx.x;
-            unsigned long long v = 2ull << 32;  // before the first tile: a running total of zero
-            if (idx >= 0) {
-                unsigned int it = 0;
-                while (((v = word[idx]) >> 32) == 0ull && ++it < (1u << 24)) {
-                }
-                if ((v >> 32) == 0ull) {
-                    *ok = false;
-                    v = 2ull << 32;
-                }
-            }
-            const unsigned int full = __ballot_sync(0xffffffffu, (v >> 32) == 2ull);
-            unsigned int add = lane <= (full ? __ffs(full) - 1 : 31) ? (unsigned int)v : 0u;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-            if (lane == 0) {
-                part[w] = add;
-                ends[w] = full;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < NW; ++j) {
-                if (!found) excl += part[j];
-                found = found || ends[j] != 0u;
-            }
-            __syncthreads();
-        }
-    }
-    if (threadIdx.x == 0) word[tile] = (2ull << 32) | (unsigned long long)(excl + agg);
-    return excl;
-}
-// by the whole CTA at its end: the last one clears the state of `nt` tiles
-__device__ __forceinline__ void lookback_finish(Lookback* L, unsigned int nt, unsigned int* sh) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        *sh = atomicAdd(&L->done, 1u);
-    }
-    __syncthreads();
-    if (*sh != nt - 1) return;
-    for (unsigned int i = threadIdx.x; i < nt; i += blockDim.x) L->word[i] = 0ull;
-    if (threadIdx.x == 0) L->ticket = L->done = 0u;
-}
-
-// ---------------------------------------------------------------------------
-// Stable compaction in two kernels: one counts each tile's elements, the other adds up
-// the counts of the tiles before its own (a few words a thread, from L2) and writes.
-// Where a pass needs thousands of tiles this beats a look-back: 1000 tiles of int marks
-// 31 us by look-back (the polling of a wave's CTAs congests the words they wait for).
+// Prefix sums over tiles in two kernels: one leaves each tile's sum, the other adds up the
+// sums of the tiles before its own (a few words a thread, from L2) and writes.  No CTA waits
+// for another.  Adding up costs the square of the number of tiles, so beyond PREFIX_TILES a
+// launch of one CTA scans the sums in between (prefix_tiles).  Scan of n counts in tiles of
+// 4096, us a call back to back, added up / scanned in between / decoupled look-back in one
+// launch: 17 tiles 8.3 / 12.3 / 6.4, 128 8.2 / 12.4 / 8.0, 1024 14.4 / 16.5 / 24.8, 4096
+// 45.4 / 48.5 / 99.8, 8192 88 / 91 / 199, 16384 170 / 168 / 395 (a look-back's polling
+// congests the words that it waits for).
+static constexpr long PREFIX_TILES = 8192;
 
 // by the whole CTA: the sum of cnt[0, tile), the same in every thread
 template <int BLOCK>
@@ -286,6 +213,13 @@ __device__ __forceinline__ unsigned int tile_prefix(const unsigned int* __restri
     for (int j = 0; j < BLOCK / 32; ++j) s += part[j];
     __syncthreads();
     return s;
+}
+
+// the same where `scanned` says that the counts have become the sums before each tile
+template <int BLOCK>
+__device__ __forceinline__ unsigned int tile_before(const unsigned int* __restrict__ cnt, unsigned int tile,
+                                                    bool scanned) {
+    return scanned ? cnt[tile] : tile_prefix<BLOCK>(cnt, tile);
 }
 
 // Offsets of a tile's flagged items: item k of thread t is element base + k * BLOCK + t,
@@ -351,12 +285,12 @@ template <class F> __global__ void __launch_bounds__(FT_BLOCK) k_flag_count(F f,
 }
 template <class F>
 __global__ void __launch_bounds__(FT_BLOCK) k_flag_fill(F f, long n, const unsigned int* __restrict__ cnt,
-                                                        unsigned int* __restrict__ out,
+                                                        bool scanned, unsigned int* __restrict__ out,
                                                         unsigned int* __restrict__ total) {
     const long base = (long)blockIdx.x * FT_TILE;
     const unsigned int flags = tile_flags(f, n, base);
     unsigned int off[FT_ITEMS], tot;
-    tile_offsets<FT_BLOCK, FT_ITEMS>(flags, tile_prefix<FT_BLOCK>(cnt, blockIdx.x), off, &tot);
+    tile_offsets<FT_BLOCK, FT_ITEMS>(flags, tile_before<FT_BLOCK>(cnt, blockIdx.x, scanned), off, &tot);
     if (threadIdx.x == 0 && blockIdx.x == gridDim.x - 1 && total) *total = tot;
 #pragma unroll
     for (int k = 0; k < FT_ITEMS; ++k)

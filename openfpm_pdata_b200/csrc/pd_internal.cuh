@@ -106,12 +106,12 @@ inline int type_size(int t) {
     }
 }
 
-// room for the look-back state of `nt` tiles in `b`, cleared when it is (re)allocated
-int lookback_ensure(Buf& b, long nt, cudaStream_t st);
-// exclusive scan of n uint32 values (in may equal out); writes the total to *total_dev;
-// ERR_TIMEOUT into *err if a wait gave up
+// the sums of `nt` tiles into the sums before each where adding them up in every tile costs
+// more (PREFIX_TILES in pd_device.cuh); *scanned says whether
+int prefix_tiles(unsigned int* cnt, long nt, cudaStream_t st, bool* scanned);
+// exclusive scan of n uint32 values (in may equal out); writes the total to *total_dev
 int scan_u32(const unsigned int* in, unsigned int* out, long n, unsigned int* total_dev, Buf& scratch,
-             cudaStream_t st, unsigned int* err);
+             cudaStream_t st);
 
 inline unsigned int grid_for(long n, int block, long cap_blocks = 148L * 64) {
     long g = (n + block - 1) / block;

@@ -235,7 +235,7 @@ int pd_slab_map_label(pd_vd h, const pd_slab_t* s, long* send_counts, void* stre
     unsigned int* tot = h->slab_tot.as<unsigned int>();
     for (int d = 0; d < P; ++d) {
         pd::launch(k_slab_eq, g, 256, 0, st, (const int*)dest, n, d, flag);
-        PD_TRY(scan_u32(flag, off, n, tot + d, h->scan_scratch, st, &h->ctrl->err));
+        PD_TRY(scan_u32(flag, off, n, tot + d, h->scan_scratch, st));
         pd::launch(k_slab_fill, g, 256, 0, st, (const unsigned int*)flag, (const unsigned int*)off, n,
                    (const unsigned int*)tot, d, (unsigned char)0, h->slab_idx.as<int>(), (unsigned char*)nullptr);
         PD_LAUNCH_CHECK();
@@ -292,7 +292,7 @@ int pd_slab_halo_label(pd_vd h, const pd_slab_t* s, int rank, long* send_counts,
         else
             pd::launch(k_slab_side<float>, g, 256, 0, st, (const float4*)h->pos, n, s->axis, sides[k].side,
                        sides[k].thr, flag);
-        PD_TRY(scan_u32(flag, off, n, tot + k, h->scan_scratch, st, &h->ctrl->err));
+        PD_TRY(scan_u32(flag, off, n, tot + k, h->scan_scratch, st));
         pd::launch(k_slab_fill, g, 256, 0, st, (const unsigned int*)flag, (const unsigned int*)off, n,
                    (const unsigned int*)tot, (int)k, sides[k].shift, h->slab_idx.as<int>(),
                    h->slab_shift.as<unsigned char>());

@@ -1,6 +1,6 @@
-"""The single-pass kernels (look-back between tiles) at the edges of their tiles: ghost
-images, compaction, index selection, sorted domain slots, multi-column reorders, and the
-device-array copies, all exact."""
+"""Kernels that work in tiles, at the edges of the tiles and where the prefix sums over them
+change their form: the scan of a cell list's counts, ghost images, compaction, index
+selection, sorted domain slots, multi-column reorders, and the device-array copies, all exact."""
 import numpy as np
 import pytest
 
@@ -14,6 +14,32 @@ def pd():
     from openfpm_pdata_b200 import pd as _pd
     _pd.lib()
     return _pd
+
+
+@pytest.mark.parametrize("gs", [(3, 4, 5), (11, 12, 31), (13, 15, 21), (16, 16, 16), (15, 17, 257), (32, 32, 64),
+                                (128, 128, 257), (31, 601, 1801), (256, 256, 512)])
+def test_cell_starts(pd, gs):
+    """Cell starts are the exclusive scan of the counts: cells + 1 elements, 4093, 4096 and 4097
+    among them (one tile, two), 65536 and 65537 (the last size that one launch scans), 33554432
+    and 33554433 (the last whose tiles each add up the ones before).  Twice in a row."""
+    rng = np.random.default_rng(sum(gs))
+    L = np.array(gs) - 2.5
+    n = 20011
+    x = rng.random((n, 3)) * L
+    x[: n // 3] = L - rng.random((n // 3, 3)) * np.minimum(L, 2.0)  # many in the last cells
+    vd = pd.VectorDist(n, np.zeros(3), L, np.zeros(3, np.int32), 0.0)
+    vd.hostToDevicePos(x)
+    cl = vd.getCellListGPU(1.0)
+    v = cl.view()
+    assert tuple(v.gs) == gs
+    c = np.floor((x - np.array(v.box_lo)) / np.array(v.spacing)).astype(np.int64) + v.pad
+    cell = c[:, 0] + gs[0] * (c[:, 1] + gs[1] * c[:, 2])
+    want = np.concatenate([[0], np.cumsum(np.bincount(cell, minlength=v.ncells))])
+    for _ in range(2):
+        vd.updateCellListGPU(cl)
+        cs, so = cl.get()
+        assert np.array_equal(cs, want)
+        assert np.array_equal(so, np.argsort(cell, kind="stable"))
 
 
 @pytest.mark.parametrize("dtype", [F32, F64])
