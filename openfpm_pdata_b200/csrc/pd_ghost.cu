@@ -70,7 +70,7 @@ __global__ void k_ghost_count(const typename V4<T>::type* __restrict__ pos, long
 // image) and leaves each tile's images as a list of (particle within the tile, box),
 // particle-major with ascending boxes, in a region of `list` taken with one atomic; the
 // regions lie in any order.  k_ghost_write gets the images of the tiles before its own
-// from the tile counts and writes one image a thread: consecutive slots, coalesced, the
+// from the tile counts (tile_before) and writes one image a thread: consecutive slots, coalesced, the
 // images of a particle in flight together.  Image j of particle p comes to slot
 // n + start(p) + j.  Measured against count, scan (three kernels) and write, which read
 // every record twice and wrote a particle's images one after the other: see
@@ -80,7 +80,8 @@ template <class T, int ITEMS>
 __global__ void __launch_bounds__(GM_BLOCK) k_ghost_find(const typename V4<T>::type* __restrict__ pos, long n,
                                                          const BoxSet<T>* __restrict__ Bp, unsigned int cap_list,
                                                          unsigned int* __restrict__ list,
-                                                         unsigned int* __restrict__ taken, uint2* __restrict__ tiles) {
+                                                         unsigned int* __restrict__ taken, uint2* __restrict__ tiles,
+                                                         unsigned int* __restrict__ cnt_t) {
     constexpr int NW = GM_BLOCK / 32, NC = ITEMS * NW;
     static_assert(NC <= 32, "one count a lane in the tile's scan");
     __shared__ BoxSet<T> B;
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(GM_BLOCK) k_ghost_find(const typename V4<T>::t
         if (lane == 31) {
             sh_base = x ? atomicAdd(taken, x) : 0u;
             tiles[blockIdx.x] = make_uint2(x, sh_base);
+            cnt_t[blockIdx.x] = x;
         }
     }
     __syncthreads();
@@ -151,18 +153,14 @@ __global__ void __launch_bounds__(GM_BLOCK) k_ghost_write(typename V4<T>::type* 
                                                           const BoxSet<T>* __restrict__ B,
                                                           const T* __restrict__ shifts,
                                                           const unsigned int* __restrict__ list, unsigned int cap_list,
-                                                          const uint2* __restrict__ tiles, int* __restrict__ src,
+                                                          const uint2* __restrict__ tiles,
+                                                          const unsigned int* __restrict__ cnt, bool scanned,
+                                                          int* __restrict__ src,
                                                           unsigned char* __restrict__ shf, long img_cap, long cap,
                                                           PropCopy pc, unsigned int* __restrict__ n_img,
                                                           unsigned int* __restrict__ err) {
-    __shared__ unsigned int part[1];
     const unsigned int t = blockIdx.x;
-    unsigned int s = 0;
-    for (unsigned int j = threadIdx.x; j < t; j += GM_BLOCK) s += tiles[j].x;
-    s = block_sum<unsigned int, GM_BLOCK>(s);
-    if (threadIdx.x == 0) part[0] = s;
-    __syncthreads();
-    const long m0 = part[0];
+    const long m0 = tile_before<GM_BLOCK>(cnt, t, scanned);
     const uint2 mine = tiles[t];
     if (threadIdx.x == 0 && t == gridDim.x - 1) *n_img = (unsigned int)m0 + mine.x;
     for (unsigned int j = threadIdx.x; j < mine.x; j += GM_BLOCK) {
@@ -368,19 +366,24 @@ static int ghost_make(pd_vd h, long m_cap, cudaStream_t st) {
     // four particles a thread, one where that would leave SMs without a tile
     const int items = n >= 148L * GM_BLOCK * 4 ? 4 : 1;
     const unsigned nt = (unsigned)((n + GM_BLOCK * items - 1) / (GM_BLOCK * items));
-    // tile records behind the word that counts the list entries taken
-    PD_TRY(h->tile_cnt.ensure(sizeof(uint2) * ((size_t)nt + 1)));
+    // tile records behind the word that counts the list entries taken, then the tiles' counts
+    PD_TRY(h->tile_cnt.ensure(sizeof(uint2) * ((size_t)nt + 1) + sizeof(unsigned int) * (size_t)nt));
     PD_TRY(h->img_list.ensure(sizeof(unsigned int) * (size_t)(m_cap > 0 ? m_cap : 1)));
     unsigned int* taken = h->tile_cnt.as<unsigned int>();
     uint2* tiles = h->tile_cnt.as<uint2>() + 1;
+    unsigned int* cnt = reinterpret_cast<unsigned int*>(tiles + nt);
+    int rc = PD_OK;
     PD_CUDA(cudaMemsetAsync(taken, 0, sizeof(unsigned int), st));
     auto go = [&](auto find, auto write, auto* pos, auto* boxes, auto* shifts) {
         pd::launch(find, nt, GM_BLOCK, 0, st, pos, n, boxes, (unsigned int)m_cap, h->img_list.as<unsigned int>(), taken,
-                   tiles);
+                   tiles, cnt);
+        bool scanned;
+        rc = prefix_tiles(cnt, nt, st, &scanned);
+        if (rc != PD_OK) return;
         pd::launch(write, nt, GM_BLOCK, 0, st, pos, h->gid, n, GM_BLOCK * items, boxes, shifts,
                    (const unsigned int*)h->img_list.as<unsigned int>(), (unsigned int)m_cap, (const uint2*)tiles,
-                   h->img_src.as<int>(), h->img_shift.as<unsigned char>(), m_cap, h->cap, pc, &h->ctrl->n_img,
-                   &h->ctrl->err);
+                   (const unsigned int*)cnt, scanned, h->img_src.as<int>(), h->img_shift.as<unsigned char>(), m_cap,
+                   h->cap, pc, &h->ctrl->n_img, &h->ctrl->err);
     };
     if (h->dtype == PD_F64) {
         const BoxSet<double>* b = h->boxes.as<BoxSet<double>>();
@@ -391,6 +394,7 @@ static int ghost_make(pd_vd h, long m_cap, cudaStream_t st) {
         const float* sh = h->shifts.as<float>();
         go(items == 4 ? k_ghost_find<float, 4> : k_ghost_find<float, 1>, k_ghost_write<float>, (float4*)h->pos, b, sh);
     }
+    PD_TRY(rc);
     PD_LAUNCH_CHECK();
     return PD_OK;
 }

@@ -42,6 +42,32 @@ def test_cell_starts(pd, gs):
         assert np.array_equal(so, np.argsort(cell, kind="stable"))
 
 
+def test_many_tiles(pd, orc):
+    """More tiles than add up their predecessors: ghost images (1,024 particles a tile), index
+    selection and removal (4,096)."""
+    import torch
+    n, g = 8400001, 0.01
+    lo, hi, bc = np.zeros(3), np.ones(3), np.ones(3, np.int32)
+    x = np.random.default_rng(8).random((n, 3), dtype=F32)
+    vd = pd.VectorDist(n, lo, hi, bc, g, dtype=F32)
+    vd.hostToDevicePos(x)
+    vd.ghost_get()
+    img, src, _ = orc.ghost_get(x, lo.astype(F32), hi.astype(F32), bc, g)
+    assert np.array_equal(vd.ghost_records()[0], src)
+    assert np.array_equal(vd.deviceToHostPos()[n:], img)
+    del vd
+    n = 8193 * 4096 + 5
+    vd = pd.VectorDist(n, lo, hi, bc, g, dtype=F32, props=[(pd.PD_I32, 1)])
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.rand((n, 3), device="cuda", generator=gen)
+    mark = (torch.rand(n, device="cuda", generator=gen) < 0.2).int()
+    vd.hostToDevicePos(x)
+    vd.hostToDeviceProp(0, mark)
+    assert torch.equal(vd.get_indexes_by_type(0, 1, device=True).long(), mark.nonzero()[:, 0])
+    vd.remove_marked(0)
+    assert torch.equal(vd.deviceToHostPos(device=True), x[mark == 0])
+
+
 @pytest.mark.parametrize("dtype", [F32, F64])
 @pytest.mark.parametrize("n,corner", [(1, True), (1023, False), (1024, False), (1025, True), (40000, False),
                                       (20001, True)])
