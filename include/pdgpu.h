@@ -265,6 +265,9 @@ int pd_get_indexes_by_type(pd_vd h, int prop, int cmp, long long value, long end
  * nothing completes the phase: the wait gives up, the kernel records the timeout
  * and returns, and the call returns PD_ETIMEOUT with the context still usable. */
 int pd_selftest_wait(long limit, int issue_copy, const float* in4, float* out4);
+/* Sets, from the host, the error bit that a device wait of `h` sets when it gives up: the
+ * next call that builds a Verlet list or runs steps on `h` returns PD_ETIMEOUT, once. */
+int pd_selftest_raise_timeout(pd_vd h);
 /* Measured vector FMA throughput of this GPU in TFLOP/s (an FMA counts two flops),
  * FP32 or FP64: the denominator of the pair kernels' arithmetic roofline. */
 int pd_measure_fma_rate(int dtype, double* tflops);

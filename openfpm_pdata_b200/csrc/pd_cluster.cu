@@ -425,6 +425,7 @@ template <class T> static int md_run_cluster_t(pd_md md, int steps, cudaStream_t
     PD_CUDA(cudaMemcpyAsync(&tot, A.tot, sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
     if (E && steps > 0) PD_CUDA(cudaMemcpyAsync(E, md->E.p, sizeof(double) * 4 * steps, cudaMemcpyDeviceToHost, st));
     PD_TRY(read_ctrl(h, st));  // synchronises the stream
+    PD_TRY(take_timeout(h, "pd_md_run", st));
     if (h->ctrl_h->err & (ERR_IMG_OVERFLOW | ERR_CELL_RANGE)) {
         set_error("pd_md_run: cluster step overflow or particle outside the cell grid (err=0x%x)", h->ctrl_h->err);
         return PD_EOVERFLOW;
@@ -873,9 +874,10 @@ template <class T> static int md_run_buckets_t(pd_md md, int steps, cudaStream_t
     h->n_total = n;
     PD_TRY(ghost_generate(h, 0, true, st));
     if (h->nbox == 0) PD_TRY(read_ctrl(h, st));
-    if (h->ctrl_h->err & (ERR_CELL_RANGE | ERR_TIMEOUT)) {
-        set_error("pd_md_run: a particle outside the cell grid or a wait that gave up (err=0x%x)", h->ctrl_h->err);
-        return (h->ctrl_h->err & ERR_TIMEOUT) ? PD_ETIMEOUT : PD_EOVERFLOW;
+    PD_TRY(take_timeout(h, "pd_md_run", st));
+    if (h->ctrl_h->err & ERR_CELL_RANGE) {
+        set_error("pd_md_run: a particle outside the cell grid (err=0x%x)", h->ctrl_h->err);
+        return PD_EOVERFLOW;
     }
     *made = (int)h->ctrl_h->run_done;
     if (*made < steps) md->bucket_off = true;  // too uneven: the one-cluster kernel from now on

@@ -481,6 +481,15 @@ int read_ctrl(pd_vd h, cudaStream_t st) {
     return PD_OK;
 }
 
+int take_timeout(pd_vd h, const char* who, cudaStream_t st) {
+    if (!(h->ctrl_h->err & ERR_TIMEOUT)) return PD_OK;
+    h->ctrl_h->err &= ~ERR_TIMEOUT;
+    PD_CUDA(cudaMemcpyAsync(&h->ctrl->err, &h->ctrl_h->err, sizeof(unsigned int), cudaMemcpyHostToDevice, st));
+    PD_CUDA(cudaStreamSynchronize(st));
+    set_error("%s: a bounded device wait gave up", who);
+    return PD_ETIMEOUT;
+}
+
 template <class T>
 __global__ void k_wrap(typename V4<T>::type* __restrict__ pos, long n, T lo0, T lo1, T lo2, T hi0, T hi1, T hi2,
                        int per0, int per1, int per2) {

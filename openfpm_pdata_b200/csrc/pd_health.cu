@@ -110,6 +110,15 @@ int pd_selftest_wait(long limit, int issue_copy, const float* in4, float* out4) 
     return PD_OK;
 }
 
+int pd_selftest_raise_timeout(pd_vd h) {
+    if (!h) return PD_EINVAL;
+    unsigned int err = 0;
+    PD_CUDA(cudaMemcpy(&err, &h->ctrl->err, sizeof(err), cudaMemcpyDeviceToHost));
+    err |= ERR_TIMEOUT;
+    PD_CUDA(cudaMemcpy(&h->ctrl->err, &err, sizeof(err), cudaMemcpyHostToDevice));
+    return PD_OK;
+}
+
 int pd_measure_fma_rate(int dtype, double* tflops) {
     if (!tflops || (dtype != PD_F32 && dtype != PD_F64)) return PD_EINVAL;
     return dtype == PD_F64 ? fma_rate<double>(tflops) : fma_rate<float>(tflops);

@@ -223,6 +223,9 @@ int alloc_storage(pd_vd h, long cap, void** pos, int** gid, std::vector<char*>& 
 void free_storage(void* pos, int* gid, const std::vector<char*>& props);
 int set_ctrl_n_img(pd_vd h, long n_img, cudaStream_t st);
 int read_ctrl(pd_vd h, cudaStream_t st);
+// PD_ETIMEOUT where the error word that read_ctrl brought says that a bounded device wait gave
+// up (the results of `who` are incomplete); the bit is cleared, so that later calls run
+int take_timeout(pd_vd h, const char* who, cudaStream_t st);
 int cl_geometry(pd_cl cl, pd_vd h, double r_cut, double enlarge, int nn_box);
 // counting sort of the particles [first, first + n_part) (ids relative to `first`)
 int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cudaStream_t st, long first = 0);

@@ -880,6 +880,7 @@ static int md_run_cl_graph(pd_md md, int steps, cudaStream_t st, double* E) {
     h->n_total = h->n_real + h->n_img;
     h->img_valid = true;
     h->img_gen_order = false;  // the step may leave the images in cell order
+    PD_TRY(take_timeout(h, "pd_md_run", st));
     if (h->ctrl_h->err & (ERR_IMG_OVERFLOW | ERR_NN_OVERFLOW | ERR_CAP_OVERFLOW)) {
         set_error("pd_md_run: device capacity overflow (err=0x%x)", h->ctrl_h->err);
         return PD_EOVERFLOW;
@@ -1380,6 +1381,7 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
     // the energies and the error word in one synchronisation
     PD_TRY(read_ctrl(h, st));
     if (md->timing) md->ev_rebuilt = std::move(rebuilt_at);  // read by pd_md_timers or the next run
+    PD_TRY(take_timeout(h, "pd_md_run", st));
     if (h->ctrl_h->err & (ERR_IMG_OVERFLOW | ERR_NN_OVERFLOW)) {
         set_error("pd_md_run: device capacity overflow (err=0x%x)", h->ctrl_h->err);
         return PD_EOVERFLOW;

@@ -609,7 +609,8 @@ int tile_build(pd_vd h, const TileGeom& tg, long ntiles, const unsigned int* csR
             *small = true;
             return PD_ESTATE;
         }
-        if (h->ctrl_h->err & (ERR_TILE_CAP | ERR_TIMEOUT)) {
+        PD_TRY(take_timeout(h, "tiled Verlet build", st));
+        if (h->ctrl_h->err & ERR_TILE_CAP) {
             set_error("tiled Verlet build failed (err=0x%x)", h->ctrl_h->err);
             return PD_EOVERFLOW;
         }

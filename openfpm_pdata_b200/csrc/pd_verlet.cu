@@ -339,6 +339,7 @@ int verlet_build(pd_vd h, pd_vl vl, long n_dom, const unsigned int* n_img_dev, c
         }
         if (!check) return PD_OK;
         PD_TRY(read_ctrl(h, st));
+        PD_TRY(take_timeout(h, "Verlet list", st));
         if (!(h->ctrl_h->err & ERR_NN_OVERFLOW)) break;
         // grow and rebuild
         vl->max_nn = (int)(h->ctrl_h->nn_max * 1.15 + 8);

@@ -136,6 +136,7 @@ def lib():
             "pd_remove_marked": ([vp, ip, vp], ip),
             "pd_save": ([vp, ctypes.c_char_p], ip),
             "pd_selftest_wait": ([ctypes.c_long, ip, vp, vp], ip),
+            "pd_selftest_raise_timeout": ([vp], ip),
             "pd_measure_fma_rate": ([ip, P(ctypes.c_double)], ip),
             "pd_load": ([vp, ctypes.c_char_p], ip),
             "pd_write": ([vp, ctypes.c_char_p, ctypes.c_char_p, ip], ip),
