@@ -386,13 +386,14 @@ __global__ void __launch_bounds__(128) k_test_force(const typename V4<T>::type* 
                         const T wq = p0[q];
                         const T rx = xq.x - xp.x, ry = xq.y - xp.y, rz = xq.z - xp.z;
                         const T r2 = rx * rx + ry * ry + rz * rz;
-                        // every pair through the same instructions; too close (the particle
-                        // itself among them): no contribution
-                        const T w = wq * rsqrt_series(r2);
-                        const T ws = r2 > min2 ? w : T(0);
-                        fx += ws * rx;
-                        fy += ws * ry;
-                        fz += ws * rz;
+                        // too close (the particle itself among them) or not a distance (NaN): no
+                        // contribution.  The direction first: w / r overflows for large weights
+                        const T y = rsqrt_series(r2);
+                        if (r2 > min2) {
+                            fx += wq * (rx * y);
+                            fy += wq * (ry * y);
+                            fz += wq * (rz * y);
+                        }
                     }
                 }
             }
