@@ -509,6 +509,7 @@ __device__ __forceinline__ bool grid_barrier(cg::cluster_group& cl, unsigned int
     __threadfence();
     cl.sync();
     if (cl.block_rank() == 0 && threadIdx.x == 0) {
+        __threadfence();  // the arrival releases what the cluster's other threads wrote before cl.sync()
         atomicAdd(bar, 1u);
         unsigned int seen = 0, it = 0;
         do {

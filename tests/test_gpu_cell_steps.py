@@ -82,3 +82,16 @@ def test_run_equals_single_steps(pd, dtype, kind, bc):
     assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[1]))
     if kind != "clump":  # (there the two kernels share the runs differently)
         assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[2]))
+
+
+def test_large_run_repeats(pd):
+    """64,000 particles, every cluster of the GPU and several cells a CTA: what a step's CTAs write is
+    there for all of them in the next, so a run repeats bit for bit and equals runs of one step."""
+    from openfpm_pdata_b200 import workloads
+    x, v, L = workloads.lj_lattice(40, 1.05, 0.05, seed=6)
+    runs = []
+    for parts in ([60], [60], [1] * 60):
+        vd, md = _md(pd, x, v, L, (1, 1, 1), F64)
+        runs.append((np.concatenate([md.run(k) for k in parts]),) + _by_id(vd))
+    for r in runs[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(runs[0], r))
