@@ -398,6 +398,8 @@ int pd_md_timers(pd_md md, double* ms, long* counts);
  * place; 0 before such a run), and the tile width in cells and lanes per particle of the tiled rows of the last
  * build (0 and 0 without them) */
 int pd_md_launch_shape(pd_md md, int* cluster_ctas, int* tile_tx, int* threads_per_particle);
+/* steps of a small cell-list system made on the whole GPU so far (the others on one cluster) */
+int pd_md_bucket_steps(pd_md md, long* steps);
 
 /* ---- serving loop -------------------------------------------------------- */
 /* Many independent periodic LJ systems (precision form, FP32 forces / FP64

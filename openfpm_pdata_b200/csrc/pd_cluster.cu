@@ -884,6 +884,7 @@ template <class T> static int md_run_buckets_t(pd_md md, int steps, cudaStream_t
     if (*made < steps) md->bucket_off = true;  // too uneven: the one-cluster kernel from now on
     md->steps += *made;
     md->builds += *made;
+    md->bucket_steps += *made;
     h->epoch++;
     return PD_OK;
 }

@@ -1408,6 +1408,12 @@ int pd_md_launch_shape(pd_md md, int* cluster_ctas, int* tile_tx, int* threads_p
     return PD_OK;
 }
 
+int pd_md_bucket_steps(pd_md md, long* steps) {
+    if (!md || !steps) return PD_EINVAL;
+    *steps = md->bucket_steps;
+    return PD_OK;
+}
+
 int pd_md_timers(pd_md md, double* ms, long* counts) {
     if (!md || !ms || !counts) return PD_EINVAL;
     md_fold_timing(md);

@@ -59,6 +59,7 @@ struct pd_md_s {
     int cluster_ctas = 0;  // CTAs of a cluster of the last small cell-list run (0: none so far)
     pd::Buf buckets;          // cell-list mode of a small system: buckets, counts, partial sums
     bool bucket_off = false;  // a bucket overflowed: an uneven system
+    long bucket_steps = 0;    // steps made by the bucket kernel
     // optional per-phase device timing (CUDA events on the run's stream)
     bool timing = false;
     std::vector<cudaEvent_t> evp;  // six per step of a timed run, recorded without synchronising

@@ -160,6 +160,7 @@ def lib():
             "pd_set_cache_limit": ([lp, P(ctypes.c_long)], ip),
             "pd_md_list_stats": ([vp, P(ctypes.c_long), P(ctypes.c_double), P(ctypes.c_int)], ip),
             "pd_md_launch_shape": ([vp, P(ctypes.c_int), P(ctypes.c_int), P(ctypes.c_int)], ip),
+            "pd_md_bucket_steps": ([vp, P(ctypes.c_long)], ip),
             "pd_celllist_build_static": ([ip, vp, lp, dp, dp, P(ctypes.c_int), ip, vp, vp, vp, vp], ip),
             "pd_slab_map_label": ([vp, P(SlabT), P(ctypes.c_long), vp], ip),
             "pd_slab_halo_label": ([vp, P(SlabT), ip, P(ctypes.c_long), vp], ip),
@@ -715,6 +716,12 @@ class MD:
         c, t, p = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
         check(lib().pd_md_launch_shape(self.h, ctypes.byref(c), ctypes.byref(t), ctypes.byref(p)))
         return {"cluster_ctas": c.value, "tile_tx": t.value, "threads_per_particle": p.value}
+
+    def bucket_steps(self):
+        """Steps of a small cell-list system made on the whole GPU so far (the others on one cluster)."""
+        n = ctypes.c_long(0)
+        check(lib().pd_md_bucket_steps(self.h, ctypes.byref(n)))
+        return n.value
 
     def stats(self):
         b, s, e = ctypes.c_long(0), ctypes.c_long(0), ctypes.c_int(0)

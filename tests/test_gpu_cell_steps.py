@@ -1,7 +1,8 @@
-"""The cell-list driver's bucket kernel against the FP64 oracle and the one-cluster kernel
-it hands over to: the smallest systems, a box of few cells, open boundaries, FP32 storage,
-and a system whose densest cell overflows a bucket.  A run equals runs of one step and a
-second identical run bit for bit (the order in which buckets fill does not matter)."""
+"""The cell-list driver's bucket kernel against the FP64 oracle: the smallest systems, a box
+of few cells, open boundaries, FP32 storage, a dense corner of an empty box.  A run equals
+runs of one step and a second identical run bit for bit (the order in which buckets fill does
+not matter).  The one-cluster kernel that it hands over to where a bucket overflows: from the
+first step, after an odd and after an even number of steps."""
 import numpy as np
 import pytest
 
@@ -39,7 +40,7 @@ def _system(kind):
     from openfpm_pdata_b200 import workloads
     if kind == "one":
         return np.array([[1.0, 7.9, 0.1]]), np.array([[3.0, 2.0, -4.0]]), 8.0
-    if kind == "clump":  # 1728 particles at spacing 1.0 in a corner of a box of 30: 15.6 a cell there, 0.2 on average
+    if kind == "clump":  # 1728 particles in a corner of a box of 60: up to 27 a cell there, 0.1 on average
         x, v, _ = workloads.lj_lattice(12, 0.98, 0.03, seed=4)
         return x + 0.5, v * 0.3, 60.0
     side, sp = {"few cells": (8, 1.02), "c1": (16, 1.0), "many": (33, 1.05)}[kind]
@@ -80,8 +81,8 @@ def test_run_equals_single_steps(pd, dtype, kind, bc):
         E = np.concatenate([md.run(k) for k in parts])
         runs.append((E,) + _by_id(vd))
     assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[1]))
-    if kind != "clump":  # (there the two kernels share the runs differently)
-        assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[2]))
+    assert all(np.array_equal(a, b) for a, b in zip(runs[0], runs[2]))
+    assert md.bucket_steps() == 17
 
 
 def test_large_run_repeats(pd):
@@ -95,3 +96,55 @@ def test_large_run_repeats(pd):
         runs.append((np.concatenate([md.run(k) for k in parts]),) + _by_id(vd))
     for r in runs[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(runs[0], r))
+
+
+DT_FLY = 0.002
+
+
+def _crowding(pd, k, extra=0):
+    """Buckets hold 32 records here (0.02 particles a cell on average).  One cell holds 32 particles at
+    rest; another flies into it and arrives with step k, leaving after about 60 steps."""
+    L = 60.0
+    vd = pd.VectorDist(1, np.zeros(3), np.full(3, L), np.ones(3, np.int32), 2.5)
+    w = vd.getCellListGPU(2.5).view()
+    a = np.array(w.box_lo) + np.array(w.spacing) * 10  # corner of a cell in the middle
+    g = np.stack(np.meshgrid(np.arange(4), np.arange(4), np.arange(2), indexing="ij"), -1).reshape(-1, 3)
+    rest = a + 0.3 + g * [0.5, 0.5, 0.8]
+    rng = np.random.default_rng(7)
+    fly = a + [-20.0 * DT_FLY * (k - 0.5), 2.2, 2.2]
+    far = rng.uniform(0, L, size=(200, 3))
+    far = far[np.abs(far - a).max(1) > 6.0]
+    x = np.concatenate([rest, [fly], far])
+    v = np.concatenate([np.zeros((32, 3)), [[20.0, 0.0, 0.0]], rng.normal(size=far.shape) * 3])
+    return x, v, L
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("k", [1, 2, 4, 5])
+def test_bucket_overflow(pd, orc, dtype, k):
+    x, v, L = _crowding(pd, k)
+    x = x.astype(dtype).astype(F64)
+    bc, steps = np.ones(3, np.int32), 12
+    t = pd.PD_F64 if dtype == F64 else pd.PD_F32
+    runs = []
+    for parts in ([steps], [1] * steps):
+        vd = pd.VectorDist(len(x), np.zeros(3), np.full(3, L), bc, 2.5, dtype=dtype, props=[(t, 3), (t, 3), (pd.PD_I32, 1)])
+        vd.hostToDevicePos(x.astype(dtype))
+        vd.hostToDeviceProp(0, v)
+        vd.hostToDeviceProp(2, np.arange(len(x)))
+        md = pd.MD(vd, 0, 1, dt=DT_FLY, skin=0.0, sigma=0.1, use_cell_list=True)
+        E = np.concatenate([md.run(p) for p in parts])
+        runs.append((E,) + _by_id(vd))
+        assert md.bucket_steps() == k - 1
+    xo, vo, Eo = orc.md_lj(x, v, np.zeros(3), np.full(3, L), bc, 2.5, 2.5, 0.0, 1.0, 0.1, DT_FLY, 1.0, steps)
+    tol = 1e-9 if dtype == F64 else 1e-4
+    np.testing.assert_allclose(runs[0][0][:, :3], Eo[1:, :3], rtol=tol, atol=tol)
+    d = runs[0][1] - xo
+    assert np.abs(d - L * np.round(d / L)).max() < (1e-9 if dtype == F64 else 1e-3)
+    assert np.array_equal(runs[0][1], runs[1][1]) and np.array_equal(runs[0][2], runs[1][2])
+    np.testing.assert_allclose(runs[0][0], runs[1][0], rtol=1e-12 if dtype == F64 else 1e-5)
+    n = vd.size_local()
+    pos = vd.deviceToHostPos()
+    img, src, _ = orc.ghost_get(pos[:n], np.zeros(3, dtype), np.full(3, L, dtype), bc, 2.5)
+    assert np.array_equal(pos[n:], img)
+    assert np.array_equal(vd.deviceToHostProp(0)[n:], vd.deviceToHostProp(0)[:n][src])
