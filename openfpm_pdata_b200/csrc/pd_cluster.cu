@@ -780,8 +780,8 @@ static int cb_capacity(pd_md md) {
     return cap && 2.0 * (double)cl->ncells * cap * h->pos_bytes <= 96e6 ? cap : 0;
 }
 
-// steps made in buckets; *made < steps where a bucket overflowed or the GPU cannot place the launch
-template <class T> static int md_run_buckets_t(pd_md md, int steps, cudaStream_t st, int* made) {
+// steps made in buckets; *made < steps where a bucket overflowed (*over) or the GPU cannot place the launch
+template <class T> static int md_run_buckets_t(pd_md md, int steps, cudaStream_t st, int* made, bool* over) {
     typedef typename V4<T>::type T4;
     pd_vd h = md->h;
     pd_cl cl = md->cl;
@@ -881,7 +881,7 @@ template <class T> static int md_run_buckets_t(pd_md md, int steps, cudaStream_t
         return PD_EOVERFLOW;
     }
     *made = (int)h->ctrl_h->run_done;
-    if (*made < steps) md->bucket_off = true;  // too uneven: the one-cluster kernel from now on
+    *over = *made < steps;
     md->steps += *made;
     md->builds += *made;
     md->bucket_steps += *made;
@@ -895,6 +895,10 @@ bool md_cluster_eligible(pd_md md) {
            h->n_real <= CL_MAXN && md->cl->pad == 1 && md->cl->ncells <= 4L * CL_MAXN;
 }
 
+// Steps in buckets as long as they hold the particles.  After an overflow 32 steps on one
+// cluster, then buckets again; twice as many each time that the buckets did not last as long, so that a
+// system too uneven for them loses a launch in thousands of steps and one that was crowded for
+// a while returns to them.
 int md_run_cluster(pd_md md, int steps, cudaStream_t st, double* E) {
     if (!md->ready) {
         PD_TRY(md_rebuild(md, st));
@@ -903,19 +907,33 @@ int md_run_cluster(pd_md md, int steps, cudaStream_t st, double* E) {
         PD_TRY(read_ctrl(md->h, st));
         md->h->n_img = md->h->ctrl_h->n_img;
     }
-    if (steps == 0) return PD_OK;
     const bool f64 = md->h->dtype == PD_F64;
-    int made = 0;
-    if (!md->bucket_off && cb_capacity(md)) {
-        PD_TRY(f64 ? md_run_buckets_t<double>(md, steps, st, &made) : md_run_buckets_t<float>(md, steps, st, &made));
-        if (E && made > 0) {
-            PD_CUDA(cudaMemcpyAsync(E, md->E.p, sizeof(double) * 4 * made, cudaMemcpyDeviceToHost, st));
-            PD_CUDA(cudaStreamSynchronize(st));
+    bool buckets = cb_capacity(md) != 0;
+    for (int s = 0; s < steps;) {
+        double* Es = E ? E + 4 * (long)s : nullptr;
+        if (buckets && md->bucket_left == 0) {
+            int made = 0;
+            bool over = false;
+            PD_TRY(f64 ? md_run_buckets_t<double>(md, steps - s, st, &made, &over)
+                       : md_run_buckets_t<float>(md, steps - s, st, &made, &over));
+            if (E && made > 0) {
+                PD_CUDA(cudaMemcpyAsync(Es, md->E.p, sizeof(double) * 4 * made, cudaMemcpyDeviceToHost, st));
+                PD_CUDA(cudaStreamSynchronize(st));
+            }
+            s += made;
+            buckets = over || s == steps;  // else the GPU cannot place the launch
+            if (over) {
+                md->bucket_wait = made > md->bucket_wait ? 32 : std::min(2 * std::max(md->bucket_wait, 16L), 4096L);
+                md->bucket_left = md->bucket_wait;
+            }
+            continue;
         }
-        if (made == steps) return PD_OK;
-        if (E) E += 4 * (long)made;
+        const int part = buckets ? (int)std::min<long>(steps - s, md->bucket_left) : steps - s;
+        PD_TRY(f64 ? md_run_cluster_t<double>(md, part, st, Es) : md_run_cluster_t<float>(md, part, st, Es));
+        s += part;
+        if (buckets) md->bucket_left -= part;
     }
-    return f64 ? md_run_cluster_t<double>(md, steps - made, st, E) : md_run_cluster_t<float>(md, steps - made, st, E);
+    return PD_OK;
 }
 
 }  // namespace pd

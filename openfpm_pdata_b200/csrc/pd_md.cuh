@@ -58,7 +58,9 @@ struct pd_md_s {
     pd::Buf eidx;
     int cluster_ctas = 0;  // CTAs of a cluster of the last small cell-list run (0: none so far)
     pd::Buf buckets;          // cell-list mode of a small system: buckets, counts, partial sums
-    bool bucket_off = false;  // a bucket overflowed: an uneven system
+    // a bucket overflowed: steps still to be made on one cluster before the buckets are tried
+    // again, and how many that were the last time
+    long bucket_left = 0, bucket_wait = 0;
     long bucket_steps = 0;    // steps made by the bucket kernel
     // optional per-phase device timing (CUDA events on the run's stream)
     bool timing = false;

@@ -148,3 +148,22 @@ def test_bucket_overflow(pd, orc, dtype, k):
     img, src, _ = orc.ghost_get(pos[:n], np.zeros(3, dtype), np.full(3, L, dtype), bc, 2.5)
     assert np.array_equal(pos[n:], img)
     assert np.array_equal(vd.deviceToHostProp(0)[n:], vd.deviceToHostProp(0)[:n][src])
+
+
+def test_returns_to_buckets(pd, orc):
+    """The crowd disperses: after some steps on one cluster the buckets are tried again, while it lasts and
+    after, in a later run and within one."""
+    x, v, L = _crowding(pd, 4)
+    bc, steps = np.ones(3, np.int32), 230
+    xo, vo, Eo = orc.md_lj(x, v, np.zeros(3), np.full(3, L), bc, 2.5, 2.5, 0.0, 1.0, 0.1, DT_FLY, 1.0, steps)
+    for parts in ([steps], [10, 30, 90, 100]):
+        vd = pd.VectorDist(len(x), np.zeros(3), np.full(3, L), bc, 2.5, props=[(pd.PD_F64, 3), (pd.PD_F64, 3), (pd.PD_I32, 1)])
+        vd.hostToDevicePos(x)
+        vd.hostToDeviceProp(0, v)
+        vd.hostToDeviceProp(2, np.arange(len(x)))
+        md = pd.MD(vd, 0, 1, dt=DT_FLY, skin=0.0, sigma=0.1, use_cell_list=True)
+        E = np.concatenate([md.run(p) for p in parts])
+        assert 100 < md.bucket_steps() < steps - 32
+        np.testing.assert_allclose(E[:, :3], Eo[1:, :3], rtol=1e-9, atol=1e-9)
+        d = _by_id(vd)[0] - xo
+        assert np.abs(d - L * np.round(d / L)).max() < 1e-9
