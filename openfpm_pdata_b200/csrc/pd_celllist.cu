@@ -116,14 +116,14 @@ __global__ void __launch_bounds__(256) k_cl_stabilise(long ncells, const unsigne
 int cl_build(pd_vd h, pd_cl cl, long n_part, const unsigned int* n_part_dev, cudaStream_t st, long first) {
     // n_part: exact count, or (with n_part_dev) an upper bound; the device count is *n_part_dev + n_real
     long nc = cl->ncells;
-    PD_TRY(cl->cell_cnt.ensure(sizeof(unsigned int) * (nc + 2)));  // and a flag word for the list build
+    PD_TRY(cl->cell_cnt.ensure(sizeof(unsigned int) * (nc + 1)));
     PD_TRY(cl->cell_start.ensure(sizeof(unsigned int) * (nc + 1)));
     long nb = n_part > 0 ? n_part : 1;
     PD_TRY(cl->sorted.ensure(sizeof(int) * nb));
     PD_TRY(cl->sorted_tmp.ensure(sizeof(int) * nb));
     PD_TRY(cl->cell_of.ensure(sizeof(unsigned int) * nb));
     PD_TRY(cl->slot.ensure(sizeof(unsigned int) * nb));
-    PD_CUDA(cudaMemsetAsync(cl->cell_cnt.p, 0, sizeof(unsigned int) * (nc + 2), st));
+    PD_CUDA(cudaMemsetAsync(cl->cell_cnt.p, 0, sizeof(unsigned int) * (nc + 1), st));
     long n_add = n_part_dev ? h->n_real : 0;
     if (n_part > 0) {
         unsigned g = grid_for(n_part, 256);

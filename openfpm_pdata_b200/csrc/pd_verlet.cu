@@ -8,8 +8,8 @@
 //   2. FP32 copies of the positions are gathered into cell order with the original
 //      index in the record's 4th word;
 //   3. one CTA per tile of TX cells along x stages the 9 neighbour rows
-//      (x-1 .. x+TX for dy, dz in {-1,0,1}; each a contiguous range of the copies),
-//      three at a time, in shared memory and every thread scans the 27-cell
+//      (x-1 .. x+TX for dy, dz in {-1,0,1}; each a contiguous range of the copies) in
+//      shared memory, all at once or one z-layer at a time, and every thread scans the 27-cell
 //      neighbourhood of its particles from there, in the reference walk order (dz,
 //      dy, dx, in-cell order), writing column-major rows nbr[k*stride + i].
 // Rows longer than the capacity set ERR_NN_OVERFLOW and record the longest row;
@@ -44,23 +44,21 @@ static double verlet_bound(pd_cl cl) {
 }
 
 // p32[k] = FP32 copy of pos[sorted[k]] with the original index in w: what the row
-// kernel stages, half the bytes of an FP64 record.  *wide is set when a coordinate
-// exceeds `bound` (or is NaN): the FP32 band then does not hold and the row kernel
-// decides every candidate in the position type.
+// kernel stages, half the bytes of an FP64 record.  A coordinate beyond `bound`, the padded
+// grid, or a NaN is stored as infinity, which no test accepts: the particle lies in a padding
+// cell (clamped), so it has no row itself and is more than a cell side, the cutoff, away from
+// every particle that has one.
 template <class T>
 __global__ void k_gather_cs(const typename V4<T>::type* __restrict__ pos, const int* __restrict__ sorted,
-                            const unsigned int* __restrict__ cs_end, float4* __restrict__ out, long n_bound, T bound,
-                            unsigned int* __restrict__ wide) {
+                            const unsigned int* __restrict__ cs_end, float4* __restrict__ out, long n_bound, T bound) {
     long n = (long)*cs_end;
     if (n > n_bound) n = n_bound;
-    bool bad = false;
+    auto f32 = [&](T c) { return fabs(c) <= bound ? (float)c : INFINITY; };
     for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
         const int i = sorted[k];
         const typename V4<T>::type r = ld4(pos, i);
-        bad = bad || !(fabs(r.x) <= bound && fabs(r.y) <= bound && fabs(r.z) <= bound);
-        out[k] = make_float4((float)r.x, (float)r.y, (float)r.z, __int_as_float(i));
+        out[k] = make_float4(f32(r.x), f32(r.y), f32(r.z), __int_as_float(i));
     }
-    if (bad) atomicOr(wide, 1u);
 }
 
 template <class T4> __device__ __forceinline__ bool lex_after(const T4& a, const T4& b) {
@@ -133,20 +131,6 @@ __device__ __forceinline__ void verlet_seg(const float4* __restrict__ c4, unsign
     }
 }
 
-// the same with every candidate decided in the position type (coordinates beyond the FP32 band's range)
-template <class T, bool SYM>
-__device__ __noinline__ void verlet_seg_wide(const float4* __restrict__ c4, unsigned int n, int i,
-                                             const typename V4<T>::type* __restrict__ pos, T r2, long n_dom,
-                                             int* __restrict__ out, long stride, int max_nn, int& c) {
-    for (unsigned int k = 0; k < n; ++k) {
-        const int q = __float_as_int(c4[k].w);
-        if (!exact_in<T>(pos, (unsigned int)i, q, r2)) continue;
-        if (SYM && !sym_keep<T>(pos, i, q, n_dom)) continue;
-        if (c < max_nn) out[(long)c * stride] = q;
-        ++c;
-    }
-}
-
 // Rows of the domain particles of one tile (TX cells of a cell row), global original
 // indices, column-major nbr[k*stride + i], in the walk order dz, dy, dx, in-cell.
 // Bound by the instructions of the candidate tests (27 cells hold about 6.4 times
@@ -164,7 +148,7 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
                                                         const unsigned int* __restrict__ cs, long n_dom, T r2,
                                                         float lo_thr, float hi_thr, int* __restrict__ nbr,
                                                         int* __restrict__ nn, long stride, int max_nn,
-                                                        unsigned int pcap, const unsigned int* __restrict__ wide,
+                                                        unsigned int pcap,
                                                         unsigned int* __restrict__ ctrl_err,
                                                         unsigned int* __restrict__ ctrl_nnmax) {
     extern __shared__ __align__(128) unsigned char tile_raw[];
@@ -175,7 +159,6 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
     const unsigned int ib = S.cR[4][1], ie = S.cR[4][ncol - 2];
     if (ib == ie) return;
     if (threadIdx.x == 0) mbar_init(&S.bar, 1);
-    const bool exact_all = *wide != 0u;
     unsigned int ph = 0;
     bool held = false;  // the whole neighbourhood is staged
     // up to MAXI particles a thread and sweep; a denser tile takes further sweeps
@@ -202,7 +185,7 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
         for (int r0 = 0; r0 < 9; r0 += layers) {
             const unsigned int base = S.oR[r0];
             const unsigned int tot = (r0 + layers < 9 ? S.oR[r0 + layers] : S.total) - base;
-            const bool staged = tot <= pcap && !exact_all;
+            const bool staged = tot <= pcap;
             if (staged && tot > 0 && (layers < 9 || !held)) {
                 if (threadIdx.x < 32)
                     stage_ranges_warp(S, r0, layers, sm, base, p32, p32, tot * (unsigned int)sizeof(float4), &S.bar);
@@ -227,8 +210,6 @@ __global__ void __launch_bounds__(TBLOCK, 8) k_verlet_rows(const typename V4<T>:
                     if (staged)
                         verlet_seg<T, SYM>(sm + (S.oR[r] - base + (a - S.cR[r][0])), n, xi[m], i, pos, r2, lo_thr,
                                            hi_thr, n_dom, nbr + i, stride, max_nn, c);
-                    else if (exact_all)
-                        verlet_seg_wide<T, SYM>(p32 + a, n, i, pos, r2, n_dom, nbr + i, stride, max_nn, c);
                     else
                         verlet_seg<T, SYM>(p32 + a, n, xi[m], i, pos, r2, lo_thr, hi_thr, n_dom, nbr + i, stride,
                                            max_nn, c);
@@ -271,7 +252,7 @@ static int choose_tx(pd_cl cl, long n_all) {
 
 template <class T>
 static int verlet_rows(pd_vd h, pd_vl vl, const float4* p32, const TileGeom& tg, long ntiles, long n_dom, long stride,
-                       const unsigned int* wide, cudaStream_t st) {
+                       cudaStream_t st) {
     typedef typename V4<T>::type T4;
     pd_cl cl = vl->cl;
     // staging: 1536 records (24 KB, eight CTAs per SM)
@@ -285,7 +266,7 @@ static int verlet_rows(pd_vd h, pd_vl vl, const float4* p32, const TileGeom& tg,
     auto go = [&](auto k) {
         pd::launch(k, (unsigned)ntiles, TBLOCK, pcap * sizeof(float4), st, (const T4*)h->pos, p32, tg,
                    (const unsigned int*)cl->cell_start.as<unsigned int>(), n_dom, r2, lo_thr, hi_thr, vl->nbr.as<int>(),
-                   vl->nn.as<int>(), stride, vl->max_nn, pcap, wide, &h->ctrl->err, &h->ctrl->nn_max);
+                   vl->nn.as<int>(), stride, vl->max_nn, pcap, &h->ctrl->err, &h->ctrl->nn_max);
     };
     if (vl->sym) go(k_verlet_rows<T, true>);
     else go(k_verlet_rows<T, false>);
@@ -300,18 +281,16 @@ int verlet_build(pd_vd h, pd_vl vl, long n_dom, const unsigned int* n_img_dev, c
     pd_cl cl = vl->cl;
     long n_all_bound = n_img_dev ? h->cap : h->n_total;
     PD_TRY(cl_build(h, cl, n_all_bound, n_img_dev, st));
-    // cell-ordered FP32 copies with original indices; the flag word of out-of-range
-    // coordinates lies behind the cell counts, which cl_build cleared
+    // cell-ordered FP32 copies with original indices
     PD_TRY(h->tmp.ensure((size_t)(n_all_bound > 0 ? n_all_bound : 1) * sizeof(float4)));
     const unsigned int* cs_end = cl->cell_start.as<unsigned int>() + cl->ncells;
-    unsigned int* wide = cl->cell_cnt.as<unsigned int>() + cl->ncells + 1;
     unsigned g = grid_for(n_all_bound, 256);
     if (h->dtype == PD_F64)
         pd::launch(k_gather_cs<double>, g, 256, 0, st, (const double4*)h->pos, cl->sorted.as<int>(), cs_end,
-                                               h->tmp.as<float4>(), n_all_bound, verlet_bound(cl), wide);
-    else  // staged as they are: nothing is out of range
+                                               h->tmp.as<float4>(), n_all_bound, verlet_bound(cl));
+    else  // staged as they are
         pd::launch(k_gather_cs<float>, g, 256, 0, st, (const float4*)h->pos, cl->sorted.as<int>(), cs_end,
-                                              h->tmp.as<float4>(), n_all_bound, INFINITY, wide);
+                                              h->tmp.as<float4>(), n_all_bound, INFINITY);
     PD_LAUNCH_CHECK();
     long stride = ((n_dom + 31) / 32) * 32;
     if (stride < 32) stride = 32;
@@ -334,8 +313,8 @@ int verlet_build(pd_vd h, pd_vl vl, long n_dom, const unsigned int* n_img_dev, c
             TileGeom tg;
             long ntiles = 0;
             PD_TRY(tile_plan(cl, n_dom, choose_tx(cl, h->n_total > 0 ? h->n_total : h->n_real), tg, ntiles));
-            if (h->dtype == PD_F64) PD_TRY(verlet_rows<double>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, wide, st));
-            else PD_TRY(verlet_rows<float>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, wide, st));
+            if (h->dtype == PD_F64) PD_TRY(verlet_rows<double>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, st));
+            else PD_TRY(verlet_rows<float>(h, vl, h->tmp.as<float4>(), tg, ntiles, n_dom, stride, st));
         }
         if (!check) return PD_OK;
         PD_TRY(read_ctrl(h, st));

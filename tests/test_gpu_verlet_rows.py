@@ -95,3 +95,37 @@ def test_pairs_at_the_cutoff(pd, orc, dtype):
     got_off, got = vd.getVerlet(r).get()
     assert np.array_equal(got_off, off)
     assert np.array_equal(got, idx)
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+@pytest.mark.parametrize("sym", [False, True])
+def test_particles_outside_the_grid(pd, dtype, sym):
+    """Beyond the padding by a little and by far, close to each other there, infinite, not a
+    number of either sign: no row and in no row; all others keep theirs."""
+    rng = np.random.default_rng(6)
+    n, L, r = 2500, 8.0, 1.0
+    x = rng.uniform(0, L, size=(n, 3)).astype(dtype)
+    out = {3: (9.6, 4, 4), 4: (9.7, 4, 4), 7: (1e9, 2, 2), 8: (1e9, 2, 2), 9: (-2.5, -2.5, 4), 10: (np.inf, 1, 1),
+           11: (1, -np.inf, 1), 12: (np.nan, 7.5, 7.5), 13: (0.2, 0.2, -np.nan), 14: (np.nan, np.nan, np.nan),
+           15: (0.1, 0.1, 1e300 if dtype == F64 else 1e38), 16: (0.5, -9.0, 0.5)}
+    for i, p in out.items():
+        x[i] = p
+    x[100:140] = rng.uniform(0, 0.6, size=(40, 3))  # near the border cells that they are clamped into
+    x[140:180] = L - rng.uniform(0, 0.6, size=(40, 3))
+    vd = pd.VectorDist(n, np.zeros(3), np.full(3, L), np.zeros(3, np.int32), 0.0, dtype=dtype)
+    vd.hostToDevicePos(x)
+    off, idx = (vd.getVerletSym(r) if sym else vd.getVerlet(r)).get()
+    ok = np.ones(n, bool)
+    ok[list(out)] = False
+    for i in range(n):
+        row = np.zeros(n, bool)
+        row[idx[off[i]:off[i + 1]]] = True
+        if not ok[i]:
+            assert not row.any()
+            continue
+        d = ((x.astype(F64) - x[i].astype(F64)) ** 2).sum(1)
+        want = ok & (np.where(ok, d, 9.0) < r * r)
+        if sym:
+            want &= np.arange(n) > i
+        sure = ~ok | (np.abs(d - r * r) > 1e-5)
+        assert np.array_equal(row[sure], want[sure])
