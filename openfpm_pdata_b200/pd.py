@@ -402,15 +402,14 @@ class VectorDist:
 
     def deviceToHostPos(self, offset=0, count=None, with_ghost=True, out=None, device=False):
         """positions [n][3]; `out` (e.g. pinned memory) receives them when given;
-        device=True returns a CUDA tensor (copied on the GPU)"""
+        device=True returns a CUDA tensor (copied on the GPU, complete on return)"""
         n = (self.size_local_with_ghost() if with_ghost else self.size_local()) - offset if count is None else count
         if device:
             import torch
             t = torch.empty((max(n, 0), 3), dtype=torch.float64 if self.dtype == np.float64 else torch.float32,
                             device="cuda")
             if n:
-                check(lib().pd_d2h_pos_rows(self.h, ctypes.c_void_p(t.data_ptr()), int(offset), int(n), None))
-                _finish_on_side_stream(torch)
+                check(lib().pd_d2h_pos(self.h, ctypes.c_void_p(t.data_ptr()), int(offset), int(n), None))
             return t
         if out is None:
             out = np.zeros((n, 3), self.dtype)

@@ -197,3 +197,20 @@ def test_device_arrays(pd, dtype, n):
         assert torch.equal(vd.deviceToHostProp(0, offset=2, count=9, device=True),
                            torch.cat([v[2:3], v[:7] * 2, v[10:11]]))
         assert torch.equal(vd.deviceToHostPos(offset=5, count=11, device=True), x[5:16])
+
+
+def test_positions_complete_on_return(pd):
+    """deviceToHostPos(device=True) returns when the positions are there: another stream may
+    read the tensor at once, although the device was busy at the call."""
+    import torch
+    n = 5000
+    x = np.random.default_rng(2).random((n, 3))
+    vd = pd.VectorDist(n, np.zeros(3), np.ones(3), np.ones(3, np.int32), 0.1)
+    vd.hostToDevicePos(x)
+    side = torch.cuda.Stream()
+    torch.cuda._sleep(1 << 27)  # about 70 ms of the default stream
+    t = vd.deviceToHostPos(device=True)
+    assert torch.cuda.default_stream().query()
+    with torch.cuda.stream(side):
+        got = t.cpu()
+    assert np.array_equal(got.numpy(), x)
