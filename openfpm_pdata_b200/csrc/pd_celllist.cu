@@ -228,16 +228,32 @@ template <int MODE> __global__ void k_move_cols(const int* __restrict__ ids, lon
 // Permutation in place (the storage keeps its addresses): up to GCOLS columns move into
 // scratch in one kernel and back in another.  A kernel and a copy for each column were
 // bound by their launches on small systems: 4,099 FP64 particles, reorder and
-// restoreOrder of four columns together 41 us of GPU time in 20 launches.
+// restoreOrder of four columns together 41 us of GPU time in 20 launches.  The columns of a
+// pair of launches take no more scratch than PERM_SCRATCH or the largest column: what is
+// gathered at random then stays in L2 with where it goes, and a large system needs no more memory
+// than one column after the other took.  Update with reorder and restoreOrder, us, by 8 / 32 / 64 MB
+// / all columns at once: 700,001 FP32 particles 219 / 169 / 168 / 170, 250,000 FP64 145 / 115 / 114 /
+// 112, 2,000,000 510 / 481 / 496 / 623, 4,000,000 898 / 898 / 940 / 1,546.
+static constexpr size_t PERM_SCRATCH = (size_t)32 << 20;
 int permute_columns(pd_vd h, const MoveCol* cols, int ncols, const int* ids, long n, bool restore, cudaStream_t st) {
     if (n <= 0) return PD_OK;
     const unsigned g = grid_for(n, 256);
     auto room = [&](int c) { return ((size_t)n * cols[c].esize + 255) & ~(size_t)255; };  // aligned scratch columns
-    for (int c0 = 0; c0 < ncols; c0 += GCOLS) {
-        const int c1 = std::min(ncols, c0 + GCOLS);
-        size_t bytes = 0;
-        for (int c = c0; c < c1; ++c) bytes += room(c);
-        PD_TRY(h->tmp2.ensure(bytes));
+    // the columns [c0, end) that move together, and their scratch
+    auto batch = [&](int c0, size_t* bytes) {
+        int c = c0;
+        for (*bytes = 0; c < ncols && c < c0 + GCOLS && (c == c0 || *bytes + room(c) <= PERM_SCRATCH); ++c)
+            *bytes += room(c);
+        return c;
+    };
+    size_t most = 0, bytes;
+    for (int c = 0; c < ncols;) {
+        c = batch(c, &bytes);
+        most = std::max(most, bytes);
+    }
+    PD_TRY(h->tmp2.ensure(most));
+    for (int c0 = 0, c1; c0 < ncols; c0 = c1) {
+        c1 = batch(c0, &bytes);
         GatherCols out{}, back{};
         out.ncol = back.ncol = c1 - c0;
         char* t = h->tmp2.as<char>();

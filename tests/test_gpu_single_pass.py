@@ -214,3 +214,37 @@ def test_positions_complete_on_return(pd):
     with torch.cuda.stream(side):
         got = t.cpu()
     assert np.array_equal(got.numpy(), x)
+
+
+def test_reorder_scratch(pd):
+    """A reorder of a large vector takes scratch for its largest column, not for all of them."""
+    import ctypes
+    import torch
+    n = 8000003
+
+    def free():
+        torch.cuda.synchronize()
+        f = ctypes.c_long(0)
+        assert pd.lib().pd_device_info(None, ctypes.byref(f), None) == 0
+        return f.value
+
+    vd = pd.VectorDist(n, np.zeros(3), np.ones(3), np.zeros(3, np.int32), 0.0, props=[(pd.PD_F64, 7), (pd.PD_F32, 2)])
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.rand((n, 3), device="cuda", dtype=torch.float64, generator=gen)
+    p = torch.rand((n, 7), device="cuda", dtype=torch.float64, generator=gen)
+    vd.hostToDevicePos(x)
+    vd.hostToDeviceProp(0, p)
+    cl = vd.getCellListGPU(0.01, opt=pd.CL_NON_SYMMETRIC)
+    vd.updateCellListGPU(cl)  # the sort's own buffers
+    cr = vd.getCellListGPU(0.01, opt=pd.CL_NON_SYMMETRIC | pd.CL_GPU_REORDER)
+    pd.lib().pd_empty_cache()
+    before = free()
+    vd.updateCellListGPU(cr)
+    sort = 5 * 4 * n + 3 * 4 * cr.view().ncells
+    assert before - free() < sort + 32 * n + (64 << 20)
+    so = torch.from_numpy(cr.get()[1].astype(np.int64)).cuda()
+    assert torch.equal(vd.deviceToHostPos(device=True), x[so])
+    assert torch.equal(vd.deviceToHostProp(0, device=True), p[so])
+    vd.restoreOrder(cr)
+    assert torch.equal(vd.deviceToHostPos(device=True), x)
+    assert torch.equal(vd.deviceToHostProp(0, device=True), p)
