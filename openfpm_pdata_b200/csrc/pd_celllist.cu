@@ -403,13 +403,14 @@ __global__ void __launch_bounds__(128) k_test_force(const typename V4<T>::type* 
                         const T rx = xq.x - xp.x, ry = xq.y - xp.y, rz = xq.z - xp.z;
                         const T r2 = rx * rx + ry * ry + rz * rz;
                         // too close (the particle itself among them) or not a distance (NaN): no
-                        // contribution.  The direction first: w / r overflows for large weights
+                        // contribution.  The direction first: w / r overflows for large weights.
+                        // The sum is selected, not the term (FP64, 16 lanes: 10.4 us, a branch 12.8)
                         const T y = rsqrt_series(r2);
-                        if (r2 > min2) {
-                            fx += wq * (rx * y);
-                            fy += wq * (ry * y);
-                            fz += wq * (rz * y);
-                        }
+                        const bool far = r2 > min2;
+                        const T tx = fma(wq, rx * y, fx), ty = fma(wq, ry * y, fy), tz = fma(wq, rz * y, fz);
+                        fx = far ? tx : fx;
+                        fy = far ? ty : fy;
+                        fz = far ? tz : fz;
                     }
                 }
             }

@@ -83,7 +83,7 @@ __device__ __forceinline__ double rsqrt_series(double x) {
 __device__ __forceinline__ float rsqrt_series(float x) {
     float y;
     asm("rsqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float e = x <= 3.402823466e38f ? fmaf(-x * y, y, 1.0f) : 0.0f;
+    const float e = fmaf(-fminf(x, 3.402823466e38f) * y, y, 1.0f);
     return fmaf(0.5f * y, e, y);
 }
 
