@@ -196,14 +196,14 @@ void Buf::release() {
 
 // ---------------------------------------------------------------------------
 // Exclusive scan in tiles of 4096 elements, n up to 2^31; no CTA waits for another.  Up to
-// SCAN_DIRECT tiles one launch, in which each CTA also adds up the elements before its tile (a few
-// 16-byte loads a thread: 4.2 us for 4 tiles, 6.4 for 16, 10.3 for 32, against 7.3, 8.3 and 8.3
-// with the tiles' sums from a launch of their own); more tiles in two launches, very many in
-// three (see PREFIX_TILES).
-static constexpr int SCAN_BLOCK = 512;
-static constexpr int SCAN_ITEMS = 8;
+// SCAN_DIRECT tiles one launch, in which each CTA also adds up the elements before its tile (one
+// 16-byte load a thread and tile: 4.9 us for 5 tiles, 6.2 for 22, 8.2 for 49, 10.3 for 64,
+// against 7.3, 8.3, 8.3 and 8.3 with the tiles' sums from a launch of their own, which also costs
+// the gap between the two); more tiles in two launches, very many in three (see PREFIX_TILES).
+static constexpr int SCAN_BLOCK = 1024;
+static constexpr int SCAN_ITEMS = 4;
 static constexpr int SCAN_TILE = SCAN_BLOCK * SCAN_ITEMS;
-static constexpr long SCAN_DIRECT = 16;
+static constexpr long SCAN_DIRECT = 48;
 
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_sums(const unsigned int* __restrict__ in, long n,
                                                           unsigned int* __restrict__ part) {
@@ -261,13 +261,14 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan(const unsigned int* in, lon
     __shared__ unsigned int wsum[SCAN_BLOCK / 32];
     const unsigned int tile = blockIdx.x;
     // each thread owns SCAN_ITEMS consecutive elements
+    static_assert(SCAN_ITEMS == 4, "one 16-byte access");
     const long i0 = (long)tile * SCAN_TILE + (long)threadIdx.x * SCAN_ITEMS;
     const bool al = (((size_t)in | (size_t)out) & 15) == 0;  // 16-byte accesses allowed
     const bool vec = al && i0 + SCAN_ITEMS <= n;
     unsigned int v[SCAN_ITEMS];
     if (vec) {
-        const uint4 a = reinterpret_cast<const uint4*>(in + i0)[0], b = reinterpret_cast<const uint4*>(in + i0)[1];
-        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+        const uint4 a = reinterpret_cast<const uint4*>(in + i0)[0];
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
     } else {
 #pragma unroll
         for (int k = 0; k < SCAN_ITEMS; ++k) v[k] = (i0 + k < n) ? in[i0 + k] : 0u;
@@ -326,7 +327,6 @@ __global__ void __launch_bounds__(SCAN_BLOCK) k_scan(const unsigned int* in, lon
     }
     if (vec) {
         reinterpret_cast<uint4*>(out + i0)[0] = make_uint4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<uint4*>(out + i0)[1] = make_uint4(v[4], v[5], v[6], v[7]);
     } else {
 #pragma unroll
         for (int k = 0; k < SCAN_ITEMS; ++k)

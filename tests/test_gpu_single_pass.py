@@ -17,11 +17,11 @@ def pd():
 
 
 @pytest.mark.parametrize("gs", [(3, 4, 5), (11, 12, 31), (13, 15, 21), (16, 16, 16), (15, 17, 257), (32, 32, 64),
-                                (128, 128, 257), (31, 601, 1801), (256, 256, 512)])
+                                (45, 17, 257), (64, 64, 48), (128, 128, 257), (31, 601, 1801), (256, 256, 512)])
 def test_cell_starts(pd, gs):
     """Cell starts are the exclusive scan of the counts: cells + 1 elements, 4093, 4096 and 4097
-    among them (one tile, two), 65536 and 65537 (the last size that one launch scans), 33554432
-    and 33554433 (the last whose tiles each add up the ones before).  Twice in a row."""
+    among them (one tile, two), 65536 and 65537, 196606 and 196609 (the last tiles that one launch
+    scans), 33554432 and 33554433 (the last that each add up the ones before).  Twice in a row."""
     rng = np.random.default_rng(sum(gs))
     L = np.array(gs) - 2.5
     n = 20011
