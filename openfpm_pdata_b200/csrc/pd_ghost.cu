@@ -422,8 +422,10 @@ int ghost_generate(pd_vd h, long img_cap, bool sync_count, cudaStream_t st) {
     if (!sync_count) return ghost_make(h, img_cap, st);
     const long n = h->n_real;
     const bool none = n <= 0 || h->nbox == 0;  // no image whatever the positions: nothing to read back
-    const long room = none ? 0 : ghost_room(h);
-    if (!none) PD_TRY(ensure_capacity(h, n + room + 1, st));
+    long room = none ? 0 : ghost_room(h);
+    // no memory for the estimate (particles that keep away from the faces may need far less): what
+    // there is, which finds the count
+    if (!none && ensure_capacity(h, n + room + 1, st) != PD_OK) room = std::max(h->cap - n - 1, 0L);
     PD_TRY(ghost_make(h, room, st));
     if (none) h->ctrl_h->n_img = 0;
     else PD_TRY(read_ctrl(h, st));

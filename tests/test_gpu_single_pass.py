@@ -248,3 +248,29 @@ def test_reorder_scratch(pd):
     vd.restoreOrder(cr)
     assert torch.equal(vd.deviceToHostPos(device=True), x)
     assert torch.equal(vd.deviceToHostProp(0, device=True), p)
+
+
+def test_ghost_get_near_the_memory_limit(pd):
+    """The room made for images before the first count is an estimate: where memory does not
+    suffice for it, particles that have no image need none."""
+    import torch
+    n = 400000
+    lo, hi, bc = np.zeros(3), np.ones(3), np.ones(3, np.int32)
+    vd = pd.VectorDist(n, lo, hi, bc, 0.49, props=[(pd.PD_F64, 64), (pd.PD_F64, 64)])
+    x = 0.5 + (np.random.default_rng(4).random((n, 3)) - 0.5) * 0.01
+    x[:5] = 0.1
+    vd.hostToDevicePos(x)
+    pd.lib().pd_empty_cache()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    block = torch.empty(free - (3 << 30), dtype=torch.uint8, device="cuda")  # 4.5 GB were wanted
+    try:
+        vd.ghost_get([])
+        vd.ghost_get([])
+    finally:
+        del block
+        torch.cuda.empty_cache()
+    assert vd.size_local_with_ghost() == n + 5 * 7
+    got = vd.deviceToHostPos()
+    assert np.array_equal(got[:n], x)
+    assert np.array_equal(np.unique(got[n:].round(6)), [0.1, 1.1])
