@@ -356,6 +356,8 @@ int pd_lj_forces(pd_vd h, pd_vl vl, pd_cl cl, const pd_lj_params_t* lj, int forc
 /* the reciprocal used by the pair kernels (Newton-Raphson on the hardware
  * approximation), evaluated on n host values -- a self-test of its error bound */
 int pd_selftest_recip(int dtype, const void* x_host, void* out_host, long n);
+/* the neighbour functor's reciprocal square root of n host values (self test) */
+int pd_selftest_rsqrt(int dtype, const void* x_host, void* out_host, long n);
 
 /* ---- velocity-Verlet LJ driver ------------------------------------------ */
 /* Binds a vector holding real particles (no ghost) to an integrator that keeps

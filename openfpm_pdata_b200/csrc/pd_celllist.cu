@@ -429,6 +429,11 @@ __global__ void __launch_bounds__(128) k_test_force(const typename V4<T>::type* 
     }
 }
 
+template <class T> __global__ void k_rsqrt_check(const T* __restrict__ x, T* __restrict__ y, long n) {
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+        y[i] = rsqrt_series(x[i]);
+}
+
 // the largest x with sqrt(x) <= d
 template <class T> static T below_distance(T d) {
     T m = d * d;
@@ -520,6 +525,27 @@ int pd_celllist_update(pd_vd h, pd_cl cl, unsigned long prop_mask, void* stream)
         set_error("cell list: particles outside the cell grid (clamped to the border cells)");
         h->ctrl_h->err = 0;
     }
+    return PD_OK;
+}
+
+int pd_selftest_rsqrt(int dtype, const void* x_host, void* out_host, long n) {
+    if ((dtype != PD_F32 && dtype != PD_F64) || !x_host || !out_host || n < 0) return PD_EINVAL;
+    if (n == 0) return PD_OK;
+    const size_t es = dtype == PD_F64 ? 8 : 4;
+    Buf a;
+    PD_TRY(a.ensure(2 * es * n));
+    char* y = a.as<char>() + es * n;
+    cudaError_t e = cudaMemcpy(a.p, x_host, es * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        if (dtype == PD_F64)
+            pd::launch(k_rsqrt_check<double>, grid_for(n, 256), 256, 0, (cudaStream_t)0, a.as<const double>(), (double*)y, n);
+        else
+            pd::launch(k_rsqrt_check<float>, grid_for(n, 256), 256, 0, (cudaStream_t)0, a.as<const float>(), (float*)y, n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out_host, y, es * n, cudaMemcpyDeviceToHost);
+    a.release();
+    PD_CUDA(e);
     return PD_OK;
 }
 

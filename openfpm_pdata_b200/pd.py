@@ -188,6 +188,7 @@ def lib():
             "pd_gen_clustered": ([lp, ctypes.c_double, ip, ctypes.c_double, ctypes.c_double, ctypes.c_ulong, ip, vp,
                                   P(ctypes.c_long)], ip),
             "pd_selftest_recip": ([ip, vp, vp, lp], ip),
+            "pd_selftest_rsqrt": ([ip, vp, vp, lp], ip),
             "pd_md_verlet_get": ([vp, vp, vp, lp, P(ctypes.c_int)], ip),
         }
         for name, (args, res) in sig.items():
@@ -271,6 +272,15 @@ def selftest_recip(x):
     code = PD_F64 if x.dtype == np.float64 else PD_F32
     out = np.zeros_like(x)
     check(lib().pd_selftest_recip(code, _ptr(x), _ptr(out), int(x.size)))
+    return out
+
+
+def selftest_rsqrt(x):
+    """The neighbour functor's reciprocal square root evaluated on the GPU for the values x."""
+    x = np.ascontiguousarray(x)
+    code = PD_F64 if x.dtype == np.float64 else PD_F32
+    out = np.zeros_like(x)
+    check(lib().pd_selftest_rsqrt(code, _ptr(x), _ptr(out), int(x.size)))
     return out
 
 
