@@ -807,8 +807,7 @@ static std::vector<uintptr_t> cl_graph_key(pd_md md) {
                                 (uintptr_t)cl->cell_cnt.p, (uintptr_t)cl->sorted.p, (uintptr_t)cl->sorted_tmp.p,
                                 (uintptr_t)cl->cell_of.p, (uintptr_t)cl->slot.p, (uintptr_t)h->tmp.p,
                                 (uintptr_t)h->tmp2.p, (uintptr_t)h->img_src.p, (uintptr_t)h->img_shift.p,
-                                (uintptr_t)h->img_cnt.p, (uintptr_t)h->img_start.p, (uintptr_t)h->boxes.p,
-                                (uintptr_t)h->shifts.p, (uintptr_t)h->scan_scratch.p, (uintptr_t)h->tile_cnt.p,
+                                (uintptr_t)h->boxes.p, (uintptr_t)h->shifts.p, (uintptr_t)h->scan_scratch.p, (uintptr_t)h->tile_cnt.p,
                                 (uintptr_t)h->img_list.p, (uintptr_t)md->gcl_img_cap};
     for (auto& P : h->props) k.push_back((uintptr_t)P.d);
     return k;

@@ -215,9 +215,9 @@ def test_md_spare_storage_across_storage_changes(pd):
 
 
 def test_md_launch_shape(pd):
-    """The driver reports the shapes its kernels ran with: the one-cluster step of
-    a small cell-list system (16 CTAs, or 8 where 16 cannot be placed) and the
-    tile width of the tiled rows."""
+    """The driver reports the shapes its kernels ran with: the CTAs of a cluster of a
+    small cell-list system's steps (8; 16 on one cluster where the GPU can place it) and
+    the tile width of the tiled rows."""
     from openfpm_pdata_b200 import workloads
     x, v, L = workloads.lj_lattice(16, 1.0, 0.05, seed=1)
     lo, hi, bc = np.zeros(3), np.full(3, L), np.ones(3, np.int32)

@@ -2,7 +2,8 @@
 of few cells, open boundaries, FP32 storage, a dense corner of an empty box.  A run equals
 runs of one step and a second identical run bit for bit (the order in which buckets fill does
 not matter).  The one-cluster kernel that it hands over to where a bucket overflows: from the
-first step, after an odd and after an even number of steps."""
+first step, after an odd and after an even number of steps; and by itself in a box of too many
+cells for buckets."""
 import numpy as np
 import pytest
 
@@ -167,3 +168,23 @@ def test_returns_to_buckets(pd, orc):
         np.testing.assert_allclose(E[:, :3], Eo[1:, :3], rtol=1e-9, atol=1e-9)
         d = _by_id(vd)[0] - xo
         assert np.abs(d - L * np.round(d / L)).max() < 1e-9
+
+
+@pytest.mark.parametrize("dtype", [F32, F64])
+def test_one_cluster_from_the_start(pd, orc, dtype):
+    """A dense corner of a wide, empty box: two sets of buckets for all its cells would not stay in L2."""
+    x, v, _ = _system("clump")
+    L, steps = 130.0, 25
+    x = x.astype(dtype).astype(F64)
+    lo, hi, bc = np.zeros(3), np.full(3, L), np.ones(3, np.int32)
+    runs = []
+    for parts in ([steps], [1] * steps):
+        vd, md = _md(pd, x, v, L, bc, dtype)
+        runs.append((np.concatenate([md.run(k) for k in parts]),) + _by_id(vd))
+        assert md.bucket_steps() == 0 and md.launch_shape()["cluster_ctas"] in (8, 16)
+    assert all(np.array_equal(a, b) for a, b in zip(*runs))
+    xo, vo, Eo = orc.md_lj(x, v, lo, hi, bc, 2.5, 2.5, 0.0, 1.0, 1.0, 0.002, 1.0, steps)
+    f64 = dtype == F64
+    np.testing.assert_allclose(runs[0][0][:, :3], Eo[1:, :3], rtol=1e-9 if f64 else 1e-3, atol=1e-9 if f64 else 1e-2)
+    d = runs[0][1] - xo
+    assert np.abs(d - L * np.round(d / L)).max() < (1e-9 if f64 else 1e-3)

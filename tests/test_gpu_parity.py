@@ -391,9 +391,10 @@ def test_md_tiled_equals_global_rows(pd):
 
 
 def test_md_cell_list_both_paths(pd, orc):
-    """Cell list every step: a small system runs in one thread-block cluster, a system
+    """Cell list every step: a small system runs in one launch of the bucket kernel, a system
     above 65,536 particles through the captured step graph; both follow the FP64
-    oracle (per-step energies within 1e-9, positions within 1e-8)."""
+    oracle (per-step energies within 1e-9, positions within 1e-8).  The one-cluster kernel
+    between the two: test_gpu_cell_steps.py."""
     from openfpm_pdata_b200 import workloads
     for side, steps in ((12, 30), (42, 6)):
         x, v, L = workloads.lj_lattice(side, 1.1, 0.05, seed=11)
