@@ -59,3 +59,37 @@ def test_limit_bounds_the_cache(pd):
     finally:
         pd.set_cache_limit(4 << 30)
         pd.empty_cache()
+
+
+def test_full_cache_takes_new_blocks(pd):
+    """Blocks of an earlier size that fill the cache make room once nothing asks for them, so that
+    vectors of another size, made and dropped in turn, find their blocks again; blocks in use in
+    turn stay although the last of them does not fit."""
+    def vec(n):
+        return pd.VectorDist(n, np.zeros(3), np.ones(3), np.ones(3, np.int32), 0.1, props=[(pd.PD_F64, 3)])
+
+    try:
+        pd.empty_cache()
+        pd.set_cache_limit(200 << 20)
+        a = [vec(400000) for _ in range(5)]  # 30 MB each, then kept
+        del a
+        old = pd.set_cache_limit()
+        assert (130 << 20) < old <= (200 << 20)
+        for _ in range(60):  # 3 blocks, 150 MB: too many beside the old ones
+            del_me = vec(2000000)
+            del del_me
+        full = pd.set_cache_limit()
+        b = vec(2000000)
+        assert full - pd.set_cache_limit() > (130 << 20)  # all of b's blocks were kept ones
+        assert full <= (200 << 20)
+        del b
+        # 300 MB in turn, 200 kept: the kept ones are found in every turn
+        for k in range(12):
+            before = pd.set_cache_limit()
+            c = [vec(2000000), vec(2100000)]
+            took = before - pd.set_cache_limit()
+            assert k == 0 or took > (90 << 20)
+            del c
+    finally:
+        pd.set_cache_limit(4 << 30)
+        pd.empty_cache()
