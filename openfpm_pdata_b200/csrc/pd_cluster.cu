@@ -506,10 +506,10 @@ __device__ __forceinline__ float4 ldcg4(const float4* p) { return __ldcg(p); }
 // a wait has given up.
 __device__ __forceinline__ bool grid_barrier(cg::cluster_group& cl, unsigned int* bar, unsigned int target,
                                              unsigned int* err) {
-    __threadfence();
     cl.sync();
     if (cl.block_rank() == 0 && threadIdx.x == 0) {
-        __threadfence();  // the arrival releases what the cluster's other threads wrote before cl.sync()
+        // the cluster's writes before cl.sync() are this thread's to release (cumulativity): one fence
+        __threadfence();
         atomicAdd(bar, 1u);
         unsigned int seen = 0, it = 0;
         do {
