@@ -10,6 +10,7 @@
 // images [n_real, n_total).
 #include <algorithm>
 #include <cstdarg>
+#include <iterator>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -67,11 +68,12 @@ thread_local AllocCtx* g_alloc_ctx = nullptr;
 // is reused without a device-wide synchronisation).  Elsewhere from cudaMalloc
 // through a bounded block cache: a freed block is kept (up to the cache limit,
 // 4 GiB by default) and handed out again for a request of 1/2 to 1 times its size.  Where
-// the limit is reached, blocks that nothing has asked for in the last STALE frees make room; else
-// the block just freed returns to the driver.  (A process that had filled the cache with blocks of
-// other sizes otherwise paid a cudaMalloc and a cudaFree for each block of a new driver, every
-// time: a dam break of 1.9 million particles, its driver made and dropped each run, 14 to 30 ms
-// a run instead of 13.0.  Blocks in use in turn, more than the limit of them, stay.)
+// the limit is reached kept blocks make room for the one just freed, each time the older of
+// two picked at random: blocks that nothing asks for leave soon, and of sizes in use in turn,
+// more than the limit of them, some stay.  (With the block just freed returned instead, a process that
+// had filled the cache with blocks of other sizes paid a cudaMalloc and a cudaFree for each block
+// of a new driver, every time: a dam break of 1.9 million particles, its driver made and dropped
+// each run, 14 to 30 ms a run instead of 13.0.)
 // cudaFree synchronises the device; the cache keeps that guarantee by
 // synchronising once before a block freed since the last synchronisation is
 // reused, so no kernel of the block's previous owner can still be running.
@@ -93,7 +95,7 @@ struct BlockCache {
     std::mutex mu;
     std::multimap<std::pair<int, size_t>, Kept> free_blocks;  // by (device, size)
     unsigned long long frees = 0;
-    static constexpr unsigned long long STALE = 128;
+    unsigned long long rng = 1;
     std::unordered_map<void*, Block> block_of;                 // every block from cudaMalloc on this path
     size_t held = 0;
     size_t limit = (size_t)4 << 30;
@@ -119,13 +121,16 @@ struct BlockCache {
         held = 0;
         dirty.clear();
     }
-    // room for `bytes` more, from the blocks kept the longest (caller holds mu); false: none
+    // room for `bytes` more (caller holds mu); false: more than the limit
     bool make_room(size_t bytes) {
+        if (bytes > limit) return false;
+        auto pick = [&] {
+            rng = rng * 6364136223846793005ull + 1442695040888963407ull;
+            return std::next(free_blocks.begin(), (long)((rng >> 33) % free_blocks.size()));
+        };
         while (held + bytes > limit) {
-            auto old = free_blocks.begin();
-            for (auto it = old; it != free_blocks.end(); ++it)
-                if (it->second.seq < old->second.seq) old = it;
-            if (old == free_blocks.end() || frees - old->second.seq < STALE) return false;
+            const auto a = pick(), b = pick();
+            const auto old = a->second.seq < b->second.seq ? a : b;
             held -= old->first.second;
             block_of.erase(old->second.p);
             cudaFree(old->second.p);
