@@ -159,8 +159,8 @@ const char* pd_last_error(void);
 /* number of CUDA kernels this library has launched so far (all handles) */
 unsigned long long pd_launch_count(void);
 /* Device blocks freed by the library (outside the serving loop) are cached for
- * reuse up to a limit (4 GiB by default): pd_empty_cache returns them to the
- * driver; pd_set_cache_limit sets the limit (bytes < 0: unchanged) and reports
+ * reuse up to a limit (4 GiB by default; beyond it kept blocks make room for newer
+ * ones): pd_empty_cache returns them to the driver; pd_set_cache_limit sets the limit (bytes < 0: unchanged) and reports
  * the bytes held.  No counterpart in the reference package (its device memory
  * comes from a dependency's allocator). */
 int pd_empty_cache(void);
