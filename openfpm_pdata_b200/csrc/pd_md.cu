@@ -1315,7 +1315,8 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
         // how far the batch came
         int done = K;
         drifted = due = false;
-        if (!always && (fused || K > 1)) {
+        const bool next = fused && s + K < steps;  // the batch drifted the step after it
+        if (!always && (K > 1 || next)) {
             PD_CUDA(cudaMemcpyAsync(md->slots_h, slots, sizeof(unsigned long long) * (K + 1), cudaMemcpyDeviceToHost,
                                     st));
             PD_CUDA(cudaStreamSynchronize(st));
@@ -1328,11 +1329,11 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
             while (done < K && !(over(done))) ++done;
             if (done < K) {  // step s + done is drifted and needs a rebuild first
                 drifted = due = true;
-            } else if (fused && s + K < steps) {
+            } else if (next) {
                 drifted = true;
                 due = over(K);
             }
-        } else if (fused && s + K < steps) {
+        } else if (next) {
             drifted = true;
             due = always;
         }
