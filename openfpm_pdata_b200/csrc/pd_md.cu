@@ -553,7 +553,8 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
     }
     const bool narrow = md->tile_tx == 0 && md->physics == 0 && h->dtype == PD_F64;
     const int tx_auto = tx_req;
-    if (narrow && md->fit_req == tx_auto) tx_req = md->fit_tx;  // as the build before found it
+    const bool sph_auto = md->tile_tx == 0 && md->physics == 1;
+    if ((narrow || sph_auto) && md->fit_req == tx_auto) tx_req = md->fit_tx;  // as the build before found it
     // what the densest tile's staging should stay within, for the automatic widths:
     //  - LJ, FP64 vectors: every tile's CTA takes the shared memory of the densest one, so
     //    on an uneven system a width from the mean occupancy costs residency.  The CTAs
@@ -562,23 +563,28 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
     //    (tiles of few particles cost more than residency).  1,000,003 particles in
     //    clusters, mean width 32: precision form 494 us at 32 cells, 371 at 18, 408 at 11;
     //    FP64 315, 291, 377.
-    //  - SPH: about 1730 staged particles (two records each; five cells of a filled tank):
-    //    fewer, wider tiles stage less per particle, which counts for more than residency.
-    //    FP64, dp = 1/128: rates 608 us at two cells (three CTAs per SM), 576 at five
-    //    (two); FP32, dp = 1/180: 733 us at four cells, 659 at five, 754 at six.  The mean
-    //    occupancy counts the empty part of the tank.
-    const long target = md->physics == 1 ? 1730 : (md->mixed ? (227 * 1024 / 5 - 10752) / 16 : (227 * 1024 / 4 - 4608) / 24);
-    const bool sph_auto = md->tile_tx == 0 && md->physics == 1;
-    // the width for a densest tile of `t` records at the current one (narrower, or the
+    //  - SPH: two records a particle; wider tiles stage less per particle, down to two CTAs per
+    //    SM in FP64 (384 threads) and four in FP32, and not more than 150 particles at the densest
+    //    tile's occupancy (the mean counts the empty part of the tank), six cells of a filled one:
+    //    small systems otherwise have too few tiles.  us a step at two, five and six cells: FP64
+    //    dp = 1/128 786, 557, 836 (one CTA per SM), 1/100 407, 306, 447, 1/60 120, 100, 99 and
+    //    130 at nine; FP32 1/128 393, 293, 318, 1/100 212, 169, 187, 1/60 70, 62, 62 and 68 at nine.
+    const long target = md->physics == 1 ? (h->dtype == PD_F64 ? 1730 : 1700)
+                                         : (md->mixed ? (227 * 1024 / 5 - 10752) / 16 : (227 * 1024 / 4 - 4608) / 24);
+    // the width for a densest tile of `t` records at the current one (LJ: narrower, or the
     // automatic one again)
     auto fit = [&](long t) {
         int tx = md->tg.TX;
+        if (sph_auto) {
+            const double column = std::max((double)t / (tx + 2), 1.0);  // records a cell along x
+            const int widest = std::min((int)TXMAX, cl->gs[0] - 2 * cl->pad);
+            const int most = std::max(1, std::min(widest, std::min((int)(150 * 9 / column), (int)(target / column) - 2)));
+            return tx > most || tx + 1 < most ? most : tx;  // (one cell more is an estimate's error)
+        }
         if (narrow && t > target)
             tx = std::min(tx, std::max((tx_auto + 1) / 2, (int)((double)(tx + 2) * (double)target / (double)t) - 2));
         else if (narrow && tx < tx_auto && t * 5 < target * 4)
             tx = tx_auto;  // the densest part thinned out
-        else if (sph_auto && tx > 1 && t > target)
-            tx = std::min(tx, std::max(1, (int)((double)(tx + 2) * (double)target / (double)t) - 2));
         return narrow ? std::min(tx, tx_auto) : tx;
     };
     auto fits = [&](unsigned int t) { return md->physics == 1 ? sph_tile_fits(h, t) : tile_fits(h, t); };
@@ -620,9 +626,12 @@ static int md_tiles(pd_md md, pd_cl cl, cudaStream_t st) {
         const int tx = fit(h->ctrl_h->tile_max);
         if (tx != md->tg.TX && tx >= 1) {
             PD_TRY(plan(tx, &ok));
+            // the estimate of a wider tile can miss what the target stands for
+            while (ok && sph_auto && (long)h->ctrl_h->tile_max > target && md->tg.TX > 1)
+                PD_TRY(plan(md->tg.TX - 1, &ok));
             if (!ok) return PD_OK;
         }
-        if (narrow) {
+        if (narrow || sph_auto) {
             md->fit_req = tx_auto;
             md->fit_tx = md->tg.TX;
         }
