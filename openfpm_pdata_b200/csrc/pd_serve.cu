@@ -349,12 +349,15 @@ __device__ __forceinline__ void b_force_tile_any(const SysDesc& d, long t, unsig
 
 // Persistent force kernel of one shape group (LANES lanes per particle, CTAs of
 // BLOCK threads): the tiles [grp[k], grp[k+1]) of the systems of that shape, from a work
-// queue.  At 48 registers and 35 KB of staging five CTAs of 256 fit an SM: 24 systems of
-// 1,017,733 particles 426 -> 379 us a step against four (80 registers, 48 KB).  Measured and
-// not kept: the queue's next entry fetched while a tile is computed (478 us) and tiles
+// queue.  PER CTAs of 256 per SM: at five (48 registers, 35 KB of staging) 24 systems of
+// 1,017,733 particles take 379 us a step, with 80 registers 426.  With no more tiles than CTAs
+// at five a step waits for one tile's latency, which the spills at 48 registers lengthen: 8 systems
+// of 4,000 particles 33.0 us at five, 27.5 at three (FEW_PER; up to half of a small system's tiles
+// hold images only). Measured and not kept: the queue's next entry fetched while a tile is computed (478 us) and tiles
 // dealt out in turn (471 us) -- a tile then waits for its CTA while others are idle.
-template <int LANES, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 5 * FBLOCK_T / BLOCK) k_b_force(const SysDesc* __restrict__ D, BatchHdr* __restrict__ B,
+static constexpr int FULL_PER = 5, FEW_PER = 3;
+template <int LANES, int BLOCK, int PER>
+__global__ void __launch_bounds__(BLOCK, PER * FBLOCK_T / BLOCK) k_b_force(const SysDesc* __restrict__ D, BatchHdr* __restrict__ B,
                                                    LJP<float> Pr, double* __restrict__ tpart,
                                                    long* __restrict__ ovf) {
     extern __shared__ __align__(128) unsigned char tile_raw[];
@@ -1123,7 +1126,8 @@ struct pd_srv_s {
     PinnedFifo outbox;
     CopyPool copier;  // submissions' copies into the inbox, results' out of the outbox
     bool adm_pending = false;
-    cudaGraphExec_t gstep[4] = {nullptr, nullptr, nullptr, nullptr};  // 1, 2, 4, 8 steps per launch
+    cudaGraphExec_t gstep[2][4] = {};  // [few tiles][1, 2, 4, 8 steps per launch]
+    int sms = 148;
     bool dirty = true;
     // autotuner: size bucket -> tile width, lanes per particle, CTA size of the force kernel
     bool autotune = true;
@@ -1282,7 +1286,7 @@ static int upload_tables(pd_srv s) {
 static constexpr int GRAPH_KERNELS = 38;  // kernel nodes per step of the step graphs
 
 // the step graphs: 2^lk velocity-Verlet steps of every active system per launch
-static int capture_graph(pd_srv s, int lk) {
+template <int PER> static int capture_graph(pd_srv s, int lk) {
     float half = (float)(0.5 * s->dt / 1.0), dt = (float)s->dt;
     LJP<float> P{};
     P.eps24 = (float)(24.0 * s->lj.eps);
@@ -1290,7 +1294,7 @@ static int capture_graph(pd_srv s, int lk) {
     P.sig2 = (float)(s->lj.sigma * s->lj.sigma);
     mixed_cutoff(s->lj, P);
 #define PD_SRV_FORCE_ATTR(L, BL) \
-    PD_CUDA(cudaFuncSetAttribute(k_b_force<L, BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SRV_SMEM));
+    PD_CUDA(cudaFuncSetAttribute(k_b_force<L, BL, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, SRV_SMEM));
     PD_SRV_FORCE_ATTR(1, FBLOCK_T)
     PD_SRV_FORCE_ATTR(2, FBLOCK_T)
     PD_SRV_FORCE_ATTR(4, FBLOCK_T)
@@ -1302,11 +1306,12 @@ static int capture_graph(pd_srv s, int lk) {
     PD_CUDA(cudaFuncSetAttribute(k_b_force_ovf<FBLOCK_T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SRV_BIG));
     PD_CUDA(cudaFuncSetAttribute(k_b_force_ovf<FBLOCK_T / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SRV_BIG));
     PD_CUDA(cudaFuncSetAttribute(k_rb_build<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SRV_BIG));
-    int sms = 148, dev = 0, per = 1, per2 = 1, perb = 1;
+    int dev = 0, per = 1, per2 = 1, perb = 1;
     PD_CUDA(cudaGetDevice(&dev));
-    PD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_b_force<2, FBLOCK_T>, FBLOCK_T, SRV_SMEM));
-    PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_b_force<2, FBLOCK_T / 2>, FBLOCK_T / 2, SRV_SMEM));
+    PD_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, dev));
+    const int sms = s->sms;
+    PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_b_force<2, FBLOCK_T, PER>, FBLOCK_T, SRV_SMEM));
+    PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, k_b_force<2, FBLOCK_T / 2, PER>, FBLOCK_T / 2, SRV_SMEM));
     PD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perb, k_rb_build<0>, TBLOCK, SRV_BSMEM));
     const int gf = sms * std::max(per, 1), gf2 = sms * std::max(per2, 1), gb = sms * std::max(perb, 1), gc = sms * 8;
     const SysDesc* D = s->desc.as<SysDesc>();
@@ -1356,12 +1361,15 @@ static int capture_graph(pd_srv s, int lk) {
     // step of every system
     k_b_replay<<<gc, CHUNK, 0, st>>>(D, B, fl);
     // one persistent force kernel per shape group (a group without systems returns at once)
-    k_b_force<1, FBLOCK_T><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
-    k_b_force<2, FBLOCK_T><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
-    k_b_force<4, FBLOCK_T><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
-    k_b_force<1, FBLOCK_T / 2><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
-    k_b_force<2, FBLOCK_T / 2><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
-    k_b_force<4, FBLOCK_T / 2><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
+    k_b_force<1, FBLOCK_T, PER><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
+    k_b_force<2, FBLOCK_T, PER><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
+    k_b_force<4, FBLOCK_T, PER><<<gf, FBLOCK_T, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
+    k_b_force<1, FBLOCK_T / 2, PER><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(),
+                                                                        s->ovf_f.as<long>());
+    k_b_force<2, FBLOCK_T / 2, PER><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(),
+                                                                        s->ovf_f.as<long>());
+    k_b_force<4, FBLOCK_T / 2, PER><<<gf2, FBLOCK_T / 2, SRV_SMEM, st>>>(D, B, P, s->tpart.as<double>(),
+                                                                        s->ovf_f.as<long>());
     k_b_force_ovf<FBLOCK_T><<<sms, FBLOCK_T, SRV_BIG, st>>>(D, B, P, s->tpart.as<double>(), s->ovf_f.as<long>());
     k_b_force_ovf<FBLOCK_T / 2><<<sms, FBLOCK_T / 2, SRV_BIG, st>>>(D, B, P, s->tpart.as<double>(),
                                                                    s->ovf_f.as<long>());
@@ -1375,7 +1383,7 @@ static int capture_graph(pd_srv s, int lk) {
         set_error("serving: graph capture failed: %s", cudaGetErrorString(ce));
         return PD_ECUDA;
     }
-    ce = cudaGraphInstantiate(&s->gstep[lk], g, 0);
+    ce = cudaGraphInstantiate(&s->gstep[PER == FEW_PER][lk], g, 0);
     cudaGraphDestroy(g);
     if (ce != cudaSuccess) {
         set_error("serving: graph instantiation failed: %s", cudaGetErrorString(ce));
@@ -1954,7 +1962,10 @@ int pd_srv_create(long hbm_budget_bytes, int max_slots, const pd_lj_params_t* lj
         // per step (cudaMemGetInfo took 10-100 ms at times on a shared node)
         s->budget = (long)std::min((size_t)s->budget, want);
     }
-    for (int lk = 0; lk < 4 && r == PD_OK; ++lk) r = capture_graph(s, lk);
+    for (int lk = 0; lk < 4 && r == PD_OK; ++lk) {
+        r = capture_graph<FULL_PER>(s, lk);
+        if (r == PD_OK) r = capture_graph<FEW_PER>(s, lk);
+    }
     if (r != PD_OK) {
         pd_srv_destroy(s);
         return r;
@@ -1979,8 +1990,9 @@ int pd_srv_destroy(pd_srv s) {
     s->inbox.destroy();
     s->outbox.destroy();
     s->slots.clear();
-    for (auto& ge : s->gstep)
-        if (ge) cudaGraphExecDestroy(ge);
+    for (auto& set : s->gstep)
+        for (auto& ge : set)
+            if (ge) cudaGraphExecDestroy(ge);
     Buf* bufs[] = {&s->desc, &s->hdr,   &s->maxd2, &s->errs, &s->flags, &s->phase,
                    &s->work, &s->nnmax, &s->tpart, &s->kpart, &s->ovf_f, &s->ovf_b};
     for (Buf* b : bufs) b->release();
@@ -2070,7 +2082,8 @@ int pd_srv_tick(pd_srv s, int* n_active, int* n_queued) {
     while (lk < 3 && (2 << lk) <= K) ++lk;
     K = 1 << lk;
     double t_step = now_s(s);
-    if (stepping) PD_CUDA(cudaGraphLaunch(s->gstep[lk], s->st));
+    const bool few = s->hhdr.tot_tiles <= (long)FULL_PER * s->sms;  // (up to half of them hold images only)
+    if (stepping) PD_CUDA(cudaGraphLaunch(s->gstep[few][lk], s->st));
     double ta = now_s(s);
     std::vector<char> used_slot(s->max_slots, 0);
     for (SrvReq* r : s->active) used_slot[r->slot] = 1;

@@ -206,3 +206,19 @@ def test_result_and_release_follow_the_request_state(pd):
     srv.release(t)
     with pytest.raises(pd.PdError):
         srv.release(t)
+
+
+def test_few_and_many_tiles_agree(pd):
+    """A system alone (few tiles: the force kernel at three CTAs per SM) and among others that fill the
+    GPU (at five) gets the same trajectory and energies bit for bit."""
+    from openfpm_pdata_b200 import workloads
+    x, v, L = workloads.serving_system(3000, 0.8, seed=1)
+    rest = [workloads.serving_system(12000, 0.8, seed=2 + k) for k in range(8)]
+    got = []
+    for others in ([], rest):
+        srv = pd.Server(2 << 30, max_slots=16, dt=0.005, skin=0.3, autotune=False)
+        t = [srv.submit(a, b, c, 15) for a, b, c in [(x, v, L)] + others]
+        srv.run_until_done(t)
+        got.append(srv.result(t[0]))
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1], got[1][1])
