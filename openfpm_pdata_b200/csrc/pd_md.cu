@@ -671,6 +671,7 @@ static unsigned long md_reorder_mask(pd_md md) {
 int md_rebuild(pd_md md, cudaStream_t st) {
     pd_vd h = md->h;
     if (md->mixed && md->off_valid) PD_TRY(mixed_to_positions(h, md->vl->cl, md->off, st));
+    md->off_valid = false;  // the positions are the state until the offsets are formed again
     h->n_total = h->n_real;
     h->img_valid = false;
     PD_TRY(wrap_positions(h, h->n_real, st));
@@ -1200,8 +1201,7 @@ static int md_images(pd_md md, const StepGuard& guard, cudaStream_t st) {
 // steps expected until the next rebuild (the last interval); a step too many costs two
 // launches that return at once.  The operations of each step and their order do not
 // depend on the batches.
-int pd_md_run(pd_md md, int steps, void* stream, double* E) {
-    if (!md || steps < 0) return PD_EINVAL;
+static int md_run(pd_md md, int steps, void* stream, double* E) {
     if (md_cluster_eligible(md)) return md_run_cluster(md, steps, S(stream), E);
     if (md->mp.use_cell_list && md->physics == 0 && !md->mixed && !md->timing)
         return md_run_cl_graph(md, steps, S(stream), E);
@@ -1396,6 +1396,14 @@ int pd_md_run(pd_md md, int steps, void* stream, double* E) {
         return PD_EOVERFLOW;
     }
     return PD_OK;
+}
+
+int pd_md_run(pd_md md, int steps, void* stream, double* E) {
+    if (!md || steps < 0) return PD_EINVAL;
+    const int rc = md_run(md, steps, stream, E);
+    // a run that stopped may have left the list half built: the next one builds it first
+    if (rc != PD_OK) md->ready = false;
+    return rc;
 }
 
 int pd_md_set_timing(pd_md md, int on) {

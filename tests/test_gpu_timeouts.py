@@ -36,7 +36,10 @@ def test_verlet_list(pd, sym):
 
 
 @pytest.mark.parametrize("form", ["f64", "f32", "mixed", "global rows", "buckets", "graph"])
-def test_md_run(pd, form):
+@pytest.mark.parametrize("rebuild", [False, True])
+def test_md_run(pd, form, rebuild):
+    """The run that reports it ends in the middle of a rebuild or between rebuilds; the next ones go on from a
+    whole state."""
     from openfpm_pdata_b200 import workloads
     cells = form in ("buckets", "graph")
     x, v, L = workloads.lj_lattice(44 if form == "graph" else 10, 1.1, 0.05, seed=3)
@@ -46,8 +49,16 @@ def test_md_run(pd, form):
                        props=[(t, 3), (t, 3)])
     vd.hostToDevicePos(x.astype(dtype))
     vd.hostToDeviceProp(0, v)
-    md = pd.MD(vd, 0, 1, dt=0.001, skin=0.0 if cells else 0.3, use_cell_list=cells,
+    skin = 0.0 if cells else (0.002 if rebuild else 0.3)  # 0.002: rebuilt at almost every step
+    md = pd.MD(vd, 0, 1, dt=0.001, skin=skin, use_cell_list=cells,
                precision=pd.PREC_MIXED if form == "mixed" else pd.PREC_FP64)
     if form == "global rows":
         md.set_tiles(False)
+    E0 = md.run(1)
     _times_out_once(pd, vd, lambda: md.run(2))
+    E = md.run(3)
+    tot, tot0 = E[:, 0] + E[:, 1], E0[0, 0] + E0[0, 1]
+    assert np.abs(tot - tot0).max() < 0.02 * abs(tot0)
+    assert np.isfinite(vd.deviceToHostPos()).all()
+    if rebuild or cells:
+        assert E[:, 3].sum() >= 2
