@@ -508,15 +508,14 @@ __device__ __forceinline__ bool grid_barrier(cg::cluster_group& cl, unsigned int
                                              unsigned int* err) {
     cl.sync();
     if (cl.block_rank() == 0 && threadIdx.x == 0) {
-        // the cluster's writes before cl.sync() are this thread's to release (cumulativity): one fence
-        __threadfence();
-        atomicAdd(bar, 1u);
+        // the cluster's writes before cl.sync() are this thread's to release (cumulativity), the
+        // other clusters' its to acquire for the cluster
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         unsigned int seen = 0, it = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
         } while (seen < target && ++it < (1u << 21));
         if (seen < target) atomicOr(err, ERR_TIMEOUT);
-        __threadfence();
     }
     cl.sync();
     return __syncthreads_or((__ldcg(err) & ERR_TIMEOUT) ? 1 : 0) == 0;
