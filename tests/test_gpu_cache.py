@@ -88,7 +88,7 @@ def test_full_cache_takes_new_blocks(pd):
             before = pd.set_cache_limit()
             c = [vec(2000000), vec(2100000)]
             took = before - pd.set_cache_limit()
-            assert k == 0 or took > (60 << 20)
+            assert k == 0 or took > (40 << 20)
             del c
     finally:
         pd.set_cache_limit(4 << 30)
